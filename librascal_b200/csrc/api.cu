@@ -218,7 +218,7 @@ struct rgpu_structures {
   DevBuf E_d, F_d, S_d, K64, t64, erow64, Wh, Wl, dX32, dC32, epart, Xh, Xl, chunk_map;
   bool feat_x32{false};  // FP32 features also kept unsplit (for export)
   DevBuf dCp, dCs, dXp;
-  DevBuf knm, W64, plist, Vvir;  // sparse kernel matrices for training
+  DevBuf knm, plist, Vvir;  // sparse kernel matrices for training
   // MD step recorded as a CUDA graph (rgpu_md_step)
   cudaGraph_t md_graph{nullptr};
   cudaGraphExec_t md_exec{nullptr};
@@ -786,6 +786,27 @@ void model_layout_bf16(rgpu_gap_model * m, rgpu_structures * s) {
 
 size_t plain_budget_bytes() { return size_t(24) << 30; }
 
+// The dots K = X_s T_s^T of every central species, as planes in s->K64.
+GapGroup species_dots(rgpu_gap_model * m, rgpu_structures * s) {
+  const FeatureDims & fd = s->fd;
+  GapGroup g;
+  g.S = fd.S;
+  for (int sI = 0; sI < fd.S; ++sI) {
+    g.rows[sI] = s->species_count[sI];
+    g.row0[sI + 1] = g.row0[sI] + g.rows[sI];
+    g.M[sI] = m->segs[sI].M;
+    g.m0[sI] = m->segs[sI].m0;
+    g.ldk[sI] = (g.M[sI] + 1) & ~1;
+    g.koff[sI] = g.plane;
+    g.plane += g.rows[sI] * g.ldk[sI];
+  }
+  gap_dots_split(g, fd.D);
+  s->K64.ensure(sizeof(double) * size_t(g.plane) * g.splits + 64);
+  launch_gap_dots_fp64(g, fd.D, s->X64.as<double>(), fd.Dpad, m->T64.as<double>(), fd.Dpad, s->K64.as<double>(),
+                       s->st);
+  return g;
+}
+
 void gap_plain(rgpu_gap_model * m, rgpu_structures * s, double * E_d, double * grad_d, bool forces,
                double * stress_d) {
   rgpu_calculator * c = m->calc;
@@ -793,31 +814,17 @@ void gap_plain(rgpu_gap_model * m, rgpu_structures * s, double * E_d, double * g
   const int64_t nc = s->nl.n_centers;
   cudaStream_t st = s->st;
   mark(s, 4);
-  // forward GEMMs per species: k = X T^T, pointwise, t = W T
-  int Mmax = 0;
-  for (auto & g : m->segs) Mmax = std::max(Mmax, g.M);
-  s->K64.ensure(sizeof(double) * size_t(nc) * std::max(Mmax, 1) + 64);
+  // k = X T^T, pointwise, t = W T, all species in one launch each
   s->erow64.ensure(sizeof(double) * (nc + 1));
   s->t64.ensure(sizeof(double) * size_t(nc) * fd.Dpad + 64);
-  launch_fill_f64(s->erow64.as<double>(), nc, 0., st);
-  int64_t row0 = 0;
-  for (int sI = 0; sI < fd.S; ++sI) {
-    const int64_t rows = s->species_count[sI];
-    const GapSpecies & g = m->segs[sI];
-    if (rows > 0 && g.M > 0) {
-      const double * Xs = s->X64.as<double>() + size_t(row0) * fd.Dpad;
-      const double * Ts = m->T64.as<double>() + size_t(g.m0) * fd.Dpad;
-      double * Kb = s->K64.as<double>();
-      gemm_nt_fp64(rows, g.M, fd.D, Xs, fd.Dpad, Ts, fd.Dpad, Kb, g.M, st);
-      launch_gap_pointwise_fp64(rows, g.M, Kb, g.M, m->alpha64.as<double>() + g.m0, m->zeta, Kb, g.M,
-                                s->erow64.as<double>() + row0, st);
-      if (forces)
-        gemm_nn_fp64(rows, fd.D, g.M, Kb, g.M, Ts, fd.Dpad, s->t64.as<double>() + size_t(row0) * fd.Dpad,
-                     fd.Dpad, st);
-    } else if (forces && rows > 0) {
-      launch_fill_f64(s->t64.as<double>() + size_t(row0) * fd.Dpad, rows * fd.Dpad, 0., st);
-    }
-    row0 += rows;
+  const GapGroup g = species_dots(m, s);
+  launch_gap_pointwise_fp64(g, s->K64.as<double>(), m->alpha64.as<double>(), m->zeta, s->erow64.as<double>(), st);
+  if (forces) {
+    launch_gap_scaled_fp64(g, fd.D, s->K64.as<double>(), m->T64.as<double>(), fd.Dpad, s->t64.as<double>(), fd.Dpad,
+                           st);
+    for (int sI = 0; sI < fd.S; ++sI)
+      if (g.rows[sI] > 0 && g.M[sI] == 0)
+        launch_fill_f64(s->t64.as<double>() + size_t(g.row0[sI]) * fd.Dpad, g.rows[sI] * fd.Dpad, 0., st);
   }
   // struct of each sorted row
   launch_energy_reduce(nc, 0, nullptr, 0, s->erow64.as<double>(), 0, s->center_of_row.as<int32_t>(),
@@ -1236,37 +1243,17 @@ static void kernel_features(rgpu_gap_model * m, rgpu_structures * s, bool grads)
   model_layout(m, s, false);
 }
 
-// K = X_s T_s^T of species sI into s->K64 (rows x M).
-static void species_dots(rgpu_gap_model * m, rgpu_structures * s, int sI, int64_t row0) {
-  const FeatureDims & fd = s->fd;
-  const GapSpecies & g = m->segs[sI];
-  const int64_t rows = s->species_count[sI];
-  s->K64.ensure(sizeof(double) * size_t(std::max<int64_t>(rows, 1)) * std::max(g.M, 1) + 64);
-  gemm_nt_fp64(rows, g.M, fd.D, s->X64.as<double>() + size_t(row0) * fd.Dpad, fd.Dpad,
-               m->T64.as<double>() + size_t(g.m0) * fd.Dpad, fd.Dpad, s->K64.as<double>(), g.M, s->st);
-}
-
 // K_NM energy rows: SparseKernelImpl<GAP>::compute for target Structure
 // (models/sparse_kernels.hh:104-131) or Atom (:165-191).
 static void sparse_kernel_impl(rgpu_gap_model * m, rgpu_structures * s, bool atom_target, double * out) {
   kernel_features(m, s, false);
-  const FeatureDims & fd = s->fd;
   const int64_t rows_out = atom_target ? s->nl.n_centers : s->n_struct;
   const size_t bytes = sizeof(double) * size_t(rows_out) * m->M;
   s->knm.ensure(bytes + 64);
   RGPU_CUDA(cudaMemsetAsync(s->knm.p, 0, bytes, s->st));
-  int64_t row0 = 0;
-  for (int sI = 0; sI < fd.S; ++sI) {
-    const int64_t rows = s->species_count[sI];
-    const GapSpecies & g = m->segs[sI];
-    if (rows > 0 && g.M > 0) {
-      species_dots(m, s, sI, row0);
-      launch_knm_rows(rows, g.M, s->K64.as<double>(), m->zeta, s->center_of_row.as<int32_t>(), row0,
-                      s->nl.center_struct, atom_target, m->ucol.as<int32_t>() + g.m0, s->knm.as<double>(), m->M,
-                      s->st);
-    }
-    row0 += rows;
-  }
+  const GapGroup g = species_dots(m, s);
+  launch_knm_rows(g, s->K64.as<double>(), m->zeta, s->center_of_row.as<int32_t>(), s->nl.center_struct, atom_target,
+                  m->ucol.as<int32_t>(), s->knm.as<double>(), m->M, s->st);
   if (bytes) RGPU_CUDA(cudaMemcpyAsync(out, s->knm.p, bytes, cudaMemcpyDeviceToHost, s->st));
   RGPU_CUDA(cudaStreamSynchronize(s->st));
 }
@@ -1293,22 +1280,10 @@ static void sparse_kernel_derivative_impl(rgpu_gap_model * m, rgpu_structures * 
     RGPU_CUDA(cudaStreamSynchronize(st));
     return;
   }
-  // zeta (X_i . T_m)^(zeta-1) of every row, species by species
-  std::vector<int64_t> woff(fd.S + 1, 0), srow0(fd.S + 1, 0);
-  for (int sI = 0; sI < fd.S; ++sI) {
-    woff[sI + 1] = woff[sI] + s->species_count[sI] * m->segs[sI].M;
-    srow0[sI + 1] = srow0[sI] + s->species_count[sI];
-  }
-  s->W64.ensure(sizeof(double) * size_t(std::max<int64_t>(woff[fd.S], 1)) + 64);
+  // zeta (X_i . T_m)^(zeta-1) of every row
   mark(s, 4);
-  for (int sI = 0; sI < fd.S; ++sI) {
-    const int64_t rows = s->species_count[sI];
-    const GapSpecies & g = m->segs[sI];
-    if (rows == 0 || g.M == 0) continue;
-    gemm_nt_fp64(rows, g.M, fd.D, s->X64.as<double>() + size_t(srow0[sI]) * fd.Dpad, fd.Dpad,
-                 m->T64.as<double>() + size_t(g.m0) * fd.Dpad, fd.Dpad, s->W64.as<double>() + woff[sI], g.M, st);
-    launch_kernel_weight(rows * g.M, s->W64.as<double>() + woff[sI], m->zeta, st);
-  }
+  const GapGroup gg = species_dots(m, s);
+  launch_kernel_weight(gg, s->K64.as<double>(), m->zeta, st);
   mark(s, 5);
   mark(s, 6);
   // The reference returns from its loop over structures at the first one
@@ -1398,8 +1373,9 @@ static void sparse_kernel_derivative_impl(rgpu_gap_model * m, rgpu_structures * 
       a.T = m->T64.as<double>() + size_t(g.m0) * fd.Dpad;
       a.ldt = fd.Dpad;
       a.M = g.M;
-      a.W = s->W64.as<double>() + woff[sI];
-      a.row0 = srow0[sI];
+      a.W = s->K64.as<double>() + gg.koff[sI];
+      a.ldw = gg.ldk[sI];
+      a.row0 = gg.row0[sI];
       a.row_of_center = s->row_of_center.as<int32_t>();
       a.pair_j = s->nl.pair_j;
       a.ucol = m->ucol.as<int32_t>() + g.m0;
@@ -1421,6 +1397,7 @@ static void sparse_kernel_derivative_impl(rgpu_gap_model * m, rgpu_structures * 
         b.ldt = a.ldt;
         b.M = g.M;
         b.W = a.W;
+        b.ldw = a.ldw;
         b.row0 = a.row0;
         b.row_of_center = a.row_of_center;
         b.center_struct = s->nl.center_struct;
@@ -1510,7 +1487,7 @@ static std::vector<const void *> md_buffers(const rgpu_gap_model * m, const rgpu
                            &s->C64, &s->X64,
                            &s->invn64, &s->C32, &s->X32, &s->xscale32, &s->E_d, &s->F_d, &s->S_d, &s->K64,
                            &s->t64, &s->erow64, &s->Wh, &s->Wl, &s->dX32, &s->dC32, &s->epart, &s->Xh, &s->Xl,
-                           &s->chunk_map, &s->dCp, &s->dCs, &s->dXp, &s->knm, &s->W64, &s->plist, &s->Vvir})
+                           &s->chunk_map, &s->dCp, &s->dCs, &s->dXp, &s->knm, &s->plist, &s->Vvir})
     v.push_back(b->p);
   const NlWork & w = s->nlw;
   for (const DevBuf * b : {&w.geom, &w.counts64, &w.scan_tmp, &w.ghost_off, &w.site_x, &w.site_type, &w.site_real,

@@ -1,159 +1,251 @@
-// FP64 tile GEMM on the CUDA cores: C[r][c] = sum_k A[r][k] B(k, c), with
-// the A rows addressed through a row-offset functor (plain strided rows, or
-// rows gathered from a list) and the result handed to an epilogue functor
-// (a plain store, or the scaled scatter of the sparse-kernel gradient
-// block). B is either N x K row-major (B_NT, C = A B^T) or K x N row-major.
+// FP64 tile GEMM on the tensor cores (mma.sync m16n8k8 f64): C[r][c] =
+// sum_k A[r][k] B(k, c), with the A rows addressed through a row-offset
+// functor (plain strided rows, or rows gathered from a list) and the result
+// handed to an epilogue functor. B is either N x K row-major (B_NT,
+// C = A B^T) or K x N row-major. Several problems (one per species) run in
+// one launch, and K can be cut into splits whose partial sums go to separate
+// planes that the caller's next kernel adds.
 //
-// Tile 128 x BN x 8 (BN = 128 or 64), 256 threads in a 16 x 16 grid.
-// Thread (ty, tx) owns rows 32 g + 2 ty + {0, 1}, g = 0..3, and columns
-// 32 g + 2 tx + {0, 1}, g < BN / 32, so every shared-memory read is a
-// 16-byte vector and the 16 column pairs of a warp are contiguous (no bank
-// conflicts). The next k-slice is loaded into registers while the current
-// one is multiplied; shared memory is double buffered, one barrier per
-// slice. BN = 64 halves the accumulators, so two blocks fit on an SM.
+// What bounds it: the FP64 tensor pipe (37.0 TFLOP/s measured with register
+// operands against 29.1 for the same chains of DFMA), which only a full
+// grid reaches. The tile is 64 x 64 rather than 128 x 128 because a warp's
+// 16 x 8 x 8 product needs so few operands (24 doubles for 1024 FMAs) that
+// shared memory does not care, and because the GAP contractions are ragged:
+// per species a few hundred to a few thousand rows by 50..2000 sparse
+// points. 128 x 128 tiles of one species at a time left 6 to 84 blocks on
+// 148 SMs. Splits of K fill the chip where even 64 x 64 tiles of every
+// species do not.
+//
+// 128 threads, 2 x 2 warps of 32 x 32; slices of 16 k in a three-deep
+// cp.async ring. The shared row strides (20 doubles for k-major tiles, 68
+// for the K x N tile, both 4 modulo 16) put the 16 operands of a half-warp
+// load in 16 different 8-byte banks.
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 
 namespace rgpu {
 
-constexpr int kDgBM = 128, kDgBN = 128, kDgBK = 8;
+constexpr int kDgBM = 64, kDgBN = 64, kDgBK = 16, kDgStages = 3, kDgThreads = 128;
+constexpr int kDgLdK = kDgBK + 4, kDgLdN = kDgBN + 4;  // shared row strides, in doubles
+constexpr int kDgStageA = kDgBM * kDgLdK;
+constexpr int kDgStageB = kDgBN * kDgLdK;  // covers the 16 x 68 tile too
+constexpr size_t kDgSmem = sizeof(double) * kDgStages * (kDgStageA + kDgStageB);
+constexpr int kDgMaxProblems = kMaxSpecies;
+static_assert(kDgBK * kDgLdN <= kDgStageB, "the K x N tile fits the stage");
 
 struct DgPlainRows {
   int64_t lda;
-  __device__ __forceinline__ int64_t operator()(int64_t r) const { return r * lda; }
+  __host__ __device__ __forceinline__ int64_t operator()(int64_t r) const { return r * lda; }
 };
 
+// C[split][r][c]; planes are `plane` values apart.
 struct DgStoreC {
   double * C;
-  int64_t ldc;
-  __device__ __forceinline__ void operator()(int64_t r, int c, double v) const { C[r * ldc + c] = v; }
+  int64_t ldc, plane;
+  __device__ __forceinline__ void operator()(int64_t r, int c, double v, int split) const {
+    C[split * plane + r * ldc + c] = v;
+  }
 };
 
-template <bool B_NT, int BN, class ARows, class Epi>
-__global__ void __launch_bounds__(256, BN == 64 ? 2 : 1)
-dgemm_kernel(int64_t M, int N, int K, const double * __restrict__ A, ARows arows,
-             const double * __restrict__ B, int64_t ldb, Epi epi) {
-  constexpr int JG = BN / 32;   // column groups of a thread; also B values per thread per slice
-  __shared__ __align__(16) double As[2][kDgBK][kDgBM];
-  __shared__ __align__(16) double Bs[2][kDgBK][BN];
-  __shared__ int64_t a_off[kDgBM];
-  const int t = threadIdx.x;
-  const int tx = t & 15, ty = t >> 4;
-  // column tiles vary fastest: the blocks that share an A row tile run
-  // together, so A comes from DRAM once and the others read it from L2
-  const int64_t r0 = int64_t(blockIdx.y) * kDgBM;
-  const int c0 = int(blockIdx.x) * BN;
-  if (t < kDgBM) a_off[t] = (r0 + t < M) ? arows(r0 + t) : int64_t(-1);
-  __syncthreads();
-  // global -> register loaders: A tiles 2 threads per row, 4 k each; B_NT
-  // tiles (BN rows) 2 threads per row with 4 k (BN = 128) or 4 threads per
-  // row with 2 k (BN = 64)
-  const int lr = t >> 1, lk = (t & 1) * 4;
-  const int64_t my_a = a_off[lr];
-  constexpr int BK_T = JG;      // k values of a B_NT row per thread: 8 * BN / 256
-  const int br = (BN == 128) ? (t >> 1) : (t >> 2);
-  const int bk = (BN == 128) ? (t & 1) * 4 : (t & 3) * 2;
-  const int64_t my_b = (c0 + br < N) ? int64_t(c0 + br) * ldb : int64_t(-1);
-  // B (K x N) tiles: 8 k-rows of BN columns, 32 threads per row, columns 32 apart
-  const int nk = t >> 5, nc = t & 31;
-  double pa[4], pb[JG];
-  auto load = [&](int k0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int k = k0 + lk + q;
-      pa[q] = (my_a >= 0 && k < K) ? A[my_a + k] : 0.;
-    }
-    if (B_NT) {
-#pragma unroll
-      for (int q = 0; q < BK_T; ++q) {
-        const int k = k0 + bk + q;
-        pb[q] = (my_b >= 0 && k < K) ? B[my_b + k] : 0.;
-      }
-    } else {
-      const int k = k0 + nk;
-#pragma unroll
-      for (int q = 0; q < JG; ++q) {
-        const int c = c0 + nc + 32 * q;
-        pb[q] = (k < K && c < N) ? B[int64_t(k) * ldb + c] : 0.;
-      }
-    }
-  };
-  auto store = [&](int buf) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) As[buf][lk + q][lr] = pa[q];
-    if (B_NT) {
-#pragma unroll
-      for (int q = 0; q < BK_T; ++q) Bs[buf][bk + q][br] = pb[q];
-    } else {
-#pragma unroll
-      for (int q = 0; q < JG; ++q) Bs[buf][nk][nc + 32 * q] = pb[q];
-    }
-  };
-  double acc[8][2 * JG];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 2 * JG; ++j) acc[i][j] = 0.;
-  load(0);
-  store(0);
-  __syncthreads();
-  int buf = 0;
-  for (int k0 = 0; k0 < K; k0 += kDgBK) {
-    const bool more = k0 + kDgBK < K;
-    if (more) load(k0 + kDgBK);
-#pragma unroll
-    for (int kk = 0; kk < kDgBK; ++kk) {
-      double a[8], b[2 * JG];
-      const double2 * ar = reinterpret_cast<const double2 *>(&As[buf][kk][0]);
-      const double2 * bs = reinterpret_cast<const double2 *>(&Bs[buf][kk][0]);
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        const double2 va = ar[16 * g + ty];
-        a[2 * g] = va.x, a[2 * g + 1] = va.y;
-      }
-#pragma unroll
-      for (int g = 0; g < JG; ++g) {
-        const double2 vb = bs[16 * g + tx];
-        b[2 * g] = vb.x, b[2 * g + 1] = vb.y;
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 2 * JG; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    if (more) {
-      store(buf ^ 1);
-      __syncthreads();
-      buf ^= 1;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int64_t r = r0 + 32 * (i >> 1) + 2 * ty + (i & 1);
-    if (r >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 2 * JG; ++j) {
-      const int c = c0 + 32 * (j >> 1) + 2 * tx + (j & 1);
-      if (c < N) epi(r, c, acc[i][j]);
-    }
-  }
+template <class ARows, class Epi>
+struct DgProblem {
+  int64_t M;
+  int N, K;
+  const double * A;
+  ARows arows;
+  const double * B;
+  int64_t ldb;
+  Epi epi;
+};
+template <class ARows, class Epi>
+struct DgGroup {
+  int n, splits;
+  int64_t tile_end[kDgMaxProblems];  // running tile counts
+  DgProblem<ARows, Epi> p[kDgMaxProblems];
+};
+
+__device__ __forceinline__ void dg_cp(double * smem, const double * gmem, int bytes, int full) {
+  const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  // bytes < full: the rest is filled with zeros
+  if (full == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void dmma(double * c, const double * a, const double * b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-template <bool B_NT, class ARows, class Epi, int BN = kDgBN>
-void launch_dgemm(int64_t M, int N, int K, const double * A, ARows arows, const double * B, int64_t ldb,
-                  Epi epi, cudaStream_t st) {
-  if (M <= 0 || N <= 0) return;
-  const int64_t row_tiles = (M + kDgBM - 1) / kDgBM;
-  const int col_tiles = div_up(N, BN);
-  if (row_tiles > 65535 || col_tiles > 0x7fffffff)
-    throw Error(RGPU_ERR_CAPACITY, "FP64 GEMM: too many rows for one launch");
-  const dim3 grid{static_cast<unsigned>(col_tiles), static_cast<unsigned>(row_tiles), 1u};
-  dgemm_kernel<B_NT, BN><<<grid, 256, 0, st>>>(M, N, K, A, arows, B, ldb, epi);
+// VEC: doubles per copy, 2 when every row of both operands starts on a
+// 16-byte boundary, else 1.
+template <bool B_NT, int VEC, class ARows, class Epi>
+__global__ void __launch_bounds__(kDgThreads)
+dgemm_kernel(const __grid_constant__ DgGroup<ARows, Epi> g) {
+  extern __shared__ __align__(16) double dsm[];
+  constexpr int kFull = 8 * VEC;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const int gid = lane >> 2, tig = lane & 3;
+  const int split = int(blockIdx.x % unsigned(g.splits));
+  const int64_t tile = blockIdx.x / unsigned(g.splits);
+  int pi = 0;
+  while (tile >= g.tile_end[pi]) ++pi;
+  const DgProblem<ARows, Epi> & p = g.p[pi];
+  const int64_t local = tile - (pi ? g.tile_end[pi - 1] : 0);
+  // column tiles vary fastest: the blocks that share an A row tile run
+  // together, so A comes from DRAM once and the others read it from L2
+  const int tiles_n = (p.N + kDgBN - 1) / kDgBN;
+  const int64_t r0 = local / tiles_n * kDgBM;
+  const int c0 = int(local % tiles_n) * kDgBN;
+  const int slices = (p.K + kDgBK - 1) / kDgBK, per = (slices + g.splits - 1) / g.splits;
+  const int k_lo = min(split * per, slices) * kDgBK, k_hi = min(min((split + 1) * per, slices) * kDgBK, p.K);
+
+  // copies: `kRow` threads side by side on a row of 16 k, rows kRows apart
+  constexpr int kRow = kDgBK / VEC, kRows = kDgThreads / kRow, kCopies = kDgBM / kRows;
+  const int lr = t / kRow, lk = (t % kRow) * VEC;
+  int64_t a_off[kCopies], b_off[kCopies];
+#pragma unroll
+  for (int q = 0; q < kCopies; ++q) {
+    const int64_t r = r0 + lr + q * kRows;
+    a_off[q] = r < p.M ? p.arows(r) : int64_t(-1);
+    const int c = c0 + lr + q * kRows;
+    b_off[q] = c < p.N ? int64_t(c) * p.ldb : int64_t(-1);
+  }
+  // the K x N tile: kCol threads side by side on a row of 64 columns
+  constexpr int kCol = kDgBN / VEC, kColRows = kDgThreads / kCol, kColCopies = kDgBK / kColRows;
+  const int nk = t / kCol, nc = (t % kCol) * VEC;
+
+  auto load = [&](int stage, int k0) {
+    double * as = dsm + stage * (kDgStageA + kDgStageB);
+    double * bs = as + kDgStageA;
+    const int kb = max(0, min(kFull, 8 * (k_hi - (k0 + lk))));
+#pragma unroll
+    for (int q = 0; q < kCopies; ++q) {
+      const int n = a_off[q] >= 0 ? kb : 0;
+      dg_cp(as + (lr + q * kRows) * kDgLdK + lk, n ? p.A + a_off[q] + k0 + lk : p.A, n, kFull);
+    }
+    if (B_NT) {
+#pragma unroll
+      for (int q = 0; q < kCopies; ++q) {
+        const int n = b_off[q] >= 0 ? kb : 0;
+        dg_cp(bs + (lr + q * kRows) * kDgLdK + lk, n ? p.B + b_off[q] + k0 + lk : p.B, n, kFull);
+      }
+    } else {
+      const int cb = max(0, min(kFull, 8 * (p.N - (c0 + nc))));
+#pragma unroll
+      for (int q = 0; q < kColCopies; ++q) {
+        const int k = k0 + nk + q * kColRows;
+        const int n = k < k_hi ? cb : 0;
+        dg_cp(bs + (nk + q * kColRows) * kDgLdN + nc, n ? p.B + int64_t(k) * p.ldb + c0 + nc : p.B, n, kFull);
+      }
+    }
+  };
+
+  double acc[2][4][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) acc[i][j][v] = 0.;
+  const int wm = (wid >> 1) * 32, wn = (wid & 1) * 32;
+  const int iters = k_hi > k_lo ? (k_hi - k_lo + kDgBK - 1) / kDgBK : 0;
+#pragma unroll
+  for (int s = 0; s < kDgStages - 1; ++s) {
+    if (s < iters) load(s, k_lo + s * kDgBK);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  int stage = 0;
+  for (int it = 0; it < iters; ++it) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kDgStages - 2) : "memory");
+    __syncthreads();  // slice `it` has landed for every thread; the slice before it is read no more
+    {
+      const int nxt = it + kDgStages - 1;
+      if (nxt < iters) load(nxt % kDgStages, k_lo + nxt * kDgBK);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    const double * as = dsm + stage * (kDgStageA + kDgStageB);
+    const double * bs = as + kDgStageA;
+    stage = stage + 1 == kDgStages ? 0 : stage + 1;
+#pragma unroll
+    for (int kk = 0; kk < kDgBK; kk += 8) {
+      double a[2][4], b[4][2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const double * q = as + (wm + 16 * i + gid) * kDgLdK + kk + tig;
+        a[i][0] = q[0];
+        a[i][1] = q[8 * kDgLdK];
+        a[i][2] = q[4];
+        a[i][3] = q[8 * kDgLdK + 4];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (B_NT) {
+          const double * q = bs + (wn + 8 * j + gid) * kDgLdK + kk + tig;
+          b[j][0] = q[0];
+          b[j][1] = q[4];
+        } else {
+          const double * q = bs + (kk + tig) * kDgLdN + wn + 8 * j + gid;
+          b[j][0] = q[0];
+          b[j][1] = q[4 * kDgLdN];
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dmma(acc[i][j], a[i], b[j]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int64_t r = r0 + wm + 16 * i + gid + 8 * (v >> 1);
+        const int c = c0 + wn + 8 * j + 2 * tig + (v & 1);
+        if (r < p.M && c < p.N) p.epi(r, c, acc[i][j][v], split);
+      }
+}
+
+// Splits of K that bring `tiles` tiles to about three blocks per SM (what
+// the ring's shared memory lets be resident), each at least 4 slices deep.
+inline int dgemm_splits(int64_t tiles, int K) {
+  if (tiles <= 0) return 1;
+  const int64_t want = std::max<int64_t>(1, 3 * 148 / tiles);
+  return int(std::min<int64_t>({want, std::max(1, K / (4 * kDgBK)), 32}));
+}
+inline int64_t dgemm_tiles(int64_t M, int N) {
+  return ((M + kDgBM - 1) / kDgBM) * int64_t((N + kDgBN - 1) / kDgBN);
+}
+
+// Launches the group (p[0..n) filled); `aligned` says that every row of A
+// and B starts on a 16-byte boundary.
+template <bool B_NT, class ARows, class Epi>
+void launch_dgemm(DgGroup<ARows, Epi> & g, bool aligned, cudaStream_t st) {
+  int64_t tiles = 0;
+  for (int i = 0; i < g.n; ++i) {
+    tiles += dgemm_tiles(g.p[i].M, g.p[i].N);
+    g.tile_end[i] = tiles;
+  }
+  if (tiles == 0) return;
+  if (tiles * g.splits > 0x7fffffff) throw Error(RGPU_ERR_CAPACITY, "FP64 GEMM: too many rows for one launch");
+  auto kernel = aligned ? dgemm_kernel<B_NT, 2, ARows, Epi> : dgemm_kernel<B_NT, 1, ARows, Epi>;
+  RGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kDgSmem)));
+  kernel<<<unsigned(tiles * g.splits), kDgThreads, kDgSmem, st>>>(g);
   RGPU_LAUNCHED();
   RGPU_CUDA(cudaGetLastError());
+}
+
+inline bool dgemm_aligned(const void * p, int64_t ld) {
+  return (ld & 1) == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
 }
 
 }  // namespace rgpu

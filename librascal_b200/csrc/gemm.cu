@@ -7,8 +7,7 @@
 // models/sparse_kernel_predict.hh:141-143, done for all centres at once).
 //
 // Two implementations:
-//  * FP64 SIMT tiles for the plain path (the reference's arithmetic,
-//    dgemm.cuh);
+//  * FP64 tensor-core tiles for the plain path (dgemm.cuh);
 //  * TF32 tensor-core tiles (mma.sync m16n8k8) with FP32 accumulation for
 //    the fast path, optionally as a 3-term split (hi*hi + hi*lo + lo*hi) that
 //    carries ~21 mantissa bits. The forward epilogue fuses k^zeta, the
@@ -27,21 +26,25 @@ __device__ __forceinline__ float pow_zeta_f(float v, int z) {
   return r;
 }
 
-__global__ void gap_pointwise_fp64_kernel(int64_t rows, int M, const double * __restrict__ Km,
-                                          int64_t ldk, const double * __restrict__ alpha, int zeta,
-                                          double * __restrict__ W, int64_t ldw,
-                                          double * __restrict__ e_row) {
-  int64_t r = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (r >= rows) return;
+// One warp per row of the sorted features; adds the planes of the dots.
+__global__ void gap_pointwise_fp64_kernel(GapGroup g, double * __restrict__ Km, const double * __restrict__ alpha,
+                                          int zeta, double * __restrict__ e_row) {
+  const int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (row >= g.row0[g.S]) return;
+  int s = 0;
+  while (row >= g.row0[s + 1]) ++s;
+  double * K = Km + g.koff[s] + (row - g.row0[s]) * g.ldk[s];
   double e = 0.;
-  for (int m = lane; m < M; m += 32) {
-    double k = Km[r * ldk + m];
-    e += alpha[m] * pow_zeta_d(k, zeta);
-    W[r * ldw + m] = alpha[m] * (zeta * pow_zeta_d(k, zeta - 1));
+  for (int m = lane; m < g.M[s]; m += 32) {
+    double k = K[m];
+    for (int p = 1; p < g.splits; ++p) k += K[p * g.plane + m];
+    const double al = alpha[g.m0[s] + m];
+    e += al * pow_zeta_d(k, zeta);
+    K[m] = al * (zeta * pow_zeta_d(k, zeta - 1));
   }
   e = warp_sum(e);
-  if (lane == 0) e_row[r] = e;
+  if (lane == 0) e_row[row] = e;
 }
 
 // ------------------------------------------------------ TF32 tensor-core GEMM
@@ -316,19 +319,48 @@ __global__ void pair_center2_kernel(int64_t c0, int64_t c1, const int64_t * __re
 
 void gemm_nt_fp64(int64_t M, int64_t N, int64_t K, const double * A, int64_t lda, const double * B,
                   int64_t ldb, double * C, int64_t ldc, cudaStream_t st) {
-  launch_dgemm<true>(M, int(N), int(K), A, DgPlainRows{lda}, B, ldb, DgStoreC{C, ldc}, st);
-}
-void gemm_nn_fp64(int64_t M, int64_t N, int64_t K, const double * A, int64_t lda, const double * B,
-                  int64_t ldb, double * C, int64_t ldc, cudaStream_t st) {
-  launch_dgemm<false>(M, int(N), int(K), A, DgPlainRows{lda}, B, ldb, DgStoreC{C, ldc}, st);
+  DgGroup<DgPlainRows, DgStoreC> g{};
+  g.n = g.splits = 1;
+  g.p[0] = {M, int(N), int(K), A, DgPlainRows{lda}, B, ldb, DgStoreC{C, ldc, 0}};
+  launch_dgemm<true>(g, dgemm_aligned(A, lda) && dgemm_aligned(B, ldb), st);
 }
 
-void launch_gap_pointwise_fp64(int64_t rows, int M, const double * Kmat, int64_t ldk,
-                               const double * alpha, int zeta, double * W, int64_t ldw,
-                               double * e_row, cudaStream_t st) {
-  if (rows <= 0) return;
-  gap_pointwise_fp64_kernel<<<div_up(rows * 32, 256), 256, 0, st>>>(rows, M, Kmat, ldk, alpha, zeta,
-                                                                   W, ldw, e_row);
+void gap_dots_split(GapGroup & g, int K) {
+  int64_t tiles = 0;
+  for (int s = 0; s < g.S; ++s)
+    if (g.M[s] > 0) tiles += dgemm_tiles(g.rows[s], g.M[s]);
+  g.splits = dgemm_splits(tiles, K);
+}
+
+void launch_gap_dots_fp64(const GapGroup & g, int K, const double * X, int64_t ldx, const double * T, int64_t ldt,
+                          double * Kmat, cudaStream_t st) {
+  DgGroup<DgPlainRows, DgStoreC> d{};
+  d.splits = g.splits;
+  for (int s = 0; s < g.S; ++s)
+    if (g.rows[s] > 0 && g.M[s] > 0)
+      d.p[d.n++] = {g.rows[s], g.M[s], K, X + g.row0[s] * ldx, DgPlainRows{ldx}, T + g.m0[s] * ldt, ldt,
+                    DgStoreC{Kmat + g.koff[s], g.ldk[s], g.plane}};
+  launch_dgemm<true>(d, dgemm_aligned(X, ldx) && dgemm_aligned(T, ldt), st);
+}
+
+void launch_gap_scaled_fp64(const GapGroup & g, int D, const double * W, const double * T, int64_t ldt, double * t,
+                            int64_t ld, cudaStream_t st) {
+  DgGroup<DgPlainRows, DgStoreC> d{};
+  d.splits = 1;
+  bool aligned = dgemm_aligned(W, 0) && dgemm_aligned(T, ldt);
+  for (int s = 0; s < g.S; ++s)
+    if (g.rows[s] > 0 && g.M[s] > 0) {
+      aligned = aligned && (g.koff[s] & 1) == 0;
+      d.p[d.n++] = {g.rows[s], D, g.M[s], W + g.koff[s], DgPlainRows{g.ldk[s]}, T + g.m0[s] * ldt, ldt,
+                    DgStoreC{t + g.row0[s] * ld, ld, 0}};
+    }
+  launch_dgemm<false>(d, aligned, st);
+}
+
+void launch_gap_pointwise_fp64(const GapGroup & g, double * Kmat, const double * alpha, int zeta, double * e_row,
+                               cudaStream_t st) {
+  if (g.row0[g.S] <= 0) return;
+  gap_pointwise_fp64_kernel<<<div_up(g.row0[g.S] * 32, 256), 256, 0, st>>>(g, Kmat, alpha, zeta, e_row);
   RGPU_LAUNCHED();
 }
 

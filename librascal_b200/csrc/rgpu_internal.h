@@ -350,15 +350,32 @@ struct GapSpecies {
   int64_t row0, rows;  // species segment in the sorted row order
   int m0, M, Mpad;     // sparse points of this species (global index m0..m0+M)
 };
-// FP64 plain GEMMs: K = X T^T (per species), energies, W, t = W T.
+// The FP64 contractions of all central species in one launch each
+// (dgemm.cuh). Species s has rows row0[s] .. row0[s] + rows[s] of the
+// species-sorted features and sparse points m0[s] .. m0[s] + M[s]; its block
+// of the kernel matrix starts at koff[s] with rows ldk[s] = M[s] rounded up
+// to even apart. The dots come in `splits` planes of `plane` values (partial
+// sums over K) that their reader adds.
+struct GapGroup {
+  int S{0}, splits{1};
+  int64_t plane{0};
+  int64_t row0[17]{}, rows[16]{}, koff[16]{};
+  int M[16]{}, m0[16]{}, ldk[16]{};
+};
+// Splits of K for the dots of a group (sets g.splits).
+void gap_dots_split(GapGroup & g, int K);
+// K = X_s T_s^T.
+void launch_gap_dots_fp64(const GapGroup & g, int K, const double * X, int64_t ldx, const double * T, int64_t ldt,
+                          double * Kmat, cudaStream_t st);
+// t_s = W_s T_s (W in plane 0 of the kernel matrix).
+void launch_gap_scaled_fp64(const GapGroup & g, int D, const double * W, const double * T, int64_t ldt, double * t,
+                            int64_t ld, cudaStream_t st);
+// k -> (e_row = sum alpha k^zeta, W = alpha zeta k^(zeta-1) into plane 0).
+void launch_gap_pointwise_fp64(const GapGroup & g, double * Kmat, const double * alpha, int zeta, double * e_row,
+                               cudaStream_t st);
+// One FP64 GEMM C = A B^T.
 void gemm_nt_fp64(int64_t M, int64_t N, int64_t K, const double * A, int64_t lda,
                   const double * B, int64_t ldb, double * C, int64_t ldc, cudaStream_t st);
-void gemm_nn_fp64(int64_t M, int64_t N, int64_t K, const double * A, int64_t lda,
-                  const double * B, int64_t ldb, double * C, int64_t ldc, cudaStream_t st);
-// k -> (e_row += alpha k^zeta, W = alpha zeta k^(zeta-1)) for FP64.
-void launch_gap_pointwise_fp64(int64_t rows, int M, const double * Kmat, int64_t ldk,
-                               const double * alpha, int zeta, double * W, int64_t ldw,
-                               double * e_row, cudaStream_t st);
 // TF32 tensor-core GEMM C = A B^T (both K-major) with optional GAP epilogue.
 struct Tf32GemmArgs {
   int64_t M, N, K;  // rows of A, rows of B, reduction length (multiple of 32)
@@ -447,13 +464,13 @@ void launch_force_contract_fp64(const FeatureDims & fd, int64_t c0, int64_t c1, 
                                 const double * pair_dist = nullptr, const double * pair_dir = nullptr,
                                 const int32_t * center_struct = nullptr, double * stress = nullptr);
 // ------------------------------------------------------------------ training
-// K_NM energy rows from K = X_s T_s^T (rows x M): k^zeta into row
-// center_of_row[row0 + r] (atom target) or added into its structure's row.
-void launch_knm_rows(int64_t rows, int M, const double * K, int zeta, const int32_t * center_of_row,
-                     int64_t row0, const int32_t * center_struct, bool atom_target, const int32_t * ucol,
-                     double * out, int64_t ldo, cudaStream_t st);
-// K <- zeta K^(zeta-1) (1 for zeta = 1), in place.
-void launch_kernel_weight(int64_t n, double * K, int zeta, cudaStream_t st);
+// K_NM energy rows from the dots of every species: k^zeta into row
+// center_of_row[row] (atom target) or added into its structure's row.
+void launch_knm_rows(const GapGroup & g, const double * K, int zeta, const int32_t * center_of_row,
+                     const int32_t * center_struct, bool atom_target, const int32_t * ucol, double * out, int64_t ldo,
+                     cudaStream_t st);
+// W = zeta k^(zeta-1) (1 for zeta = 1), in place (plane 0).
+void launch_kernel_weight(const GapGroup & g, double * K, int zeta, cudaStream_t st);
 // K_MM block of one species: out[ucol[a]][ucol[b]] = K[a][b]^zeta.
 void launch_kmm_scatter(int M, const double * K, int zeta, const int32_t * ucol, double * out, int64_t ldo,
                         cudaStream_t st);
@@ -466,7 +483,8 @@ struct KnmDerArgs {
   const double * T;  // sparse points of the species, M rows of stride ldt
   int64_t ldt;
   int M;
-  const double * W;  // zeta k^(zeta-1) of the species' rows, [row - row0][M]
+  const double * W;  // zeta k^(zeta-1) of the species' rows, [row - row0][ldw]
+  int64_t ldw;
   int64_t row0;
   const int32_t * row_of_center;
   const int32_t * pair_j;
@@ -490,6 +508,7 @@ struct KnmStressArgs {
   int64_t ldt;
   int M;
   const double * W;
+  int64_t ldw;
   int64_t row0;
   const int32_t * row_of_center;
   const int32_t * center_struct;

@@ -23,29 +23,42 @@
 namespace rgpu {
 namespace {
 
-__global__ void knm_rows_kernel(int64_t rows, int M, const double * __restrict__ K, int zeta,
-                                const int32_t * __restrict__ center_of_row, int64_t row0,
+// One warp per row of the sorted features; adds the planes of the dots.
+__global__ void knm_rows_kernel(GapGroup g, const double * __restrict__ Km, int zeta,
+                                const int32_t * __restrict__ center_of_row,
                                 const int32_t * __restrict__ center_struct, int atom_target,
-                                const int32_t * __restrict__ ucol, double * __restrict__ out,
-                                int64_t ldo) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= rows * M) return;
-  const int64_t r = i / M;
-  const int m = int(i - r * M);
-  const double v = pow_zeta_d(K[i], zeta);
-  const int64_t ci = center_of_row[row0 + r];
-  if (atom_target)
-    out[ci * ldo + ucol[m]] = v;
-  else
-    atomicAdd(&out[int64_t(center_struct[ci]) * ldo + ucol[m]], v);
+                                const int32_t * __restrict__ ucol, double * __restrict__ out, int64_t ldo) {
+  const int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  if (row >= g.row0[g.S]) return;
+  int s = 0;
+  while (row >= g.row0[s + 1]) ++s;
+  const double * K = Km + g.koff[s] + (row - g.row0[s]) * g.ldk[s];
+  const int64_t ci = center_of_row[row];
+  double * o = out + (atom_target ? ci : int64_t(center_struct[ci])) * ldo;
+  for (int m = threadIdx.x & 31; m < g.M[s]; m += 32) {
+    double k = K[m];
+    for (int p = 1; p < g.splits; ++p) k += K[p * g.plane + m];
+    const double v = pow_zeta_d(k, zeta);
+    if (atom_target)
+      o[ucol[g.m0[s] + m]] = v;
+    else
+      atomicAdd(&o[ucol[g.m0[s] + m]], v);
+  }
 }
 
 // W = zeta k^(zeta-1); exactly 1 for zeta = 1, where the reference skips the
 // factor (models/sparse_kernels.hh:320-331, :393-396).
-__global__ void kernel_weight_kernel(int64_t n, double * __restrict__ K, int zeta) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  K[i] = zeta > 1 ? double(zeta) * pow_zeta_d(K[i], zeta - 1) : 1.;
+__global__ void kernel_weight_kernel(GapGroup g, double * __restrict__ Km, int zeta) {
+  const int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  if (row >= g.row0[g.S]) return;
+  int s = 0;
+  while (row >= g.row0[s + 1]) ++s;
+  double * K = Km + g.koff[s] + (row - g.row0[s]) * g.ldk[s];
+  for (int m = threadIdx.x & 31; m < g.M[s]; m += 32) {
+    double k = K[m];
+    for (int p = 1; p < g.splits; ++p) k += K[p * g.plane + m];
+    K[m] = zeta > 1 ? double(zeta) * pow_zeta_d(k, zeta - 1) : 1.;
+  }
 }
 
 __global__ void kmm_scatter_kernel(int M, const double * __restrict__ K, int zeta,
@@ -73,16 +86,16 @@ struct PairScatter {
   int64_t p_base, row0;
   const int32_t * row_of_center;
   const double * W;
-  int M;
+  int64_t ldw;
   const int32_t * pair_j;
   const int32_t * ucol;
   double * out;
   int64_t ldo;
-  __device__ __forceinline__ void operator()(int64_t r, int m, double v) const {
+  __device__ __forceinline__ void operator()(int64_t r, int m, double v, int) const {
     const int64_t k = r / 3;
     const int c = int(r - 3 * k);
     const int64_t ci = list[2 * k + 1];
-    const double w = W[(int64_t(row_of_center[ci]) - row0) * M + m];
+    const double w = W[(int64_t(row_of_center[ci]) - row0) * ldw + m];
     const int64_t j = pair_j[p_base + list[2 * k]];
     atomicAdd(&out[(3 * j + c) * ldo + ucol[m]], v * w);
   }
@@ -95,16 +108,16 @@ struct StressScatter {
   int64_t row0, stress_row0;
   const int32_t * row_of_center;
   const double * W;
-  int M;
+  int64_t ldw;
   const int32_t * center_struct;
   const int32_t * ucol;
   double * out;
   int64_t ldo;
-  __device__ __forceinline__ void operator()(int64_t r, int m, double v) const {
+  __device__ __forceinline__ void operator()(int64_t r, int m, double v, int) const {
     const int64_t k = r / 6;
     const int e = int(r - 6 * k);
     const int64_t ci = centres[k];
-    const double w = W[(int64_t(row_of_center[ci]) - row0) * M + m];
+    const double w = W[(int64_t(row_of_center[ci]) - row0) * ldw + m];
     atomicAdd(&out[(stress_row0 + 6 * int64_t(center_struct[ci]) + e) * ldo + ucol[m]], v * w);
   }
 };
@@ -159,19 +172,19 @@ virial_rows_kernel(const int32_t * __restrict__ centres, int64_t n, const int64_
 
 }  // namespace
 
-void launch_knm_rows(int64_t rows, int M, const double * K, int zeta, const int32_t * center_of_row,
-                     int64_t row0, const int32_t * center_struct, bool atom_target, const int32_t * ucol,
-                     double * out, int64_t ldo, cudaStream_t st) {
-  if (rows <= 0 || M <= 0) return;
-  knm_rows_kernel<<<div_up(rows * M, 256), 256, 0, st>>>(rows, M, K, zeta, center_of_row, row0, center_struct,
-                                                        int(atom_target), ucol, out, ldo);
+void launch_knm_rows(const GapGroup & g, const double * K, int zeta, const int32_t * center_of_row,
+                     const int32_t * center_struct, bool atom_target, const int32_t * ucol, double * out, int64_t ldo,
+                     cudaStream_t st) {
+  if (g.row0[g.S] <= 0) return;
+  knm_rows_kernel<<<div_up(g.row0[g.S] * 32, 256), 256, 0, st>>>(g, K, zeta, center_of_row, center_struct,
+                                                                int(atom_target), ucol, out, ldo);
   RGPU_LAUNCHED();
   RGPU_CUDA(cudaGetLastError());
 }
 
-void launch_kernel_weight(int64_t n, double * K, int zeta, cudaStream_t st) {
-  if (n <= 0) return;
-  kernel_weight_kernel<<<div_up(n, 256), 256, 0, st>>>(n, K, zeta);
+void launch_kernel_weight(const GapGroup & g, double * K, int zeta, cudaStream_t st) {
+  if (g.row0[g.S] <= 0) return;
+  kernel_weight_kernel<<<div_up(g.row0[g.S] * 32, 256), 256, 0, st>>>(g, K, zeta);
   RGPU_LAUNCHED();
   RGPU_CUDA(cudaGetLastError());
 }
@@ -186,10 +199,11 @@ void launch_kmm_scatter(int M, const double * K, int zeta, const int32_t * ucol,
 
 void launch_knm_derivative(const KnmDerArgs & a, cudaStream_t st) {
   if (a.n_list <= 0 || a.M <= 0) return;
-  PairScatter epi{a.list, a.p_base, a.row0, a.row_of_center, a.W, a.M, a.pair_j, a.ucol, a.out, a.ldo};
-  // 128 x 64 tiles: two blocks per SM (3 % faster than 128 x 128 here)
-  launch_dgemm<true, PairRows, PairScatter, 64>(3 * a.n_list, a.M, a.D, a.dX, PairRows{a.list, a.D}, a.T, a.ldt,
-                                                epi, st);
+  PairScatter epi{a.list, a.p_base, a.row0, a.row_of_center, a.W, a.ldw, a.pair_j, a.ucol, a.out, a.ldo};
+  DgGroup<PairRows, PairScatter> g{};
+  g.n = g.splits = 1;
+  g.p[0] = {3 * a.n_list, a.M, a.D, a.dX, PairRows{a.list, a.D}, a.T, a.ldt, epi};
+  launch_dgemm<true>(g, dgemm_aligned(a.dX, a.D) && dgemm_aligned(a.T, a.ldt), st);
 }
 
 void launch_knm_stress(const KnmStressArgs & a, cudaStream_t st) {
@@ -198,9 +212,12 @@ void launch_knm_stress(const KnmStressArgs & a, cudaStream_t st) {
                                                           a.pair_dist, a.pair_dir, a.dX, a.D, a.V);
   RGPU_LAUNCHED();
   RGPU_CUDA(cudaGetLastError());
-  StressScatter epi{a.centres, a.row0, a.stress_row0, a.row_of_center, a.W, a.M, a.center_struct, a.ucol,
+  StressScatter epi{a.centres, a.row0, a.stress_row0, a.row_of_center, a.W, a.ldw, a.center_struct, a.ucol,
                     a.out, a.ldo};
-  launch_dgemm<true>(6 * a.n_centres, a.M, a.D, a.V, DgPlainRows{a.D}, a.T, a.ldt, epi, st);
+  DgGroup<DgPlainRows, StressScatter> g{};
+  g.n = g.splits = 1;
+  g.p[0] = {6 * a.n_centres, a.M, a.D, a.V, DgPlainRows{a.D}, a.T, a.ldt, epi};
+  launch_dgemm<true>(g, dgemm_aligned(a.V, a.D) && dgemm_aligned(a.T, a.ldt), st);
 }
 
 }  // namespace rgpu
