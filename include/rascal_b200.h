@@ -61,7 +61,7 @@ typedef struct rgpu_gap_model rgpu_gap_model;
 
 /* Arithmetic of a compute call. */
 enum {
-  RGPU_PRECISION_FP64 = 0, /* plain path: FP64 everywhere, reference data flow */
+  RGPU_PRECISION_FP64 = 0, /* FP64 everywhere, the reference's dense feature order */
   RGPU_PRECISION_FP32 = 1  /* fast path: FP32 features, BF16x3 tensor-core GEMMs, adjoint forces */
 };
 
@@ -208,10 +208,10 @@ rgpu_status rgpu_gap_model_create(rgpu_calculator * calc, int32_t n_species,
                                   rgpu_gap_model ** out);
 rgpu_status rgpu_gap_model_destroy(rgpu_gap_model * m);
 /* Energies (n_structures, baseline included) and forces (n_atoms x 3, FP64,
- * = -dE/dr). RGPU_PRECISION_FP64 runs the reference's own algorithm on the
- * GPU (materialised dX/dr contracted with the scaled sparse points);
- * RGPU_PRECISION_FP32 runs the adjoint path (dE/dC contracted with dC/dr
- * recomputed per pair). Either output may be NULL. */
+ * = -dE/dr). Both precisions contract dE/dC with dC/dr recomputed per pair
+ * instead of materialising dX/dr: RGPU_PRECISION_FP64 in FP64 throughout,
+ * RGPU_PRECISION_FP32 with FP32 features and BF16x3 tensor-core GEMMs.
+ * Either output may be NULL. */
 rgpu_status rgpu_gap_predict(rgpu_gap_model * m, rgpu_structures * s,
                              int precision, double * energies,
                              double * forces);
@@ -314,8 +314,8 @@ int64_t rgpu_kernel_launches(int reset);
 /* Device time (ms) of the stages of the last rgpu_gap_predict call, from
  * CUDA events on the structure set's stream: 0 = whole call, 1 = neighbour
  * list, 2 = expansion, 3 = power spectrum, 4 = forward GEMMs, 5 = backward
- * GEMMs, 6 = power-spectrum backward (plain path: the materialised gradient
- * chunks and their contraction), 7 = pair adjoint. After
+ * GEMMs, 6 = power-spectrum backward (FP64: with the pair adjoint), 7 = pair
+ * adjoint (FP32). After
  * rgpu_sparse_kernel_derivative: 0 = its device time after the features and
  * before the copy to the host, 4 = the zeta k^(zeta-1) GEMMs, 6 = the
  * gradient chunks (materialised dX/dr and the gathered GEMMs). */

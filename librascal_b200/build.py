@@ -41,6 +41,7 @@ SOURCES = [
     ("adjoint.cu", ["-DRGPU_ADJ_L0=7", "-DRGPU_ADJ_L1=9"], "adjoint_l7"),
     ("adjoint.cu", ["-DRGPU_ADJ_L0=10", "-DRGPU_ADJ_L1=11"], "adjoint_l10"),
     ("adjoint.cu", ["-DRGPU_ADJ_L0=12", "-DRGPU_ADJ_L1=12"], "adjoint_l12"),
+    ("adjoint_f64.cu", [], "adjoint_f64"),
     ("training.cu", [], "training"),
     ("api.cu", [], "api"),
     ("radial_gto.cpp", ["-Xcompiler", "-ffp-contract=off"], "radial_gto"),

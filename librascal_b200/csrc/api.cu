@@ -209,7 +209,7 @@ struct rgpu_structures {
   FeatureDims fd{};
   std::vector<int64_t> species_count;
   DevBuf row_of_center, center_of_row, species_count_d, sort_tmp, present, tile_mask;
-  DevBuf C64, X64, invn64, C32, X32, xscale32;  // xscale32[row] = 1/|p| (FP32 path)
+  DevBuf C64, X64, invn64, dC64, C32, X32, xscale32;  // xscale32[row] = 1/|p| (FP32 path)
   int feat_precision{-1};
   const rgpu_calculator * feat_calc{nullptr};
   bool feat_gradients{false};
@@ -807,8 +807,8 @@ GapGroup species_dots(rgpu_gap_model * m, rgpu_structures * s) {
   return g;
 }
 
-void gap_plain(rgpu_gap_model * m, rgpu_structures * s, double * E_d, double * grad_d, bool forces,
-               double * stress_d) {
+// FP64 prediction: energies, forces (F_d, = -dE/dr) and stress sums.
+void gap_plain(rgpu_gap_model * m, rgpu_structures * s, double * E_d, double * F_d, bool forces, double * stress_d) {
   rgpu_calculator * c = m->calc;
   const FeatureDims & fd = s->fd;
   const int64_t nc = s->nl.n_centers;
@@ -832,43 +832,16 @@ void gap_plain(rgpu_gap_model * m, rgpu_structures * s, double * E_d, double * g
   mark(s, 5);
   mark(s, 6);
   if (!forces) return;
-  // gradients, chunked by a memory budget: materialised d c/d r and d x/d r
-  const size_t per_pair = sizeof(double) * (3 * size_t(fd.D) + 3 * size_t(fd.nK));
-  const size_t per_center = sizeof(double) * size_t(fd.S) * 3 * fd.nK;
-  const size_t budget = plain_budget_bytes();
-  ExpansionArgs ea = exp_args(c, s);
   PsArgs pa;
   pa.fd = fd;
   pa.n_centers = nc;
   pa.normalize = c->hy.normalize;
   pa.row_of_center = s->row_of_center.as<int32_t>();
-  const std::vector<int64_t> & poff = pair_offsets_host(s);
-  int64_t c0 = 0;
-  while (c0 < nc) {
-    int64_t c1 = c0;
-    size_t bytes = 0;
-    while (c1 < nc) {
-      size_t add = per_pair * size_t(poff[c1 + 1] - poff[c1]) + per_center;
-      if (c1 > c0 && bytes + add > budget) break;
-      bytes += add;
-      ++c1;
-    }
-    const int64_t p_base = poff[c0];
-    const int64_t np = poff[c1] - p_base;
-    s->dCp.ensure(sizeof(double) * size_t(np) * 3 * fd.nK + 64);
-    s->dCs.ensure(per_center * size_t(c1 - c0) + 64);
-    s->dXp.ensure(sizeof(double) * size_t(np) * 3 * fd.D + 64);
-    launch_expansion_grad_fp64(ea, c0, c1, p_base, s->dCp.as<double>(), st);
-    launch_expansion_selfgrad_fp64(ea, c0, c1, p_base, s->dCp.as<double>(), s->dCs.as<double>(), st);
-    launch_ps_grad_fp64(pa, ea, c0, c1, p_base, s->C64.as<double>(), s->X64.as<double>(),
-                        s->invn64.as<double>(), s->dCp.as<double>(), s->dCs.as<double>(),
-                        s->dXp.as<double>(), st);
-    launch_force_contract_fp64(fd, c0, c1, p_base, s->nl.pair_off, s->nl.pair_j,
-                               s->row_of_center.as<int32_t>(), s->dXp.as<double>(), s->t64.as<double>(),
-                               fd.Dpad, grad_d, st, s->nl.pair_dist, s->nl.pair_dir, s->nl.center_struct,
-                               stress_d);
-    c0 = c1;
-  }
+  pa.present = s->present.as<uint32_t>();
+  s->dC64.ensure(sizeof(double) * size_t(nc) * fd.S * fd.nK + 64);
+  launch_adjoint_fp64(pa, exp_args(c, s), s->C64.as<double>(), s->X64.as<double>(), s->invn64.as<double>(),
+                      s->t64.as<double>(), s->dC64.as<double>(), s->nl.pair_center, s->nl.n_pairs, F_d,
+                      s->nl.center_struct, stress_d, st);
   mark(s, 7);
 }
 
@@ -1159,8 +1132,6 @@ static void gap_predict_impl(rgpu_gap_model * m, rgpu_structures * s, int precis
       const std::vector<double> y0 = structure_baselines(m, s);
       for (int st = 0; st < s->n_struct; ++st) energies[st] += y0[st];
     }
-    if (forces && precision == RGPU_PRECISION_FP64)
-      for (int64_t i = 0; i < 3 * na; ++i) forces[i] = -forces[i];
     if (neg_stress)
       for (int st = 0; st < s->n_struct; ++st) {
         const double v = cell_volume(&s->cells_h[9 * size_t(st)]);
@@ -1485,7 +1456,7 @@ static std::vector<const void *> md_buffers(const rgpu_gap_model * m, const rgpu
                            &s->ncent_d, &s->center_off_d, &s->atom_struct_d, &s->lut, &s->row_of_center,
                            &s->center_of_row, &s->species_count_d, &s->sort_tmp, &s->present, &s->tile_mask,
                            &s->C64, &s->X64,
-                           &s->invn64, &s->C32, &s->X32, &s->xscale32, &s->E_d, &s->F_d, &s->S_d, &s->K64,
+                           &s->invn64, &s->dC64, &s->C32, &s->X32, &s->xscale32, &s->E_d, &s->F_d, &s->S_d, &s->K64,
                            &s->t64, &s->erow64, &s->Wh, &s->Wl, &s->dX32, &s->dC32, &s->epart, &s->Xh, &s->Xl,
                            &s->chunk_map, &s->dCp, &s->dCs, &s->dXp, &s->knm, &s->plist, &s->Vvir})
     v.push_back(b->p);

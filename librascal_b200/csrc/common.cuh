@@ -58,6 +58,57 @@ __device__ __forceinline__ double rs_grad(const RadialScalingDev & p, double r) 
   return -p.rate * p.exponent * ff / r / (d * d);
 }
 
+// cos(x) for x within 0.02 of pi, correctly rounded: -cos(pi - x) by its
+// Taylor series in double-double (pi - x is exact by Sterbenz' lemma plus the
+// low word of pi). The switching function needs it because 1 + cos(x)
+// cancels there: an ulp of difference between two libm's cos becomes a
+// relative error of ulp / f_c in f_c.
+__device__ __forceinline__ double cos_near_pi(double x) {
+  const double pi_hi = 3.141592653589793116, pi_lo = 1.2246467991473532e-16;
+  double th = pi_hi - x;
+  double s = th + pi_lo;
+  double tl = pi_lo - (s - th);
+  th = s;
+  double u = th * th;
+  double ue = fma(th, th, -u) + 2.0 * th * tl;
+  double h = u * 0.5, hl = ue * 0.5;
+  double c = 1.0 - h;
+  double ce = ((1.0 - c) - h) - hl;
+  double tail = u * u * (1.0 / 24.0) - u * u * u * (1.0 / 720.0) + u * u * u * u * (1.0 / 40320.0);
+  return -(c + (ce + tail));
+}
+
+__device__ __forceinline__ double fc_cos(double r, double rc, double sw) {
+  if (r <= (rc - sw)) return 1.0;
+  if (r > rc) return 0.0;
+  double rs = 3.14159265358979323846264338327950288 * (r - rc + sw) / sw;
+  double c = (rs > 3.121592653589793) ? cos_near_pi(rs) : cos(rs);
+  return 0.5 * (1. + c);
+}
+__device__ __forceinline__ double dfc_cos(double r, double rc, double sw) {
+  if (r <= (rc - sw)) return 0.0;
+  if (r > rc) return 0.0;
+  double rs = 3.14159265358979323846264338327950288 * (r - rc + sw) / sw;
+  return -0.5 * 3.14159265358979323846264338327950288 / sw * sin(rs);
+}
+// the cutoff function of the calculator: shifted cosine, times the
+// RadialScaling factor when that is the cutoff type
+__device__ __forceinline__ double cutoff_fc(const ExpansionArgs & a, double r) {
+  const double s = fc_cos(r, a.rc, a.sw);
+  return a.rs.on ? rs_value(a.rs, r) * s : s;
+}
+__device__ __forceinline__ void cutoff_fc_dfc(const ExpansionArgs & a, double r, double & fc, double & dfc) {
+  const double s = fc_cos(r, a.rc, a.sw), ds = dfc_cos(r, a.rc, a.sw);
+  if (a.rs.on) {
+    const double u = rs_value(a.rs, r);
+    fc = u * s;
+    dfc = rs_grad(a.rs, r) * s + u * ds;
+  } else {
+    fc = s;
+    dfc = ds;
+  }
+}
+
 // v^zeta of the GAP kernel (models/kernels.hh:48-61)
 __device__ __forceinline__ double pow_zeta_d(double v, int z) {
   if (z == 0) return 1.;

@@ -260,61 +260,6 @@ __global__ void energy_reduce_kernel(int64_t rows, int n_parts, const float * __
   if (key >= 0 && leader == lane) atomicAdd(&E[key], sum);
 }
 
-// Plain path: gradients[j] += dX_i(pair) . t_i, one warp per pair.
-__global__ void force_contract_kernel(int64_t p_first, int64_t np, int D, int64_t p_base,
-                                      const int64_t * __restrict__ pair_center,
-                                      const int32_t * __restrict__ pair_j,
-                                      const int32_t * __restrict__ row_of_center,
-                                      const double * __restrict__ dX, const double * __restrict__ t,
-                                      int64_t ldt, double * __restrict__ grad,
-                                      const double * __restrict__ pair_dist,
-                                      const double * __restrict__ pair_dir,
-                                      const int32_t * __restrict__ center_struct,
-                                      double * __restrict__ stress) {
-  int64_t q = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (q >= np) return;
-  int64_t p = p_first + q;
-  int64_t ci = pair_center[q];
-  const double * tr = t + size_t(row_of_center[ci]) * ldt;
-  const double * g = dX + size_t(p - p_base) * 3 * D;
-  double s[3] = {0., 0., 0.};
-  for (int d = lane; d < D; d += 32) {
-    double tv = tr[d];
-    s[0] += g[d] * tv;
-    s[1] += g[D + d] * tv;
-    s[2] += g[2 * D + d] * tv;
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) s[c] = warp_sum(s[c]);
-  if (lane == 0) {
-    int64_t j = pair_j[p];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) atomicAdd(&grad[3 * j + c], s[c]);
-    // r_ji (x) dE_i/dr_j, Voigt xx yy zz yz xz xy
-    // (models/sparse_kernel_predict.hh:355-366); the self pair has r_ji = 0
-    if (stress && pair_dist[p] > 0.) {
-      const double r = pair_dist[p];
-      const double rx = -r * pair_dir[3 * p], ry = -r * pair_dir[3 * p + 1], rz = -r * pair_dir[3 * p + 2];
-      double * st = stress + 6 * size_t(center_struct[ci]);
-      atomicAdd(st + 0, rx * s[0]);
-      atomicAdd(st + 4, rz * s[0]);
-      atomicAdd(st + 1, ry * s[1]);
-      atomicAdd(st + 5, rx * s[1]);
-      atomicAdd(st + 2, rz * s[2]);
-      atomicAdd(st + 3, ry * s[2]);
-    }
-  }
-}
-
-__global__ void pair_center2_kernel(int64_t c0, int64_t c1, const int64_t * __restrict__ pair_off,
-                                    int64_t p_first, int64_t * __restrict__ pc) {
-  int64_t ci = c0 + int64_t(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5);
-  if (ci >= c1) return;
-  for (int64_t p = pair_off[ci] + (threadIdx.x & 31); p < pair_off[ci + 1]; p += 32)
-    pc[p - p_first] = ci;
-}
-
 }  // namespace
 
 void gemm_nt_fp64(int64_t M, int64_t N, int64_t K, const double * A, int64_t lda, const double * B,
@@ -390,32 +335,6 @@ void launch_energy_reduce(int64_t rows, int n_parts, const float * e_part, int64
   energy_reduce_kernel<<<div_up(rows, 256), 256, 0, st>>>(rows, n_parts, e_part, ld, e_row_fp64, row0,
                                                          center_of_row, center_struct, energies);
   RGPU_LAUNCHED();
-}
-
-void launch_force_contract_fp64(const FeatureDims & fd, int64_t c0, int64_t c1, int64_t p_base,
-                                const int64_t * pair_off, const int32_t * pair_j,
-                                const int32_t * row_of_center, const double * dX, const double * t,
-                                int64_t ldt, double * grad, cudaStream_t st, const double * pair_dist,
-                                const double * pair_dir, const int32_t * center_struct, double * stress) {
-  if (c1 <= c0) return;
-  int64_t p_first = 0, p_last = 0;
-  RGPU_CUDA(cudaMemcpyAsync(&p_first, pair_off + c0, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  RGPU_CUDA(cudaMemcpyAsync(&p_last, pair_off + c1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  RGPU_CUDA(cudaStreamSynchronize(st));
-  const int64_t np = p_last - p_first;
-  if (np <= 0) return;
-  // per host thread and per device: another device's buffer is not memory this launch may use
-  static thread_local PerDevice<DevBuf> pc_tab;
-  DevBuf & pc = pc_tab.at(current_device());
-  pc.ensure(sizeof(int64_t) * np);
-  pair_center2_kernel<<<div_up(c1 - c0, 8), 256, 0, st>>>(c0, c1, pair_off, p_first, pc.as<int64_t>());
-  RGPU_LAUNCHED();
-  force_contract_kernel<<<div_up(np * 32, 256), 256, 0, st>>>(p_first, np, fd.D, p_base,
-                                                             pc.as<int64_t>(), pair_j, row_of_center,
-                                                             dX, t, ldt, grad, pair_dist, pair_dir,
-                                                             center_struct, stress);
-  RGPU_LAUNCHED();
-  RGPU_CUDA(cudaGetLastError());
 }
 
 }  // namespace rgpu

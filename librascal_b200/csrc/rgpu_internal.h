@@ -456,13 +456,14 @@ void launch_energy_reduce(int64_t rows, int n_parts, const float * e_part, int64
                           const double * e_row_fp64, int64_t row0, const int32_t * center_of_row,
                           const int32_t * center_struct, double * energies, cudaStream_t st);
 
-// Plain force contraction: grad[j] += dX[p] . t_i for pairs of centres [c0,c1).
-void launch_force_contract_fp64(const FeatureDims & fd, int64_t c0, int64_t c1, int64_t p_base,
-                                const int64_t * pair_off, const int32_t * pair_j,
-                                const int32_t * row_of_center, const double * dX,
-                                const double * t, int64_t ldt, double * grad, cudaStream_t st,
-                                const double * pair_dist = nullptr, const double * pair_dir = nullptr,
-                                const int32_t * center_struct = nullptr, double * stress = nullptr);
+// FP64 adjoint: dE/dc of every centre from the dE/dx rows t (reference order,
+// stride Dpad; ps.present: the FP64 expansion's species masks) into dC
+// [centre][lm][S n], then forces F (= -dE/dr) and, with stress, the unscaled
+// negative stress sums per structure from one pass over the pairs.
+void launch_adjoint_fp64(const PsArgs & ps, const ExpansionArgs & a, const double * C, const double * X,
+                         const double * inv_norm, const double * t, double * dC, const int32_t * pair_center,
+                         int64_t n_pairs, double * F, const int32_t * center_struct, double * stress,
+                         cudaStream_t st);
 // ------------------------------------------------------------------ training
 // K_NM energy rows from the dots of every species: k^zeta into row
 // center_of_row[row] (atom target) or added into its structure's row.

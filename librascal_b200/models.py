@@ -7,11 +7,11 @@ KRR.predict / predict_forces (models/krr.py:92-166) and
 compute_sparse_kernel_gradients (bind_py_models.cc:148-200). Energies and
 forces of a whole AtomsList come from one rgpu_gap_predict call:
 
-  precision="fp64"  the reference's own algorithm on the GPU (materialised
-                    dX/dr contracted with the scaled sparse points), FP64;
-  precision="fp32"  the adjoint path: FP32 expansion, TF32 tensor-core GEMMs
-                    with FP32 accumulation, dE/dC contracted with dC/dr
-                    recomputed per pair; FP64 energy reduction.
+  precision="fp64"  FP64 throughout, within 1e-10 of the reference: dE/dC
+                    contracted with dC/dr recomputed per pair;
+  precision="fp32"  the same adjoint in FP32: FP32 expansion, BF16x3
+                    tensor-core GEMMs with FP32 accumulation; FP64 energy
+                    reduction.
 
 PyTorch is used only by GAPEnergy (a torch.autograd.Function around the
 adjoint path) and is imported lazily.
