@@ -211,7 +211,8 @@ rgpu_status rgpu_gap_model_destroy(rgpu_gap_model * m);
  * = -dE/dr). Both precisions contract dE/dC with dC/dr recomputed per pair
  * instead of materialising dX/dr: RGPU_PRECISION_FP64 in FP64 throughout,
  * RGPU_PRECISION_FP32 with FP32 features and BF16x3 tensor-core GEMMs.
- * Either output may be NULL. */
+ * Either output may be NULL: with energies alone the force half is not run,
+ * with neither both are computed and left on the device. */
 rgpu_status rgpu_gap_predict(rgpu_gap_model * m, rgpu_structures * s,
                              int precision, double * energies,
                              double * forces);

@@ -167,7 +167,7 @@ struct PredictGraph {
   cudaGraph_t graph{nullptr};
   cudaGraphExec_t exec{nullptr};
   const rgpu_gap_model * model{nullptr};
-  bool stress{false}, outputs{false};
+  bool stress{false}, outputs{false}, forces{true};
   int n_struct{0};
   int64_t n_atoms{0};
   std::vector<int> species;
@@ -831,7 +831,10 @@ void gap_plain(rgpu_gap_model * m, rgpu_structures * s, double * E_d, double * F
                        s->nl.center_struct, E_d, st);
   mark(s, 5);
   mark(s, 6);
-  if (!forces) return;
+  if (!forces) {
+    mark(s, 7);
+    return;
+  }
   PsArgs pa;
   pa.fd = fd;
   pa.n_centers = nc;
@@ -893,9 +896,9 @@ void set_segments(Bf16x3Gemm & a, const rgpu_structures * s, const TileMaskArgs 
 }
 
 // Fast path, forward half: the grouped tcgen05 GEMM with the GAP epilogue
-// (energy partials and W = alpha zeta k^(zeta-1) as a BF16 pair), then the
-// per-structure energies (baseline not included).
-void gap_fast_forward(rgpu_gap_model * m, rgpu_structures * s, double * E_d) {
+// (energy partials and, for the backward half, W = alpha zeta k^(zeta-1) as
+// a BF16 pair), then the per-structure energies (baseline not included).
+void gap_fast_forward(rgpu_gap_model * m, rgpu_structures * s, double * E_d, bool need_w = true) {
   const FeatureDims & fd = s->fd;
   const int64_t nc = s->nl.n_centers;
   cudaStream_t st = s->st;
@@ -904,13 +907,13 @@ void gap_fast_forward(rgpu_gap_model * m, rgpu_structures * s, double * E_d) {
   // per-species W (BF16 hi/lo) and energy partial buffers
   int64_t wtot = 0, eparts = 0;
   for (int sI = 0; sI < fd.S; ++sI) {
-    wtot += s->species_count[sI] * m->segs[sI].Mpad;
+    if (need_w) wtot += s->species_count[sI] * m->segs[sI].Mpad;
     eparts += s->species_count[sI] * ((m->segs[sI].M + kTcTileN - 1) / kTcTileN);
   }
   s->Wh.ensure(sizeof(uint16_t) * size_t(std::max<int64_t>(wtot, 1)) + 64);
   s->Wl.ensure(sizeof(uint16_t) * size_t(std::max<int64_t>(wtot, 1)) + 64);
   s->epart.ensure(sizeof(float) * size_t(std::max<int64_t>(eparts, 1)) + 64);
-  s->dX32.ensure(sizeof(float) * size_t(nc) * fd.Dg + 64);
+  if (need_w) s->dX32.ensure(sizeof(float) * size_t(nc) * fd.Dg + 64);
   // species present in each 128-row tile (rows sorted by species and mask)
   const TileMaskArgs tm = tile_mask_args(s);
   if (fd.G > 1) {
@@ -939,8 +942,8 @@ void gap_fast_forward(rgpu_gap_model * m, rgpu_structures * s, double * E_d) {
       a.B_lo = m->Tl.as<__nv_bfloat16>() + size_t(g.m0) * fd.Dg;
       a.ldb = fd.Dg;
       a.epilogue = 1;
-      a.W_hi = Wh + wofs[sI];
-      a.W_lo = Wl + wofs[sI];
+      a.W_hi = need_w ? Wh + wofs[sI] : nullptr;
+      a.W_lo = need_w ? Wl + wofs[sI] : nullptr;
       a.ldw = g.Mpad;
       a.alpha = m->alpha32.as<float>() + g.m0;
       a.zeta = m->zeta;
@@ -1032,8 +1035,13 @@ void gap_fast_backward(rgpu_gap_model * m, rgpu_structures * s, double * F_d, do
 
 void gap_fast(rgpu_gap_model * m, rgpu_structures * s, double * E_d, double * F_d, bool forces,
               double * stress_d) {
-  gap_fast_forward(m, s, E_d);
-  if (forces) gap_fast_backward(m, s, F_d, stress_d);
+  gap_fast_forward(m, s, E_d, forces);
+  if (forces) {
+    gap_fast_backward(m, s, F_d, stress_d);
+  } else {
+    mark(s, 6);
+    mark(s, 7);
+  }
 }
 
 }  // namespace
@@ -1085,7 +1093,9 @@ static void gap_predict_impl(rgpu_gap_model * m, rgpu_structures * s, int precis
     calculator_to_device(m->calc);
     s->timed = true;
     mark(s, 0);
-    const bool want_forces = true;
+    // energies alone need neither the second GEMM nor the adjoint; a call
+    // that asks for no output leaves both on the device
+    const bool want_forces = forces || neg_stress || !energies;
     // neighbour list, layout, features
     build_nl(s, m->calc->hy.cutoff);
     mark(s, 1);
@@ -1095,7 +1105,7 @@ static void gap_predict_impl(rgpu_gap_model * m, rgpu_structures * s, int precis
     s->E_d.ensure(sizeof(double) * (s->n_struct + 1));
     s->F_d.ensure(sizeof(double) * 3 * (na + 1));
     RGPU_CUDA(cudaMemsetAsync(s->E_d.p, 0, sizeof(double) * s->n_struct, s->st));
-    RGPU_CUDA(cudaMemsetAsync(s->F_d.p, 0, sizeof(double) * 3 * na, s->st));
+    if (want_forces) RGPU_CUDA(cudaMemsetAsync(s->F_d.p, 0, sizeof(double) * 3 * na, s->st));
     double * stress_d = nullptr;
     if (neg_stress) {
       s->S_d.ensure(sizeof(double) * 6 * (s->n_struct + 1));
@@ -1488,7 +1498,7 @@ static void md_drop(rgpu_structures * s) {
 // outputs (energies, forces, stress sums) into pinned out_h (null: left on
 // the device), and the status word copied to the host at the end.
 static void graph_enqueue(rgpu_gap_model * m, rgpu_structures * s, bool stress, const double * pos_h,
-                          double * out_h, const NlCaps & caps) {
+                          double * out_h, const NlCaps & caps, bool forces = true) {
   rgpu_calculator * c = m->calc;
   cudaStream_t st = s->st;
   const int64_t na = s->n_atoms;
@@ -1523,12 +1533,13 @@ static void graph_enqueue(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   launch_ps_fwd_fast(pa, s->C32.as<float>(), nullptr, s->Xh.as<__nv_bfloat16>(), s->Xl.as<__nv_bfloat16>(),
                      s->xscale32.as<float>(), st);
   RGPU_CUDA(cudaMemsetAsync(s->E_d.p, 0, sizeof(double) * s->n_struct, st));
-  RGPU_CUDA(cudaMemsetAsync(s->F_d.p, 0, sizeof(double) * 3 * na, st));
+  if (forces) RGPU_CUDA(cudaMemsetAsync(s->F_d.p, 0, sizeof(double) * 3 * na, st));
   if (stress) RGPU_CUDA(cudaMemsetAsync(s->S_d.p, 0, sizeof(double) * 6 * s->n_struct, st));
-  gap_fast(m, s, s->E_d.as<double>(), s->F_d.as<double>(), true, stress ? s->S_d.as<double>() : nullptr);
+  gap_fast(m, s, s->E_d.as<double>(), s->F_d.as<double>(), forces, stress ? s->S_d.as<double>() : nullptr);
   if (double * out = out_h) {
     RGPU_CUDA(cudaMemcpyAsync(out, s->E_d.p, sizeof(double) * s->n_struct, cudaMemcpyDeviceToHost, st));
-    RGPU_CUDA(cudaMemcpyAsync(out + s->n_struct, s->F_d.p, sizeof(double) * 3 * na, cudaMemcpyDeviceToHost, st));
+    if (forces)
+      RGPU_CUDA(cudaMemcpyAsync(out + s->n_struct, s->F_d.p, sizeof(double) * 3 * na, cudaMemcpyDeviceToHost, st));
     if (stress)
       RGPU_CUDA(cudaMemcpyAsync(out + s->n_struct + 3 * na, s->S_d.p, sizeof(double) * 6 * s->n_struct,
                                 cudaMemcpyDeviceToHost, st));
@@ -1735,12 +1746,12 @@ static bool pgraph_replay(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   calculator_to_device(m->calc);
   set_layout(s, m->calc->hy, m->species);
   model_layout(m, s, true);
-  const bool outputs = energies || forces || neg_stress;
+  const bool outputs = energies || forces || neg_stress, want_forces = forces || neg_stress || !energies;
   const std::vector<int64_t> cnt = centres_per_species(s);
   std::vector<const void *> bufs;
   for (PredictGraph & g : s->pgraphs) {
-    if (g.model != m || g.stress != stress || g.outputs != outputs || g.n_struct != s->n_struct ||
-        g.n_atoms != s->n_atoms || g.species != s->species || g.species_count != cnt)
+    if (g.model != m || g.stress != stress || g.outputs != outputs || g.forces != want_forces ||
+        g.n_struct != s->n_struct || g.n_atoms != s->n_atoms || g.species != s->species || g.species_count != cnt)
       continue;
     if (bufs.empty()) bufs = md_buffers(m, s);
     if (g.buffers != bufs) continue;
@@ -1778,7 +1789,7 @@ static bool pgraph_replay(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
 // nothing may be allocated while recording, and checks that the call fits
 // them), then the recording. A failure leaves the handle on the ordinary
 // path for this bucket.
-static void pgraph_record(rgpu_gap_model * m, rgpu_structures * s, bool stress, bool outputs) {
+static void pgraph_record(rgpu_gap_model * m, rgpu_structures * s, bool stress, bool outputs, bool forces) {
   constexpr size_t kMaxGraphs = 4;
   PredictGraph g;
   int64_t sites = 0, boxes = 0;
@@ -1789,6 +1800,7 @@ static void pgraph_record(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   g.model = m;
   g.stress = stress;
   g.outputs = outputs;
+  g.forces = forces;
   g.n_struct = s->n_struct;
   g.n_atoms = s->n_atoms;
   g.species = s->species;
@@ -1801,7 +1813,7 @@ static void pgraph_record(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   s->timed = false;
   bool ok = true;
   try {
-    graph_enqueue(m, s, stress, nullptr, g.out_h, g.caps);
+    graph_enqueue(m, s, stress, nullptr, g.out_h, g.caps, forces);
     RGPU_CUDA(cudaStreamSynchronize(s->st));
     ok = s->status_h->code == 0 && gemm_tc_timeout(true) == 0;
   } catch (...) {
@@ -1811,7 +1823,7 @@ static void pgraph_record(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
     ok = cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
       try {
-        graph_enqueue(m, s, stress, nullptr, g.out_h, g.caps);
+        graph_enqueue(m, s, stress, nullptr, g.out_h, g.caps, forces);
       } catch (...) {
         ok = false;
       }
@@ -1856,7 +1868,8 @@ static void gap_predict_entry(rgpu_gap_model * m, rgpu_structures * s, int preci
   const bool stress = neg_stress != nullptr;
   if (graphs && pgraph_replay(m, s, stress, energies, forces, neg_stress)) return;
   gap_predict_impl(m, s, precision, energies, forces, neg_stress);
-  if (graphs) pgraph_record(m, s, stress, energies || forces || neg_stress);
+  if (graphs)
+    pgraph_record(m, s, stress, energies || forces || neg_stress, forces || neg_stress || !energies);
 }
 
 // ===================================================================== C ABI

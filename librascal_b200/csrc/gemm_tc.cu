@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_grouped_kernel(const __gr
             hw[k / 2] = *reinterpret_cast<const uint32_t *>(&h);
             lw[k / 2] = *reinterpret_cast<const uint32_t *>(&l);
           }
-          if (row >= G.M) continue;
+          if (row >= G.M || !G.W_hi) continue;  // W_hi null: energies only
           uint4 * dh = reinterpret_cast<uint4 *>(G.W_hi + row * G.ldw + col);
           uint4 * dl = reinterpret_cast<uint4 *>(G.W_lo + row * G.ldw + col);
 #pragma unroll
