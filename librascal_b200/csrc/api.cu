@@ -848,14 +848,6 @@ void gap_plain(rgpu_gap_model * m, rgpu_structures * s, double * E_d, double * F
   mark(s, 7);
 }
 
-// Offset of species sI's energy partials ([ceil(M/256)][rows]) in epart: the
-// grouped forward GEMM writes every species' partials in one launch.
-int64_t eofs_of(const rgpu_structures * s, const rgpu_gap_model * m, int sI) {
-  int64_t o = 0;
-  for (int k = 0; k < sI; ++k) o += s->species_count[k] * ((m->segs[k].M + kTcTileN - 1) / kTcTileN);
-  return o;
-}
-
 // W offsets of the species segments (rows x Mpad BF16 each) in s->Wh/Wl.
 std::vector<int64_t> w_offsets(const rgpu_gap_model * m, const rgpu_structures * s) {
   std::vector<int64_t> wofs(s->fd.S);
@@ -904,11 +896,15 @@ void gap_fast_forward(rgpu_gap_model * m, rgpu_structures * s, double * E_d, boo
   cudaStream_t st = s->st;
   s->fwd_model = nullptr;
   mark(s, 4);
-  // per-species W (BF16 hi/lo) and energy partial buffers
-  int64_t wtot = 0, eparts = 0;
+  // per-species W (BF16 hi/lo) and energy partials ([tiles along M][rows])
+  int points[kMaxSpecies];
+  for (int sI = 0; sI < fd.S; ++sI) points[sI] = m->segs[sI].M;
+  const int tile_n = gemm_forward_tile(s->species_count.data(), points, fd.S, fd.Dg);
+  int64_t wtot = 0, eparts = 0, eofs[kMaxSpecies];
   for (int sI = 0; sI < fd.S; ++sI) {
     if (need_w) wtot += s->species_count[sI] * m->segs[sI].Mpad;
-    eparts += s->species_count[sI] * ((m->segs[sI].M + kTcTileN - 1) / kTcTileN);
+    eofs[sI] = eparts;
+    eparts += s->species_count[sI] * ((points[sI] + tile_n - 1) / tile_n);
   }
   s->Wh.ensure(sizeof(uint16_t) * size_t(std::max<int64_t>(wtot, 1)) + 64);
   s->Wl.ensure(sizeof(uint16_t) * size_t(std::max<int64_t>(wtot, 1)) + 64);
@@ -947,21 +943,21 @@ void gap_fast_forward(rgpu_gap_model * m, rgpu_structures * s, double * E_d, boo
       a.ldw = g.Mpad;
       a.alpha = m->alpha32.as<float>() + g.m0;
       a.zeta = m->zeta;
-      a.e_part = s->epart.as<float>() + eofs_of(s, m, sI);
+      a.e_part = s->epart.as<float>() + eofs[sI];
       a.row_scale = s->xscale32.as<float>() + row0;  // k = (p . t) / |p|
       set_segments(a, s, tm, sI, 1);  // K blocks of species pairs absent from a tile are skipped
       fwd.push_back(a);
     }
     row0 += rows;
   }
-  gemm_bf16x3_grouped(fwd.data(), int(fwd.size()), st, tile_config(fd.S, fd.n, fd.L).gemm_variant);
+  gemm_bf16x3_grouped(fwd.data(), int(fwd.size()), st, tile_config(fd.S, fd.n, fd.L).gemm_variant, tile_n);
   row0 = 0;
   for (int sI = 0; sI < fd.S; ++sI) {
     const int64_t rows = s->species_count[sI];
     const GapSpecies & g = m->segs[sI];
     if (rows > 0 && g.M > 0) {
-      const int nparts = (g.M + kTcTileN - 1) / kTcTileN;
-      launch_energy_reduce(rows, nparts, s->epart.as<float>() + eofs_of(s, m, sI), rows, nullptr, row0,
+      const int nparts = (g.M + tile_n - 1) / tile_n;
+      launch_energy_reduce(rows, nparts, s->epart.as<float>() + eofs[sI], rows, nullptr, row0,
                            s->center_of_row.as<int32_t>(), s->nl.center_struct, E_d, st);
     }
     row0 += rows;

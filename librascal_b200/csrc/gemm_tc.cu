@@ -751,7 +751,8 @@ void grouped_launch(const Bf16x3Gemm * gs, int n, cudaStream_t st) {
       throw Error(RGPU_ERR_INVALID_ARGUMENT, "grouped GEMM: groups must share the epilogue");
     p.epilogue = g.epilogue;
     p.zeta = g.zeta;
-    if (g.K % BK != 0) throw Error(RGPU_ERR_INVALID_ARGUMENT, "grouped GEMM: K must be a multiple of the K block");
+    // a last K block that reaches past K is filled with zeros by its copies
+    if (g.K % 32 != 0) throw Error(RGPU_ERR_INVALID_ARGUMENT, "grouped GEMM: K must be a multiple of 32");
     p.a_hi[ng] = make_map(g.A_hi, g.M, g.K, g.lda, kBM, BK);
     p.a_lo[ng] = make_map(g.A_lo, g.M, g.K, g.lda, kBM, BK);
     p.b_hi[ng] = make_map(g.B_hi, g.N, g.K, g.ldb, BN, BK);
@@ -807,11 +808,43 @@ void grouped_launch(const Bf16x3Gemm * gs, int n, cudaStream_t st) {
   cuda_check(cudaGetLastError(), "gemm_tc_grouped launch");
 }
 
-// Pipelines of the grouped GEMM (tile 128 x kTcTileN): 0 = 4 stages of K
-// blocks of 32 (64-byte swizzle, 192 KB of stages), 1 = 3 stages of 32,
-// 2 = 2 stages of K blocks of 64 (128-byte swizzle), used only when every
-// group's K is a multiple of 64 (else variant 0 runs).
-void gemm_bf16x3_grouped(const Bf16x3Gemm * gs, int n, cudaStream_t st, int variant) {
+// Width of the forward's tiles. 256 columns load the least per product (48 KB
+// per 32 k against 24 KB for 64) and stay as soon as the tiles fill the SMs;
+// below that the narrower tiles put more SMs to work on a chain that is K
+// blocks long. Per 32 k a tile took about 0.52 us at 256 columns and 0.39 at
+// 64 (what bounds it there is the issue of copies and MMAs by one thread
+// each, hence K blocks of 64 for the narrow tiles: 0.48 with blocks of 32),
+// plus about 2 us and 6 us per 256 columns of epilogue. At 100 clusters with
+// 1 000 sparse points (22 tiles of 256, 185 K blocks) 64 columns took 76 us
+// instead of 103; at 84 tiles and 32 K blocks 256 columns remain the choice.
+int gemm_forward_tile(const int64_t * rows, const int * M, int n, int64_t K) {
+  constexpr int kSms = 148;
+  const int widths[3] = {256, 128, 64};
+  const double per_block[3] = {0.52, 0.44, 0.39};
+  int best = widths[0];
+  double best_us = 0.;
+  for (int w = 0; w < 3; ++w) {
+    int64_t tiles = 0;
+    for (int i = 0; i < n; ++i)
+      if (rows[i] > 0 && M[i] > 0) tiles += (rows[i] + kBM - 1) / kBM * ((M[i] + widths[w] - 1) / widths[w]);
+    const double us =
+        double((tiles + kSms - 1) / kSms) * (2. + double(K) / 32. * per_block[w] + 6. * widths[w] / 256.);
+    if (w == 0 || us < best_us) {
+      best = widths[w];
+      best_us = us;
+    }
+  }
+  return best;
+}
+
+// Pipelines of the grouped GEMM at tile width 256: 0 = 4 stages of K blocks
+// of 32 (64-byte swizzle, 192 KB of stages), 1 = 3 stages of 32, 2 = 2 stages
+// of K blocks of 64 (128-byte swizzle), used only when every group's K is a
+// multiple of 64 (else variant 0 runs). Narrower tiles keep the same 192 KB
+// in flight, in K blocks of 64.
+void gemm_bf16x3_grouped(const Bf16x3Gemm * gs, int n, cudaStream_t st, int variant, int tile_n) {
+  if (tile_n == 64) return grouped_launch<64, 4, 64>(gs, n, st);
+  if (tile_n == 128) return grouped_launch<128, 3, 64>(gs, n, st);
   if (variant == 2) {
     for (int i = 0; i < n; ++i)
       if (gs[i].M > 0 && gs[i].N > 0 && gs[i].K % 64 != 0) variant = 0;

@@ -430,7 +430,10 @@ constexpr int kTcTileN = 256;
 void gemm_bf16x3(const Bf16x3Gemm & g, cudaStream_t st);
 // Several GEMMs of the same epilogue kind (up to 16; K may differ) in one
 // persistent launch with a double-buffered TMEM accumulator.
-void gemm_bf16x3_grouped(const Bf16x3Gemm * gs, int n, cudaStream_t st, int variant = 0);
+// The forward's energy partials have one row per tile of `tile_n` columns
+// (64, 128 or 256; gemm_forward_tile picks it).
+void gemm_bf16x3_grouped(const Bf16x3Gemm * gs, int n, cudaStream_t st, int variant = 0, int tile_n = kTcTileN);
+int gemm_forward_tile(const int64_t * rows, const int * M, int n, int64_t K);
 // 0 when no bounded wait of the tcgen05 GEMM gave up, else where it did.
 int gemm_tc_timeout(bool reset);
 // Polls of the tcgen05 GEMMs' MMA-warp operand waits (negative: the
