@@ -315,11 +315,9 @@ int64_t rgpu_kernel_launches(int reset);
 /* Device time (ms) of the stages of the last rgpu_gap_predict call, from
  * CUDA events on the structure set's stream: 0 = whole call, 1 = neighbour
  * list, 2 = expansion, 3 = power spectrum, 4 = forward GEMMs, 5 = backward
- * GEMMs, 6 = power-spectrum backward (FP64: with the pair adjoint), 7 = pair
- * adjoint (FP32). After
+ * GEMMs, 6 = power-spectrum backward, 7 = pair adjoint. After
  * rgpu_sparse_kernel_derivative: 0 = its device time after the features and
- * before the copy to the host, 4 = the zeta k^(zeta-1) GEMMs, 6 = the
- * gradient chunks (materialised dX/dr and the gathered GEMMs). */
+ * before the copy to the host, 4 = the X T GEMMs, 6 = the gradient rows. */
 rgpu_status rgpu_stage_times(const rgpu_structures * s, double * ms_out,
                              int32_t n_stages);
 /* Launch shapes of the FP32 path per feature shape (n_species, max_radial,

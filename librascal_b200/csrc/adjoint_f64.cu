@@ -254,10 +254,29 @@ pair_adjoint_f64_kernel(ExpansionArgs a, const int32_t * __restrict__ pair_cente
     for (int k = 0; k < 6; ++k) atomicAdd(&stress[6 * size_t(sid) + k], t6[k]);
 }
 
+// Spherical harmonics and their gradients of pairs list[0..n) (pair indices
+// of the neighbour list), for the training matrices: out[k] = [4][K], the
+// values and their x, y, z derivatives.
 template <int L>
-void adjoint_f64(const PsArgs & ps, const ExpansionArgs & a, const double * C, const double * X,
-                 const double * inv_norm, const double * t, double * dC, const int32_t * pair_center, int64_t n_pairs,
-                 double * F, const int32_t * center_struct, double * stress, cudaStream_t st) {
+__global__ void __launch_bounds__(kPairThreads)
+pair_harmonics_kernel(ExpansionArgs a, int64_t n, const int32_t * __restrict__ list, double * __restrict__ out) {
+  constexpr int K = (L + 1) * (L + 1);
+  const int64_t k = int64_t(blockIdx.x) * kPairThreads + threadIdx.x;
+  if (k >= n) return;
+  const int64_t p = list[k];
+  double * o = out + k * 4 * K;
+  spherical_harmonics<L, true, double>(a.pair_dir[3 * p], a.pair_dir[3 * p + 1], a.pair_dir[3 * p + 2],
+                                       [&](int lm, double y, double gx, double gy, double gz) {
+                                         o[lm] = y;
+                                         o[K + lm] = gx;
+                                         o[2 * K + lm] = gy;
+                                         o[3 * K + lm] = gz;
+                                       });
+}
+
+template <int L>
+void ps_bwd_f64(const PsArgs & ps, const double * C, const double * X, const double * inv_norm, const double * t,
+                double * dC, cudaStream_t st) {
   const FeatureDims & fd = ps.fd;
   const int pnn = fd.P * fd.n * fd.n;
   // a row that only fits without the padding (what the forward needs) goes
@@ -271,44 +290,60 @@ void adjoint_f64(const PsArgs & ps, const ExpansionArgs & a, const double * C, c
   }
   RGPU_CUDA(cudaFuncSetAttribute(ps_bwd_f64_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   ps_bwd_f64_kernel<L><<<unsigned(ps.n_centers), kBwdThreads, smem, st>>>(ps, plane, C, X, inv_norm, t, dC);
-  RGPU_LAUNCHED();
-  RGPU_CUDA(cudaGetLastError());
-  pair_adjoint_f64_kernel<L><<<unsigned((n_pairs + kPairThreads - 1) / kPairThreads), kPairThreads, 0, st>>>(
-      a, pair_center, n_pairs, dC, F, center_struct, stress);
-  RGPU_LAUNCHED();
-  RGPU_CUDA(cudaGetLastError());
 }
 
 }  // namespace
 
-void launch_adjoint_fp64(const PsArgs & ps, const ExpansionArgs & a, const double * C, const double * X,
-                         const double * inv_norm, const double * t, double * dC, const int32_t * pair_center,
-                         int64_t n_pairs, double * F, const int32_t * center_struct, double * stress,
-                         cudaStream_t st) {
-  if (ps.n_centers == 0 || n_pairs == 0) return;
-  sph_constants_tu();
-#define RGPU_ADJ64_CASE(LL)                                                                              \
-  case LL:                                                                                               \
-    adjoint_f64<LL>(ps, a, C, X, inv_norm, t, dC, pair_center, n_pairs, F, center_struct, stress, st); \
-    break;
-  switch (a.fd.L) {
-    RGPU_ADJ64_CASE(0)
-    RGPU_ADJ64_CASE(1)
-    RGPU_ADJ64_CASE(2)
-    RGPU_ADJ64_CASE(3)
-    RGPU_ADJ64_CASE(4)
-    RGPU_ADJ64_CASE(5)
-    RGPU_ADJ64_CASE(6)
-    RGPU_ADJ64_CASE(7)
-    RGPU_ADJ64_CASE(8)
-    RGPU_ADJ64_CASE(9)
-    RGPU_ADJ64_CASE(10)
-    RGPU_ADJ64_CASE(11)
-    RGPU_ADJ64_CASE(12)
-    default:
-      throw Error(RGPU_ERR_INVALID_ARGUMENT, "max_angular above 12 is not supported on the GPU");
+#define RGPU_ADJ64_SWITCH(L_, CASE)                                                              \
+  switch (L_) {                                                                                  \
+    CASE(0) CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8) CASE(9) CASE(10)     \
+    CASE(11) CASE(12)                                                                            \
+    default:                                                                                     \
+      throw Error(RGPU_ERR_INVALID_ARGUMENT, "max_angular above 12 is not supported on the GPU"); \
   }
-#undef RGPU_ADJ64_CASE
+
+void launch_ps_bwd_fp64(const PsArgs & ps, const double * C, const double * X, const double * inv_norm,
+                        const double * t, double * dC, cudaStream_t st) {
+  if (ps.n_centers == 0) return;
+#define RGPU_CASE(LL)                                \
+  case LL:                                           \
+    ps_bwd_f64<LL>(ps, C, X, inv_norm, t, dC, st); \
+    break;
+  RGPU_ADJ64_SWITCH(ps.fd.L, RGPU_CASE)
+#undef RGPU_CASE
+  RGPU_LAUNCHED();
+  RGPU_CUDA(cudaGetLastError());
+}
+
+void launch_pair_adjoint_fp64(const ExpansionArgs & a, const double * dC, const int32_t * pair_center,
+                              int64_t n_pairs, double * F, const int32_t * center_struct, double * stress,
+                              cudaStream_t st) {
+  if (a.n_centers == 0 || n_pairs == 0) return;
+  sph_constants_tu();
+  const unsigned grid = unsigned((n_pairs + kPairThreads - 1) / kPairThreads);
+#define RGPU_CASE(LL)                                                                                             \
+  case LL:                                                                                                        \
+    pair_adjoint_f64_kernel<LL><<<grid, kPairThreads, 0, st>>>(a, pair_center, n_pairs, dC, F, center_struct, stress); \
+    break;
+  RGPU_ADJ64_SWITCH(a.fd.L, RGPU_CASE)
+#undef RGPU_CASE
+  RGPU_LAUNCHED();
+  RGPU_CUDA(cudaGetLastError());
+}
+
+void launch_pair_harmonics_fp64(const ExpansionArgs & a, int64_t n, const int32_t * list, double * out,
+                                cudaStream_t st) {
+  if (n <= 0) return;
+  sph_constants_tu();
+  const unsigned grid = unsigned((n + kPairThreads - 1) / kPairThreads);
+#define RGPU_CASE(LL)                                                          \
+  case LL:                                                                     \
+    pair_harmonics_kernel<LL><<<grid, kPairThreads, 0, st>>>(a, n, list, out); \
+    break;
+  RGPU_ADJ64_SWITCH(a.fd.L, RGPU_CASE)
+#undef RGPU_CASE
+  RGPU_LAUNCHED();
+  RGPU_CUDA(cudaGetLastError());
 }
 
 }  // namespace rgpu

@@ -218,7 +218,7 @@ struct rgpu_structures {
   DevBuf E_d, F_d, S_d, K64, t64, erow64, Wh, Wl, dX32, dC32, epart, Xh, Xl, chunk_map;
   bool feat_x32{false};  // FP32 features also kept unsplit (for export)
   DevBuf dCp, dCs, dXp;
-  DevBuf knm, plist, Vvir;  // sparse kernel matrices for training
+  DevBuf knm, plist, Tq;  // sparse kernel matrices for training
   // MD step recorded as a CUDA graph (rgpu_md_step)
   cudaGraph_t md_graph{nullptr};
   cudaGraphExec_t md_exec{nullptr};
@@ -842,10 +842,11 @@ void gap_plain(rgpu_gap_model * m, rgpu_structures * s, double * E_d, double * F
   pa.row_of_center = s->row_of_center.as<int32_t>();
   pa.present = s->present.as<uint32_t>();
   s->dC64.ensure(sizeof(double) * size_t(nc) * fd.S * fd.nK + 64);
-  launch_adjoint_fp64(pa, exp_args(c, s), s->C64.as<double>(), s->X64.as<double>(), s->invn64.as<double>(),
-                      s->t64.as<double>(), s->dC64.as<double>(), s->nl.pair_center, s->nl.n_pairs, F_d,
-                      s->nl.center_struct, stress_d, st);
+  launch_ps_bwd_fp64(pa, s->C64.as<double>(), s->X64.as<double>(), s->invn64.as<double>(), s->t64.as<double>(),
+                     s->dC64.as<double>(), st);
   mark(s, 7);
+  launch_pair_adjoint_fp64(exp_args(c, s), s->dC64.as<double>(), s->nl.pair_center, s->nl.n_pairs, F_d,
+                           s->nl.center_struct, stress_d, st);
 }
 
 // W offsets of the species segments (rows x Mpad BF16 each) in s->Wh/Wl.
@@ -1236,9 +1237,8 @@ static void sparse_kernel_impl(rgpu_gap_model * m, rgpu_structures * s, bool ato
 }
 
 // K_NM gradient rows: SparseKernelImpl<GAP>::compute_derivative
-// (models/sparse_kernels.hh:258-499). dX/dr is materialised chunk by chunk
-// as in the plain prediction path and contracted with the sparse points of
-// each central species by one gathered GEMM per species and chunk.
+// (models/sparse_kernels.hh:258-499): the pairs' power-spectrum gradients are
+// formed chunk by chunk and contracted with the sparse points (training.cu).
 static void sparse_kernel_derivative_impl(rgpu_gap_model * m, rgpu_structures * s, bool neg_stress,
                                           double * out) {
   kernel_features(m, s, true);
@@ -1257,10 +1257,10 @@ static void sparse_kernel_derivative_impl(rgpu_gap_model * m, rgpu_structures * 
     RGPU_CUDA(cudaStreamSynchronize(st));
     return;
   }
-  // zeta (X_i . T_m)^(zeta-1) of every row
+  // x_i . T_m of every row
   mark(s, 4);
   const GapGroup gg = species_dots(m, s);
-  launch_kernel_weight(gg, s->K64.as<double>(), m->zeta, st);
+  launch_dots_sum(gg, s->K64.as<double>(), st);
   mark(s, 5);
   mark(s, 6);
   // The reference returns from its loop over structures at the first one
@@ -1279,112 +1279,49 @@ static void sparse_kernel_derivative_impl(rgpu_gap_model * m, rgpu_structures * 
     }
   }
   const std::vector<int64_t> & poff = pair_offsets_host(s);
-  const size_t per_pair = sizeof(double) * (3 * size_t(fd.D) + 3 * size_t(fd.nK));
-  const size_t per_center =
-      sizeof(double) * (size_t(fd.S) * 3 * fd.nK + (neg_stress ? 6 * size_t(fd.D) : 0));
-  const size_t budget = plain_budget_bytes();
-  ExpansionArgs ea = exp_args(c, s);
-  PsArgs pa;
-  pa.fd = fd;
-  pa.n_centers = nc;
-  pa.normalize = c->hy.normalize;
-  pa.row_of_center = s->row_of_center.as<int32_t>();
-  std::vector<std::vector<int32_t>> lists(fd.S), centres(fd.S);
+  KnmGradArgs a{};
+  a.fd = fd;
+  a.ea = exp_args(c, s);
+  a.normalize = c->hy.normalize;
+  a.pair_center = s->nl.pair_center;
+  a.row_of_center = s->row_of_center.as<int32_t>();
+  a.center_struct = s->nl.center_struct;
+  a.C = s->C64.as<double>();
+  a.inv_norm = s->invn64.as<double>();
+  if (a.normalize) {
+    // d(x . p)/dc: the power-spectrum backward of t = x without its
+    // projection (inv_norm is applied by the pair rows)
+    PsArgs pa;
+    pa.fd = fd;
+    pa.n_centers = nc;
+    pa.normalize = false;
+    pa.row_of_center = s->row_of_center.as<int32_t>();
+    pa.present = s->present.as<uint32_t>();
+    s->dC64.ensure(sizeof(double) * size_t(nc) * fd.S * fd.nK + 64);
+    launch_ps_bwd_fp64(pa, s->C64.as<double>(), s->X64.as<double>(), s->invn64.as<double>(), s->X64.as<double>(),
+                       s->dC64.as<double>(), st);
+  }
+  a.U = s->dC64.as<double>();
+  s->Tq.ensure(sizeof(double) * size_t(fd.S) * M * knm_row_len(fd) + 64);
+  launch_knm_points(fd, M, m->T64.as<double>(), fd.Dpad, s->Tq.as<double>(), st);
+  a.Tq = s->Tq.as<double>();
+  a.M = M;
+  a.dots = &gg;
+  a.K = s->K64.as<double>();
+  a.zeta = m->zeta;
+  a.ucol = m->ucol.as<int32_t>();
+  a.out = s->knm.as<double>();
+  a.ldo = M;
+  a.stress_row0 = neg_stress ? 3 * nc : -1;
+  // pairs in chunks of a bounded scratch
+  const int64_t chunk = std::max<int64_t>(1, int64_t(plain_budget_bytes() / knm_pair_bytes(fd)));
   int64_t c0 = 0;
   while (c0 < c_stop) {
-    int64_t c1 = c0;
-    size_t used = 0;
-    while (c1 < c_stop) {
-      size_t add = per_pair * size_t(poff[c1 + 1] - poff[c1]) + per_center;
-      if (c1 > c0 && used + add > budget) break;
-      used += add;
-      ++c1;
-    }
-    const int64_t p_base = poff[c0];
-    const int64_t np = poff[c1] - p_base;
-    // pairs of the chunk listed by the species of their centre: (pair - p_base, centre)
-    for (auto & l : lists) l.clear();
-    for (auto & l : centres) l.clear();
-    for (int64_t ci = c0; ci < c1; ++ci) {
-      const int sI = sp_index[s->types[ci]];
-      std::vector<int32_t> & l = lists[sI];
-      centres[sI].push_back(int32_t(ci));
-      for (int64_t p = poff[ci]; p < poff[ci + 1]; ++p) {
-        l.push_back(int32_t(p - p_base));
-        l.push_back(int32_t(ci));
-      }
-    }
-    // one upload: [pair lists of all species][centre lists of all species]
-    std::vector<int32_t> flat;
-    std::vector<int64_t> loff(fd.S + 1, 0), coff(fd.S + 1, 0);
-    for (int sI = 0; sI < fd.S; ++sI) {
-      loff[sI] = int64_t(flat.size()) / 2;
-      flat.insert(flat.end(), lists[sI].begin(), lists[sI].end());
-    }
-    loff[fd.S] = int64_t(flat.size()) / 2;
-    const int64_t cbase = int64_t(flat.size());
-    for (int sI = 0; sI < fd.S; ++sI) {
-      coff[sI] = int64_t(flat.size()) - cbase;
-      flat.insert(flat.end(), centres[sI].begin(), centres[sI].end());
-    }
-    coff[fd.S] = int64_t(flat.size()) - cbase;
-    upload(s, s->plist, flat.data(), sizeof(int32_t) * flat.size());
-    if (neg_stress) s->Vvir.ensure(sizeof(double) * 6 * size_t(fd.D) * size_t(c1 - c0) + 64);
-    s->dCp.ensure(sizeof(double) * size_t(np) * 3 * fd.nK + 64);
-    s->dCs.ensure(per_center * size_t(c1 - c0) + 64);
-    s->dXp.ensure(sizeof(double) * size_t(np) * 3 * fd.D + 64);
-    launch_expansion_grad_fp64(ea, c0, c1, p_base, s->dCp.as<double>(), st);
-    launch_expansion_selfgrad_fp64(ea, c0, c1, p_base, s->dCp.as<double>(), s->dCs.as<double>(), st);
-    launch_ps_grad_fp64(pa, ea, c0, c1, p_base, s->C64.as<double>(), s->X64.as<double>(), s->invn64.as<double>(),
-                        s->dCp.as<double>(), s->dCs.as<double>(), s->dXp.as<double>(), st);
-    for (int sI = 0; sI < fd.S; ++sI) {
-      const GapSpecies & g = m->segs[sI];
-      const int64_t n_list = loff[sI + 1] - loff[sI];
-      if (n_list == 0 || g.M == 0) continue;
-      KnmDerArgs a{};
-      a.list = s->plist.as<int32_t>() + 2 * loff[sI];
-      a.n_list = n_list;
-      a.p_base = p_base;
-      a.dX = s->dXp.as<double>();
-      a.D = fd.D;
-      a.T = m->T64.as<double>() + size_t(g.m0) * fd.Dpad;
-      a.ldt = fd.Dpad;
-      a.M = g.M;
-      a.W = s->K64.as<double>() + gg.koff[sI];
-      a.ldw = gg.ldk[sI];
-      a.row0 = gg.row0[sI];
-      a.row_of_center = s->row_of_center.as<int32_t>();
-      a.pair_j = s->nl.pair_j;
-      a.ucol = m->ucol.as<int32_t>() + g.m0;
-      a.out = s->knm.as<double>();
-      a.ldo = M;
-      launch_knm_derivative(a, st);
-      if (neg_stress) {
-        KnmStressArgs b{};
-        b.centres = s->plist.as<int32_t>() + cbase + coff[sI];
-        b.n_centres = coff[sI + 1] - coff[sI];
-        b.p_base = p_base;
-        b.pair_off = s->nl.pair_off;
-        b.pair_dist = s->nl.pair_dist;
-        b.pair_dir = s->nl.pair_dir;
-        b.dX = s->dXp.as<double>();
-        b.D = fd.D;
-        b.V = s->Vvir.as<double>();
-        b.T = a.T;
-        b.ldt = a.ldt;
-        b.M = g.M;
-        b.W = a.W;
-        b.ldw = a.ldw;
-        b.row0 = a.row0;
-        b.row_of_center = a.row_of_center;
-        b.center_struct = s->nl.center_struct;
-        b.ucol = a.ucol;
-        b.out = a.out;
-        b.ldo = M;
-        b.stress_row0 = 3 * nc;
-        launch_knm_stress(b, st);
-      }
-    }
+    int64_t c1 = c0 + 1;
+    while (c1 < c_stop && poff[c1 + 1] - poff[c0] <= chunk) ++c1;
+    a.p0 = poff[c0];
+    a.p1 = poff[c1];
+    launch_knm_gradient(a, s->plist, s->dXp, st);
     c0 = c1;
   }
   mark(s, 7);
@@ -1464,7 +1401,7 @@ static std::vector<const void *> md_buffers(const rgpu_gap_model * m, const rgpu
                            &s->C64, &s->X64,
                            &s->invn64, &s->dC64, &s->C32, &s->X32, &s->xscale32, &s->E_d, &s->F_d, &s->S_d, &s->K64,
                            &s->t64, &s->erow64, &s->Wh, &s->Wl, &s->dX32, &s->dC32, &s->epart, &s->Xh, &s->Xl,
-                           &s->chunk_map, &s->dCp, &s->dCs, &s->dXp, &s->knm, &s->plist, &s->Vvir})
+                           &s->chunk_map, &s->dCp, &s->dCs, &s->dXp, &s->knm, &s->plist, &s->Tq})
     v.push_back(b->p);
   const NlWork & w = s->nlw;
   for (const DevBuf * b : {&w.geom, &w.counts64, &w.scan_tmp, &w.ghost_off, &w.site_x, &w.site_type, &w.site_real,

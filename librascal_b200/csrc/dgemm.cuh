@@ -1,7 +1,6 @@
 // FP64 tile GEMM on the tensor cores (mma.sync m16n8k8 f64): C[r][c] =
-// sum_k A[r][k] B(k, c), with the A rows addressed through a row-offset
-// functor (plain strided rows, or rows gathered from a list) and the result
-// handed to an epilogue functor. B is either N x K row-major (B_NT,
+// sum_k A[r][k] B(k, c), the result handed to an epilogue functor (what a row
+// needs is looked up once per row). B is either N x K row-major (B_NT,
 // C = A B^T) or K x N row-major. Several problems (one per species) run in
 // one launch, and K can be cut into splits whose partial sums go to separate
 // planes that the caller's next kernel adds.
@@ -38,35 +37,29 @@ constexpr size_t kDgSmem = sizeof(double) * kDgStages * (kDgStageA + kDgStageB);
 constexpr int kDgMaxProblems = kMaxSpecies;
 static_assert(kDgBK * kDgLdN <= kDgStageB, "the K x N tile fits the stage");
 
-struct DgPlainRows {
-  int64_t lda;
-  __host__ __device__ __forceinline__ int64_t operator()(int64_t r) const { return r * lda; }
-};
-
 // C[split][r][c]; planes are `plane` values apart.
 struct DgStoreC {
   double * C;
   int64_t ldc, plane;
-  __device__ __forceinline__ void operator()(int64_t r, int c, double v, int split) const {
-    C[split * plane + r * ldc + c] = v;
-  }
+  __device__ __forceinline__ double * row(int64_t r) const { return C + r * ldc; }
+  __device__ __forceinline__ void put(double * o, int c, double v, int split) const { o[split * plane + c] = v; }
 };
 
-template <class ARows, class Epi>
+template <class Epi>
 struct DgProblem {
   int64_t M;
   int N, K;
   const double * A;
-  ARows arows;
+  int64_t lda;
   const double * B;
   int64_t ldb;
   Epi epi;
 };
-template <class ARows, class Epi>
+template <class Epi>
 struct DgGroup {
   int n, splits;
   int64_t tile_end[kDgMaxProblems];  // running tile counts
-  DgProblem<ARows, Epi> p[kDgMaxProblems];
+  DgProblem<Epi> p[kDgMaxProblems];
 };
 
 __device__ __forceinline__ void dg_cp(double * smem, const double * gmem, int bytes, int full) {
@@ -86,9 +79,9 @@ __device__ __forceinline__ void dmma(double * c, const double * a, const double 
 
 // VEC: doubles per copy, 2 when every row of both operands starts on a
 // 16-byte boundary, else 1.
-template <bool B_NT, int VEC, class ARows, class Epi>
+template <bool B_NT, int VEC, class Epi>
 __global__ void __launch_bounds__(kDgThreads)
-dgemm_kernel(const __grid_constant__ DgGroup<ARows, Epi> g) {
+dgemm_kernel(const __grid_constant__ DgGroup<Epi> g) {
   extern __shared__ __align__(16) double dsm[];
   constexpr int kFull = 8 * VEC;
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
@@ -97,7 +90,7 @@ dgemm_kernel(const __grid_constant__ DgGroup<ARows, Epi> g) {
   const int64_t tile = blockIdx.x / unsigned(g.splits);
   int pi = 0;
   while (tile >= g.tile_end[pi]) ++pi;
-  const DgProblem<ARows, Epi> & p = g.p[pi];
+  const DgProblem<Epi> & p = g.p[pi];
   const int64_t local = tile - (pi ? g.tile_end[pi - 1] : 0);
   // column tiles vary fastest: the blocks that share an A row tile run
   // together, so A comes from DRAM once and the others read it from L2
@@ -114,7 +107,7 @@ dgemm_kernel(const __grid_constant__ DgGroup<ARows, Epi> g) {
 #pragma unroll
   for (int q = 0; q < kCopies; ++q) {
     const int64_t r = r0 + lr + q * kRows;
-    a_off[q] = r < p.M ? p.arows(r) : int64_t(-1);
+    a_off[q] = r < p.M ? r * p.lda : int64_t(-1);
     const int c = c0 + lr + q * kRows;
     b_off[q] = c < p.N ? int64_t(c) * p.ldb : int64_t(-1);
   }
@@ -206,13 +199,18 @@ dgemm_kernel(const __grid_constant__ DgGroup<ARows, Epi> g) {
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int h = 0; h < 2; ++h) {
+      const int64_t r = r0 + wm + 16 * i + gid + 8 * h;
+      if (r >= p.M) continue;
+      const auto row = p.epi.row(r);
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int64_t r = r0 + wm + 16 * i + gid + 8 * (v >> 1);
-        const int c = c0 + wn + 8 * j + 2 * tig + (v & 1);
-        if (r < p.M && c < p.N) p.epi(r, c, acc[i][j][v], split);
-      }
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          const int c = c0 + wn + 8 * j + 2 * tig + v;
+          if (c < p.N) p.epi.put(row, c, acc[i][j][2 * h + v], split);
+        }
+    }
 }
 
 // Splits of K that bring `tiles` tiles to about three blocks per SM (what
@@ -228,8 +226,8 @@ inline int64_t dgemm_tiles(int64_t M, int N) {
 
 // Launches the group (p[0..n) filled); `aligned` says that every row of A
 // and B starts on a 16-byte boundary.
-template <bool B_NT, class ARows, class Epi>
-void launch_dgemm(DgGroup<ARows, Epi> & g, bool aligned, cudaStream_t st) {
+template <bool B_NT, class Epi>
+void launch_dgemm(DgGroup<Epi> & g, bool aligned, cudaStream_t st) {
   int64_t tiles = 0;
   for (int i = 0; i < g.n; ++i) {
     tiles += dgemm_tiles(g.p[i].M, g.p[i].N);
@@ -237,7 +235,7 @@ void launch_dgemm(DgGroup<ARows, Epi> & g, bool aligned, cudaStream_t st) {
   }
   if (tiles == 0) return;
   if (tiles * g.splits > 0x7fffffff) throw Error(RGPU_ERR_CAPACITY, "FP64 GEMM: too many rows for one launch");
-  auto kernel = aligned ? dgemm_kernel<B_NT, 2, ARows, Epi> : dgemm_kernel<B_NT, 1, ARows, Epi>;
+  auto kernel = aligned ? dgemm_kernel<B_NT, 2, Epi> : dgemm_kernel<B_NT, 1, Epi>;
   RGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kDgSmem)));
   kernel<<<unsigned(tiles * g.splits), kDgThreads, kDgSmem, st>>>(g);
   RGPU_LAUNCHED();

@@ -264,9 +264,9 @@ __global__ void energy_reduce_kernel(int64_t rows, int n_parts, const float * __
 
 void gemm_nt_fp64(int64_t M, int64_t N, int64_t K, const double * A, int64_t lda, const double * B,
                   int64_t ldb, double * C, int64_t ldc, cudaStream_t st) {
-  DgGroup<DgPlainRows, DgStoreC> g{};
+  DgGroup<DgStoreC> g{};
   g.n = g.splits = 1;
-  g.p[0] = {M, int(N), int(K), A, DgPlainRows{lda}, B, ldb, DgStoreC{C, ldc, 0}};
+  g.p[0] = {M, int(N), int(K), A, lda, B, ldb, DgStoreC{C, ldc, 0}};
   launch_dgemm<true>(g, dgemm_aligned(A, lda) && dgemm_aligned(B, ldb), st);
 }
 
@@ -279,24 +279,24 @@ void gap_dots_split(GapGroup & g, int K) {
 
 void launch_gap_dots_fp64(const GapGroup & g, int K, const double * X, int64_t ldx, const double * T, int64_t ldt,
                           double * Kmat, cudaStream_t st) {
-  DgGroup<DgPlainRows, DgStoreC> d{};
+  DgGroup<DgStoreC> d{};
   d.splits = g.splits;
   for (int s = 0; s < g.S; ++s)
     if (g.rows[s] > 0 && g.M[s] > 0)
-      d.p[d.n++] = {g.rows[s], g.M[s], K, X + g.row0[s] * ldx, DgPlainRows{ldx}, T + g.m0[s] * ldt, ldt,
+      d.p[d.n++] = {g.rows[s], g.M[s], K, X + g.row0[s] * ldx, ldx, T + g.m0[s] * ldt, ldt,
                     DgStoreC{Kmat + g.koff[s], g.ldk[s], g.plane}};
   launch_dgemm<true>(d, dgemm_aligned(X, ldx) && dgemm_aligned(T, ldt), st);
 }
 
 void launch_gap_scaled_fp64(const GapGroup & g, int D, const double * W, const double * T, int64_t ldt, double * t,
                             int64_t ld, cudaStream_t st) {
-  DgGroup<DgPlainRows, DgStoreC> d{};
+  DgGroup<DgStoreC> d{};
   d.splits = 1;
   bool aligned = dgemm_aligned(W, 0) && dgemm_aligned(T, ldt);
   for (int s = 0; s < g.S; ++s)
     if (g.rows[s] > 0 && g.M[s] > 0) {
       aligned = aligned && (g.koff[s] & 1) == 0;
-      d.p[d.n++] = {g.rows[s], D, g.M[s], W + g.koff[s], DgPlainRows{g.ldk[s]}, T + g.m0[s] * ldt, ldt,
+      d.p[d.n++] = {g.rows[s], D, g.M[s], W + g.koff[s], g.ldk[s], T + g.m0[s] * ldt, ldt,
                     DgStoreC{t + g.row0[s] * ld, ld, 0}};
     }
   launch_dgemm<false>(d, aligned, st);

@@ -459,68 +459,61 @@ void launch_energy_reduce(int64_t rows, int n_parts, const float * e_part, int64
                           const double * e_row_fp64, int64_t row0, const int32_t * center_of_row,
                           const int32_t * center_struct, double * energies, cudaStream_t st);
 
-// FP64 adjoint: dE/dc of every centre from the dE/dx rows t (reference order,
+// FP64 adjoint. dE/dc of every centre from the dE/dx rows t (reference order,
 // stride Dpad; ps.present: the FP64 expansion's species masks) into dC
-// [centre][lm][S n], then forces F (= -dE/dr) and, with stress, the unscaled
-// negative stress sums per structure from one pass over the pairs.
-void launch_adjoint_fp64(const PsArgs & ps, const ExpansionArgs & a, const double * C, const double * X,
-                         const double * inv_norm, const double * t, double * dC, const int32_t * pair_center,
-                         int64_t n_pairs, double * F, const int32_t * center_struct, double * stress,
-                         cudaStream_t st);
+// [centre][lm][S n]; without ps.normalize t is taken as the gradient of the
+// unnormalised p times inv_norm = 1.
+void launch_ps_bwd_fp64(const PsArgs & ps, const double * C, const double * X, const double * inv_norm,
+                        const double * t, double * dC, cudaStream_t st);
+// Forces F (= -dE/dr) and, with stress, the unscaled negative stress sums per
+// structure from one pass over the pairs.
+void launch_pair_adjoint_fp64(const ExpansionArgs & a, const double * dC, const int32_t * pair_center,
+                              int64_t n_pairs, double * F, const int32_t * center_struct, double * stress,
+                              cudaStream_t st);
+// [4][K] harmonics and their gradients of the listed pairs.
+void launch_pair_harmonics_fp64(const ExpansionArgs & a, int64_t n, const int32_t * list, double * out,
+                                cudaStream_t st);
 // ------------------------------------------------------------------ training
 // K_NM energy rows from the dots of every species: k^zeta into row
 // center_of_row[row] (atom target) or added into its structure's row.
 void launch_knm_rows(const GapGroup & g, const double * K, int zeta, const int32_t * center_of_row,
                      const int32_t * center_struct, bool atom_target, const int32_t * ucol, double * out, int64_t ldo,
                      cudaStream_t st);
-// W = zeta k^(zeta-1) (1 for zeta = 1), in place (plane 0).
-void launch_kernel_weight(const GapGroup & g, double * K, int zeta, cudaStream_t st);
 // K_MM block of one species: out[ucol[a]][ucol[b]] = K[a][b]^zeta.
 void launch_kmm_scatter(int M, const double * K, int zeta, const int32_t * ucol, double * out, int64_t ldo,
                         cudaStream_t st);
-// Gradient block of one central species over one chunk of pairs.
-struct KnmDerArgs {
-  const int32_t * list;  // [n_list][2]: pair index relative to p_base, centre
-  int64_t n_list, p_base;
-  const double * dX;  // materialised dX/dr of the chunk, [pair][3][D]
-  int D;
-  const double * T;  // sparse points of the species, M rows of stride ldt
-  int64_t ldt;
-  int M;
-  const double * W;  // zeta k^(zeta-1) of the species' rows, [row - row0][ldw]
-  int64_t ldw;
-  int64_t row0;
-  const int32_t * row_of_center;
-  const int32_t * pair_j;
-  const int32_t * ucol;  // output column of each sparse point
-  double * out;
-  int64_t ldo;
-};
-void launch_knm_derivative(const KnmDerArgs & a, cudaStream_t st);
-// Negative-stress rows of one central species over one chunk: 6 virial rows
-// per centre into V, contracted with the sparse points.
-struct KnmStressArgs {
-  const int32_t * centres;  // centres of the species in the chunk
-  int64_t n_centres, p_base;
-  const int64_t * pair_off;
-  const double * pair_dist;
-  const double * pair_dir;
-  const double * dX;  // chunk [pair][3][D]
-  int D;
-  double * V;  // [n_centres][6][D] scratch
-  const double * T;
-  int64_t ldt;
-  int M;
-  const double * W;
-  int64_t ldw;
-  int64_t row0;
+// The gradient rows of one chunk of pairs [p0, p1) (training.cu).
+struct KnmGradArgs {
+  FeatureDims fd;
+  ExpansionArgs ea;
+  bool normalize;
+  int64_t p0, p1;
+  const int32_t * pair_center;
   const int32_t * row_of_center;
   const int32_t * center_struct;
+  const double * C;         // expansion coefficients
+  const double * inv_norm;  // 1/|p| per centre
+  const double * U;         // d(x . p)/dc per centre, [centre][lm][S n]
+  const double * Tq;        // sparse points against the neighbour's species, [S][M][Kd] (launch_knm_points)
+  int M;                    // sparse points in all
+  const GapGroup * dots;    // the layout of K
+  const double * K;         // x . T, planes added
+  int zeta;
   const int32_t * ucol;
   double * out;
-  int64_t ldo, stress_row0;
+  int64_t ldo;
+  int64_t stress_row0;  // < 0: no stress rows
 };
-void launch_knm_stress(const KnmStressArgs & a, cudaStream_t st);
+inline int knm_row_len(const FeatureDims & fd) { return (fd.S * fd.n * fd.n * (fd.L + 1) + 15) & ~15; }
+// Sparse points rearranged for pairs whose neighbour has species sj: row
+// [sj][m] holds [l][b][n1][n2], n1 the radial index of sj, n2 that of species
+// b; the two halves of the symmetric block b = sj are added.
+void launch_knm_points(const FeatureDims & fd, int M, const double * T, int64_t ldt, double * Tq, cudaStream_t st);
+// Adds the planes of the dots into plane 0.
+void launch_dots_sum(const GapGroup & g, double * K, cudaStream_t st);
+// Bytes of scratch per pair of a chunk.
+size_t knm_pair_bytes(const FeatureDims & fd);
+void launch_knm_gradient(const KnmGradArgs & a, DevBuf & list, DevBuf & scratch, cudaStream_t st);
 
 // Adjoint pair kernel: forces from dE/dC (FP32, the layout written by
 // launch_ps_bwd_fp32) and recomputed dC/dr. With stress, also the unscaled
