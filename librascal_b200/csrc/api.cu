@@ -208,7 +208,7 @@ struct rgpu_structures {
   DevBuf lut;
   FeatureDims fd{};
   std::vector<int64_t> species_count;
-  DevBuf row_of_center, center_of_row, species_count_d, sort_tmp, present, tile_mask;
+  DevBuf row_of_center, center_of_row, sort_tmp, present, tile_mask;
   DevBuf C64, X64, invn64, dC64, C32, X32, xscale32;  // xscale32[row] = 1/|p| (FP32 path)
   int feat_precision{-1};
   const rgpu_calculator * feat_calc{nullptr};
@@ -216,6 +216,7 @@ struct rgpu_structures {
   bool feat_valid{false};
   // GAP work
   DevBuf E_d, F_d, S_d, K64, t64, erow64, Wh, Wl, dX32, dC32, epart, Xh, Xl, chunk_map;
+  int chunk_map_of[3]{0, 0, 0};  // the (S, n, L) that chunk_map holds
   bool feat_x32{false};  // FP32 features also kept unsplit (for export)
   DevBuf dCp, dCs, dXp;
   DevBuf knm, plist, Tq;  // sparse kernel matrices for training
@@ -477,29 +478,50 @@ ExpansionArgs exp_args(const rgpu_calculator * c, const rgpu_structures * s) {
   return a;
 }
 
-// Species sort of the centres: row order of X (grouped by central species).
-void sort_rows(rgpu_structures * s) {
+// Rows and 128-row tiles of each central species (rows in species order).
+TileMaskArgs tile_mask_args(const rgpu_structures * s) {
+  TileMaskArgs a{};
+  a.S = s->fd.S;
+  int64_t r = 0, t = 0;
+  for (int sI = 0; sI < s->fd.S; ++sI) {
+    a.row0[sI] = r;
+    a.rows[sI] = s->species_count[sI];
+    a.tile_off[sI] = t;
+    r += s->species_count[sI];
+    t += (s->species_count[sI] + 127) / 128;
+  }
+  a.tile_off[s->fd.S] = t;
+  return a;
+}
+
+// Row order of X: grouped by central species. The FP32 path's layouts of more
+// than one segment group are sorted by the presence masks as well, after the
+// expansion that writes them (sort_rows_by_mask), so they skip this.
+void sort_rows(rgpu_structures * s, bool by_mask) {
   const int64_t nc = s->nl.n_centers;
   s->row_of_center.ensure(sizeof(int32_t) * (nc + 1));
   s->center_of_row.ensure(sizeof(int32_t) * (nc + 1));
-  s->species_count_d.ensure(sizeof(int64_t) * kMaxSpecies);
-  launch_species_sort(nc, s->types_d.as<int32_t>(), s->nl.center_atom, s->lut.as<int8_t>(), s->fd.S,
-                      s->species_count_d.as<int64_t>(), s->row_of_center.as<int32_t>(),
-                      s->center_of_row.as<int32_t>(), s->sort_tmp, s->st);
+  if (!by_mask)
+    launch_species_sort(nc, s->types_d.as<int32_t>(), s->nl.center_atom, s->lut.as<int8_t>(), s->fd.S,
+                        s->row_of_center.as<int32_t>(), s->center_of_row.as<int32_t>(), s->sort_tmp, s->st);
   // the counts per central species are known on the host since the upload
   s->species_count.assign(s->fd.S, 0);
   for (int sI = 0; sI < s->fd.S; ++sI) s->species_count[sI] = s->centres_of_type[s->species[sI]];
 }
 
-// After the FP32 expansion (which writes the presence masks): rows of one
-// species ordered by their neighbour species, so that the GEMM tiles of the
-// packed layout's species segments can skip what none of their rows holds.
-// Only layouts with more than one segment group need it.
+bool sorts_by_mask(const rgpu_calculator * c, const rgpu_structures * s) {
+  return c->hy.kind == "sphericalinvariants" && s->fd.G > 1;
+}
+
+// Rows of one species ordered by their neighbour species, so that the GEMM
+// tiles of the packed layout's species segments can skip what none of their
+// rows holds; and the species present in each 128-row tile.
 void sort_rows_by_mask(rgpu_structures * s) {
-  if (s->fd.G < 2) return;
+  const TileMaskArgs tm = tile_mask_args(s);
+  s->tile_mask.ensure(sizeof(uint32_t) * size_t(std::max<int64_t>(tm.tile_off[s->fd.S], 1)) + 64);
   launch_mask_sort(s->nl.n_centers, s->types_d.as<int32_t>(), s->nl.center_atom, s->lut.as<int8_t>(),
-                   s->present.as<uint32_t>(), s->fd.S, s->row_of_center.as<int32_t>(), s->center_of_row.as<int32_t>(),
-                   s->sort_tmp, s->st);
+                   s->present.as<uint32_t>(), s->fd.S, tm, s->row_of_center.as<int32_t>(),
+                   s->center_of_row.as<int32_t>(), s->tile_mask.as<uint32_t>(), s->sort_tmp, s->st);
 }
 
 void compute_features(rgpu_calculator * c, rgpu_structures * s, int precision, bool grads,
@@ -513,7 +535,8 @@ void compute_features(rgpu_calculator * c, rgpu_structures * s, int precision, b
   }
   s->fwd_model = nullptr;
   mark(s, 2);
-  sort_rows(s);
+  const bool by_mask = precision == RGPU_PRECISION_FP32 && sorts_by_mask(c, s);
+  sort_rows(s, by_mask);
   const int64_t nc = s->nl.n_centers;
   const FeatureDims & fd = s->fd;
   ExpansionArgs ea = exp_args(c, s);
@@ -535,7 +558,7 @@ void compute_features(rgpu_calculator * c, rgpu_structures * s, int precision, b
   } else {
     s->C32.ensure(sizeof(float) * size_t(nc) * fd.S * fd.n * row_stride(fd.L) + 64);
     launch_expansion_fp32(ea, s->C32.as<float>(), s->present.as<uint32_t>(), s->st);
-    if (c->hy.kind == "sphericalinvariants") sort_rows_by_mask(s);
+    if (by_mask) sort_rows_by_mask(s);
     mark(s, 3);
     if (c->hy.kind == "sphericalinvariants") {
       if (need_x32) s->X32.ensure(sizeof(float) * size_t(nc) * fd.Dg + 64);
@@ -827,7 +850,7 @@ void gap_plain(rgpu_gap_model * m, rgpu_structures * s, double * E_d, double * F
         launch_fill_f64(s->t64.as<double>() + size_t(g.row0[sI]) * fd.Dpad, g.rows[sI] * fd.Dpad, 0., st);
   }
   // struct of each sorted row
-  launch_energy_reduce(nc, 0, nullptr, 0, s->erow64.as<double>(), 0, s->center_of_row.as<int32_t>(),
+  launch_energy_reduce(nc, EnergyParts{}, nullptr, s->erow64.as<double>(), s->center_of_row.as<int32_t>(),
                        s->nl.center_struct, E_d, st);
   mark(s, 5);
   mark(s, 6);
@@ -858,22 +881,6 @@ std::vector<int64_t> w_offsets(const rgpu_gap_model * m, const rgpu_structures *
     woff += s->species_count[sI] * m->segs[sI].Mpad;
   }
   return wofs;
-}
-
-// Rows and 128-row tiles of each central species (rows in species order).
-TileMaskArgs tile_mask_args(const rgpu_structures * s) {
-  TileMaskArgs a{};
-  a.S = s->fd.S;
-  int64_t r = 0, t = 0;
-  for (int sI = 0; sI < s->fd.S; ++sI) {
-    a.row0[sI] = r;
-    a.rows[sI] = s->species_count[sI];
-    a.tile_off[sI] = t;
-    r += s->species_count[sI];
-    t += (s->species_count[sI] + 127) / 128;
-  }
-  a.tile_off[s->fd.S] = t;
-  return a;
 }
 
 // Species skipping of a grouped GEMM over the packed columns (mode 1: K, the
@@ -911,12 +918,7 @@ void gap_fast_forward(rgpu_gap_model * m, rgpu_structures * s, double * E_d, boo
   s->Wl.ensure(sizeof(uint16_t) * size_t(std::max<int64_t>(wtot, 1)) + 64);
   s->epart.ensure(sizeof(float) * size_t(std::max<int64_t>(eparts, 1)) + 64);
   if (need_w) s->dX32.ensure(sizeof(float) * size_t(nc) * fd.Dg + 64);
-  // species present in each 128-row tile (rows sorted by species and mask)
   const TileMaskArgs tm = tile_mask_args(s);
-  if (fd.G > 1) {
-    s->tile_mask.ensure(sizeof(uint32_t) * size_t(std::max<int64_t>(tm.tile_off[fd.S], 1)) + 64);
-    launch_tile_masks(tm, s->center_of_row.as<int32_t>(), s->present.as<uint32_t>(), s->tile_mask.as<uint32_t>(), st);
-  }
   const __nv_bfloat16 * Xh = s->Xh.as<__nv_bfloat16>();
   const __nv_bfloat16 * Xl = s->Xl.as<__nv_bfloat16>();
   __nv_bfloat16 * Wh = s->Wh.as<__nv_bfloat16>();
@@ -952,18 +954,28 @@ void gap_fast_forward(rgpu_gap_model * m, rgpu_structures * s, double * E_d, boo
     row0 += rows;
   }
   gemm_bf16x3_grouped(fwd.data(), int(fwd.size()), st, tile_config(fd.S, fd.n, fd.L).gemm_variant, tile_n);
-  row0 = 0;
+  EnergyParts ep;
+  ep.S = fd.S;
   for (int sI = 0; sI < fd.S; ++sI) {
-    const int64_t rows = s->species_count[sI];
-    const GapSpecies & g = m->segs[sI];
-    if (rows > 0 && g.M > 0) {
-      const int nparts = (g.M + tile_n - 1) / tile_n;
-      launch_energy_reduce(rows, nparts, s->epart.as<float>() + eofs[sI], rows, nullptr, row0,
-                           s->center_of_row.as<int32_t>(), s->nl.center_struct, E_d, st);
-    }
-    row0 += rows;
+    ep.row0[sI + 1] = ep.row0[sI] + s->species_count[sI];
+    ep.ofs[sI] = eofs[sI];
+    ep.parts[sI] = (points[sI] + tile_n - 1) / tile_n;
   }
+  launch_energy_reduce(nc, ep, s->epart.as<float>(), nullptr, s->center_of_row.as<int32_t>(), s->nl.center_struct,
+                       E_d, st);
   mark(s, 5);
+}
+
+// The power-spectrum backward's chunk map depends on the layout alone: written
+// when the layout changes, also before the replay of a graph recorded with
+// another one than the last call's.
+void ensure_chunk_map(rgpu_structures * s, const FeatureDims & fd) {
+  if (s->chunk_map_of[0] == fd.S && s->chunk_map_of[1] == fd.n && s->chunk_map_of[2] == fd.L) return;
+  s->chunk_map.ensure(sizeof(uint32_t) * size_t(fd.Dg / 4) + 64);
+  launch_chunk_map(fd, s->chunk_map.as<uint32_t>(), s->st);
+  s->chunk_map_of[0] = fd.S;
+  s->chunk_map_of[1] = fd.n;
+  s->chunk_map_of[2] = fd.L;
 }
 
 // Fast path, backward half: dE/dx = W T (grouped GEMM), the power-spectrum
@@ -1018,7 +1030,7 @@ void gap_fast_backward(rgpu_gap_model * m, rgpu_structures * s, double * F_d, do
   pa.normalize = c->hy.normalize;
   pa.row_of_center = s->row_of_center.as<int32_t>();
   s->dC32.ensure(sizeof(float) * size_t(nc) * fd.S * fd.nK + 64);
-  s->chunk_map.ensure(sizeof(uint32_t) * size_t(fd.Dg / 4) + 64);
+  ensure_chunk_map(s, fd);
   launch_ps_bwd_fp32(pa, s->C32.as<float>(), Xh, Xl, s->xscale32.as<float>(), s->dX32.as<float>(),
                      s->chunk_map.as<uint32_t>(), s->present.as<uint32_t>(), s->dC32.as<float>(), st);
   if (struct_scale)
@@ -1397,7 +1409,7 @@ static std::vector<const void *> md_buffers(const rgpu_gap_model * m, const rgpu
   std::vector<const void *> v;
   for (const DevBuf * b : {&s->atom_off_d, &s->pos_d, &s->types_d, &s->cells_d, &s->pbc_d, &s->tag2idx_d,
                            &s->ncent_d, &s->center_off_d, &s->atom_struct_d, &s->lut, &s->row_of_center,
-                           &s->center_of_row, &s->species_count_d, &s->sort_tmp, &s->present, &s->tile_mask,
+                           &s->center_of_row, &s->sort_tmp, &s->present, &s->tile_mask,
                            &s->C64, &s->X64,
                            &s->invn64, &s->dC64, &s->C32, &s->X32, &s->xscale32, &s->E_d, &s->F_d, &s->S_d, &s->K64,
                            &s->t64, &s->erow64, &s->Wh, &s->Wl, &s->dX32, &s->dC32, &s->epart, &s->Xh, &s->Xl,
@@ -1405,8 +1417,8 @@ static std::vector<const void *> md_buffers(const rgpu_gap_model * m, const rgpu
     v.push_back(b->p);
   const NlWork & w = s->nlw;
   for (const DevBuf * b : {&w.geom, &w.counts64, &w.scan_tmp, &w.ghost_off, &w.site_x, &w.site_type, &w.site_real,
-                           &w.site_shift, &w.site_box, &w.box_base, &w.box_count, &w.box_ptr, &w.box_fill,
-                           &w.sorted, &w.sorted_x, &w.sorted_info, &w.pair_count, &w.center_atom,
+                           &w.site_shift, &w.site_box, &w.box_base, &w.box_count, &w.box_ptr, &w.binned,
+                           &w.sorted, &w.sorted_x, &w.pair_count, &w.center_atom,
                            &w.center_struct, &w.pair_off, &w.pair_j, &w.pair_shift, &w.pair_dist, &w.pair_dir,
                            &w.pair_center})
     v.push_back(b->p);
@@ -1451,7 +1463,8 @@ static void graph_enqueue(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   in.n_centers_total = s->center_off_h[s->n_struct];
   build_neighbour_list(in, c->hy.cutoff, s->nlw, s->nl, s->status_d, s->status_h, st, &caps);
   // features (the FP32 branch of compute_features, layout unchanged)
-  sort_rows(s);
+  const bool by_mask = sorts_by_mask(c, s);
+  sort_rows(s, by_mask);
   const int64_t nc = s->nl.n_centers;
   const FeatureDims & fd = s->fd;
   ExpansionArgs ea = exp_args(c, s);
@@ -1461,7 +1474,7 @@ static void graph_enqueue(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   pa.normalize = c->hy.normalize;
   pa.row_of_center = s->row_of_center.as<int32_t>();
   launch_expansion_fp32(ea, s->C32.as<float>(), s->present.as<uint32_t>(), st);
-  sort_rows_by_mask(s);
+  if (by_mask) sort_rows_by_mask(s);
   pa.present = s->present.as<uint32_t>();
   launch_ps_fwd_fast(pa, s->C32.as<float>(), nullptr, s->Xh.as<__nv_bfloat16>(), s->Xl.as<__nv_bfloat16>(),
                      s->xscale32.as<float>(), st);
@@ -1541,6 +1554,7 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
   }
   if (replay) {
     std::memcpy(s->md_pos_h, positions, sizeof(double) * 3 * na);
+    ensure_chunk_map(s, make_dims(m->calc->hy, int(s->species.size())));
     RGPU_CUDA(cudaGraphLaunch(s->md_exec, s->st));
     RGPU_CUDA(cudaStreamSynchronize(s->st));
     ++s->md_replays;
@@ -1689,6 +1703,7 @@ static bool pgraph_replay(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
     if (bufs.empty()) bufs = md_buffers(m, s);
     if (g.buffers != bufs) continue;
     s->timed = false;
+    if (g.forces) ensure_chunk_map(s, s->fd);
     RGPU_CUDA(cudaGraphLaunch(g.exec, s->st));
     RGPU_CUDA(cudaStreamSynchronize(s->st));
     // the list on the device is the capacity-bound one: nothing computed here

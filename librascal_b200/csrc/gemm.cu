@@ -227,9 +227,8 @@ gemm_tf32_kernel(Tf32GemmArgs g) {
   }
 }
 
-__global__ void energy_reduce_kernel(int64_t rows, int n_parts, const float * __restrict__ e_part,
-                                     int64_t ld, const double * __restrict__ e_row, int64_t row0,
-                                     const int32_t * __restrict__ center_of_row,
+__global__ void energy_reduce_kernel(int64_t rows, EnergyParts parts, const float * __restrict__ e_part,
+                                     const double * __restrict__ e_row, const int32_t * __restrict__ center_of_row,
                                      const int32_t * __restrict__ center_struct,
                                      double * __restrict__ E) {
   const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -239,9 +238,13 @@ __global__ void energy_reduce_kernel(int64_t rows, int n_parts, const float * __
     if (e_row) {
       e = e_row[r];
     } else {
-      for (int t = 0; t < n_parts; ++t) e += double(e_part[int64_t(t) * ld + r]);
+      int s = 0;
+      while (r >= parts.row0[s + 1]) ++s;
+      const int64_t ld = parts.row0[s + 1] - parts.row0[s];
+      const float * p = e_part + parts.ofs[s] + (r - parts.row0[s]);
+      for (int t = 0; t < parts.parts[s]; ++t) e += double(p[int64_t(t) * ld]);
     }
-    key = center_struct[center_of_row[row0 + r]];
+    key = center_struct[center_of_row[r]];
   }
   // the warp's rows of one structure are summed first, so a structure with
   // many centres (one large box) takes one atomic per warp, not per row
@@ -328,12 +331,12 @@ void gemm_tf32(const Tf32GemmArgs & g, cudaStream_t st) {
   RGPU_CUDA(cudaGetLastError());
 }
 
-void launch_energy_reduce(int64_t rows, int n_parts, const float * e_part, int64_t ld,
-                          const double * e_row_fp64, int64_t row0, const int32_t * center_of_row,
-                          const int32_t * center_struct, double * energies, cudaStream_t st) {
+void launch_energy_reduce(int64_t rows, const EnergyParts & parts, const float * e_part, const double * e_row_fp64,
+                          const int32_t * center_of_row, const int32_t * center_struct, double * energies,
+                          cudaStream_t st) {
   if (rows <= 0) return;
-  energy_reduce_kernel<<<div_up(rows, 256), 256, 0, st>>>(rows, n_parts, e_part, ld, e_row_fp64, row0,
-                                                         center_of_row, center_struct, energies);
+  energy_reduce_kernel<<<div_up(rows, 256), 256, 0, st>>>(rows, parts, e_part, e_row_fp64, center_of_row,
+                                                         center_struct, energies);
   RGPU_LAUNCHED();
 }
 

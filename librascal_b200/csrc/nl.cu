@@ -16,6 +16,7 @@
 // pair sets, distances and directions are bit-identical to it.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 
@@ -44,13 +45,9 @@ __device__ void inv3(const double * m, double * r) {
   r[8] = (m[0] * m[4] - m[1] * m[3]) * inv;
 }
 
-__global__ void nl_setup_kernel(int n_struct, const int64_t * __restrict__ atom_off,
-                                const double * __restrict__ cells, const int32_t * __restrict__ pbc,
-                                const int32_t * __restrict__ n_centers, double cutoff,
-                                NlGeom * __restrict__ geom, int64_t * __restrict__ nbox,
-                                DevStatus * st) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n_struct) return;
+__device__ int64_t setup_structure(int s, const int64_t * __restrict__ atom_off, const double * __restrict__ cells,
+                                   const int32_t * __restrict__ pbc, const int32_t * __restrict__ n_centers,
+                                   double cutoff, NlGeom * __restrict__ geom, DevStatus * st) {
   NlGeom g;
   bool zero = true;
   for (int i = 0; i < 3; ++i)
@@ -61,10 +58,18 @@ __global__ void nl_setup_kernel(int n_struct, const int64_t * __restrict__ atom_
   g.n_atoms = int(atom_off[s + 1] - atom_off[s]);
   g.n_centers = n_centers[s];
   if (zero) {
+    // an empty mesh of 27 boxes without images keeps what follows in bounds
     set_status(st, 100, s, 0);
-    nbox[s] = 1;
+    for (int i = 0; i < 9; ++i) g.cinv[i] = 0.;
+    for (int i = 0; i < 3; ++i) {
+      g.mesh_min[i] = g.ghost_min[i] = g.ghost_max[i] = 0.;
+      g.nboxes[i] = 3;
+      g.pmin[i] = 0;
+      g.reps[i] = 1;
+    }
+    g.bound_tol = 0.;
     geom[s] = g;
-    return;
+    return 27;
   }
   inv3(g.cell, g.cinv);
   for (int i = 0; i < 3; ++i) {
@@ -106,23 +111,37 @@ __global__ void nl_setup_kernel(int n_struct, const int64_t * __restrict__ atom_
     g.reps[i] = -g.pmin[i] + pmax + 1;
   }
   geom[s] = g;
-  nbox[s] = int64_t(g.nboxes[0]) * g.nboxes[1] * g.nboxes[2];
+  return int64_t(g.nboxes[0]) * g.nboxes[1] * g.nboxes[2];
 }
 
-__global__ void nl_check_kernel(int64_t n_atoms, const int32_t * __restrict__ atom_struct,
-                                const double * __restrict__ pos, const int32_t * __restrict__ types,
-                                const NlGeom * __restrict__ geom, DevStatus * st) {
-  int64_t a = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (a >= n_atoms) return;
-  int s = atom_struct[a];
-  int t = types[a];
-  if (t < 0 || t >= 130) set_status(st, 101, s, t);
-  const NlGeom & g = geom[s];
-  double x = pos[3 * a], y = pos[3 * a + 1], z = pos[3 * a + 2];
-  for (int i = 0; i < 3; ++i) {
-    double v = g.cinv[i * 3 + 0] * x + g.cinv[i * 3 + 1] * y + g.cinv[i * 3 + 2] * z;
-    if (v < -1e-10 || v > 1. + 1e-10) set_status(st, 102, s, int(a));
+// Geometry and box count of every structure. One block also scans the counts
+// into box_base (box_base[n_struct] = the total); more structures than it has
+// threads leave the counts in nbox for a scan of their own.
+constexpr int kSetupBlock = 512;
+__global__ void __launch_bounds__(kSetupBlock)
+nl_setup_kernel(int n_struct, const int64_t * __restrict__ atom_off, const double * __restrict__ cells,
+                const int32_t * __restrict__ pbc, const int32_t * __restrict__ n_centers, double cutoff,
+                NlGeom * __restrict__ geom, int64_t * __restrict__ nbox, int64_t * __restrict__ box_base,
+                DevStatus * st) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t n = s < n_struct ? setup_structure(s, atom_off, cells, pbc, n_centers, cutoff, geom, st) : 0;
+  if (gridDim.x > 1) {
+    if (s < n_struct) nbox[s] = n;
+    return;
   }
+  __shared__ int64_t warp_tot[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int64_t x = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warp_tot[wid] = x;
+  __syncthreads();
+  for (int w = 0; w < wid; ++w) x += warp_tot[w];
+  if (s < n_struct) box_base[s] = x - n;
+  if (s == max(n_struct - 1, 0)) box_base[n_struct] = x;
 }
 
 __device__ __forceinline__ void image_of(const NlGeom & g, int k, int p[3]) {
@@ -144,20 +163,39 @@ __device__ __forceinline__ bool ghost_pos(const NlGeom & g, const double * x0, c
   return inside;
 }
 
-__global__ void nl_ghost_count_kernel(int64_t n_atoms, const int32_t * __restrict__ atom_struct,
-                                      const int32_t * __restrict__ tag2idx,
-                                      const double * __restrict__ pos,
-                                      const NlGeom * __restrict__ geom,
-                                      int32_t * __restrict__ count) {
-  int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= n_atoms) return;
-  const NlGeom & g = geom[atom_struct[t]];
-  int ntot = g.reps[0] * g.reps[1] * g.reps[2];
+// kImageLanes lanes share an atom: with 27 and more images per atom of a
+// periodic structure, one thread's loop over them was a chain of 10 to 40 us
+// whatever the batch.
+constexpr int kImageLanes = 8;
+__device__ __forceinline__ unsigned image_group_bits(unsigned ballot) {
+  return (ballot >> ((threadIdx.x & 31) & ~(kImageLanes - 1))) & ((1u << kImageLanes) - 1u);
+}
+
+// Checks the atoms (type, inside the cell) and counts the ghost images of
+// each.
+__global__ void nl_count_kernel(int64_t n_atoms, const int32_t * __restrict__ atom_struct,
+                                const int32_t * __restrict__ tag2idx, const double * __restrict__ pos,
+                                const int32_t * __restrict__ types, const NlGeom * __restrict__ geom,
+                                int32_t * __restrict__ count, DevStatus * st) {
+  const int64_t t = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / kImageLanes;
+  const int sub = threadIdx.x & (kImageLanes - 1);
+  const bool on = t < n_atoms;
+  const int s = on ? atom_struct[t] : 0;
+  const NlGeom & g = geom[s];
+  const int64_t a = on ? (tag2idx ? tag2idx[t] : t) : 0;
+  const double x0[3] = {pos[3 * a], pos[3 * a + 1], pos[3 * a + 2]};
+  if (on && sub == 0) {
+    const int ty = types[a];
+    if (ty < 0 || ty >= 130) set_status(st, 101, s, ty);
+    for (int i = 0; i < 3; ++i) {
+      double v = g.cinv[i * 3 + 0] * x0[0] + g.cinv[i * 3 + 1] * x0[1] + g.cinv[i * 3 + 2] * x0[2];
+      if (v < -1e-10 || v > 1. + 1e-10) set_status(st, 102, s, int(a));
+    }
+  }
+  const int ntot = on ? g.reps[0] * g.reps[1] * g.reps[2] : 1;
   int c = 0;
   if (ntot > 1) {
-    int64_t a = tag2idx ? tag2idx[t] : t;
-    double x0[3] = {pos[3 * a], pos[3 * a + 1], pos[3 * a + 2]};
-    for (int k = 0; k < ntot; ++k) {
+    for (int k = sub; k < ntot; k += kImageLanes) {
       int p[3];
       image_of(g, k, p);
       if (p[0] == 0 && p[1] == 0 && p[2] == 0) continue;
@@ -165,7 +203,9 @@ __global__ void nl_ghost_count_kernel(int64_t n_atoms, const int32_t * __restric
       if (ghost_pos(g, x0, p, gp)) ++c;
     }
   }
-  count[t] = c;
+#pragma unroll
+  for (int o = kImageLanes / 2; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  if (on && sub == 0) count[t] = c;
 }
 
 __device__ __forceinline__ bool box_of(const NlGeom & g, const double * x, double cutoff,
@@ -191,16 +231,17 @@ __global__ void nl_sites_kernel(int64_t n_atoms, const int64_t * __restrict__ at
                                 int32_t * __restrict__ site_real, int32_t * __restrict__ site_shift,
                                 int64_t * __restrict__ site_box, int32_t * __restrict__ box_count,
                                 DevStatus * st, int64_t site_cap, int64_t box_cap) {
-  int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= n_atoms) return;
-  int s = atom_struct[t];
+  const int64_t t = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / kImageLanes;
+  const int sub = threadIdx.x & (kImageLanes - 1);
+  const bool on = t < n_atoms;
+  const int s = on ? atom_struct[t] : 0;
   const NlGeom & g = geom[s];
-  int64_t a0 = atom_off[s];
-  int64_t gbase = ghost_off[a0];
-  int64_t site_base = a0 + gbase;
-  int64_t a = tag2idx ? tag2idx[t] : t;
-  double x0[3] = {pos[3 * a], pos[3 * a + 1], pos[3 * a + 2]};
-  int typ = types[a];
+  const int64_t a0 = atom_off[s];
+  const int64_t gbase = ghost_off[a0];
+  const int64_t site_base = a0 + gbase;
+  const int64_t a = on ? (tag2idx ? tag2idx[t] : t) : 0;
+  const double x0[3] = {pos[3 * a], pos[3 * a + 1], pos[3 * a + 2]};
+  const int typ = types[a];
   auto put = [&](int64_t site, const double * x, const int * p) {
     if (site >= site_cap) {
       set_status(st, 104, s, int(a));  // more sites than the capacity
@@ -228,18 +269,24 @@ __global__ void nl_sites_kernel(int64_t n_atoms, const int64_t * __restrict__ at
     site_box[site] = box;
     atomicAdd(&box_count[box], 1);
   };
-  int zero[3] = {0, 0, 0};
-  put(site_base + (t - a0), x0, zero);
-  int ntot = g.reps[0] * g.reps[1] * g.reps[2];
-  if (ntot > 1) {
-    int64_t slot = site_base + g.n_atoms + (ghost_off[t] - gbase);
-    for (int k = 0; k < ntot; ++k) {
-      int p[3];
+  const int zero[3] = {0, 0, 0};
+  if (on && sub == 0) put(site_base + (t - a0), x0, zero);
+  const int ntot = on ? g.reps[0] * g.reps[1] * g.reps[2] : 1;
+  // the warp's lanes loop together: an atom's ghosts take slots in image order
+  const int steps = __reduce_max_sync(0xffffffffu, ntot > 1 ? (ntot + kImageLanes - 1) / kImageLanes : 0);
+  int64_t slot = on ? site_base + g.n_atoms + (ghost_off[t] - gbase) : 0;
+  for (int i = 0; i < steps; ++i) {
+    const int k = i * kImageLanes + sub;
+    int p[3] = {0, 0, 0};
+    double gp[3];
+    bool is = ntot > 1 && k < ntot;
+    if (is) {
       image_of(g, k, p);
-      if (p[0] == 0 && p[1] == 0 && p[2] == 0) continue;
-      double gp[3];
-      if (ghost_pos(g, x0, p, gp)) put(slot++, gp, p);
+      is = !(p[0] == 0 && p[1] == 0 && p[2] == 0) && ghost_pos(g, x0, p, gp);
     }
+    const unsigned bits = image_group_bits(__ballot_sync(0xffffffffu, is));
+    if (is) put(slot + __popc(bits & ((1u << sub) - 1u)), gp, p);
+    slot += __popc(bits);
   }
 }
 
@@ -253,43 +300,52 @@ __device__ __forceinline__ int64_t site_count(int64_t n_sites, const int64_t * g
 
 __global__ void nl_scatter_kernel(int64_t n_sites, const int64_t * __restrict__ site_box,
                                   const int64_t * __restrict__ box_ptr,
-                                  int32_t * __restrict__ box_fill, int64_t * __restrict__ sorted,
+                                  int32_t * __restrict__ box_count, int64_t * __restrict__ binned,
                                   const int64_t * __restrict__ ghosts_dev, int64_t n_atoms) {
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= site_count(n_sites, ghosts_dev, n_atoms)) return;
   int64_t b = site_box[i];
   if (b < 0) return;  // a site past the box capacity
-  int64_t slot = box_ptr[b] + atomicAdd(&box_fill[b], 1);
-  sorted[slot] = i;
+  // the counts are used up from the top; the order inside a box is made below
+  binned[box_ptr[b] + atomicSub(&box_count[b], 1) - 1] = i;
 }
 
-// Ascending site (= tag) order inside every box, then pack positions.
-__global__ void nl_boxsort_kernel(int64_t n_boxes, const int64_t * __restrict__ box_ptr,
-                                  int64_t * __restrict__ sorted) {
-  int64_t b = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (b >= n_boxes) return;  // boxes past the used ones (capacity mode) are empty
-  int64_t lo = box_ptr[b], hi = box_ptr[b + 1];
-  for (int64_t i = lo + 1; i < hi; ++i) {
-    int64_t v = sorted[i];
-    int64_t j = i - 1;
-    while (j >= lo && sorted[j] > v) {
-      sorted[j + 1] = sorted[j];
-      --j;
+// Ascending site (= tag) order inside every box, with the positions packed in
+// that order. A warp takes `per` boxes and sorts the occupied ones by rank, one
+// lane per site (a thread per box was an insertion sort in global memory).
+// One box per warp where the boxes are few, 32 where they are many and mostly
+// empty: at 1 000 boxes of a dense cell 32 took 18 to 23 us, a chain of 32.
+__global__ void nl_boxsort_kernel(int64_t n_boxes, int per, const int64_t * __restrict__ box_ptr,
+                                  const int64_t * __restrict__ binned, const double * __restrict__ site_x,
+                                  int64_t * __restrict__ sorted, double * __restrict__ sorted_x) {
+  const int lane = threadIdx.x & 31;
+  const int64_t b = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * per + lane;
+  // boxes past the used ones (capacity mode) are empty
+  const bool mine = lane < per && b < n_boxes;
+  const int64_t lo = mine ? box_ptr[b] : 0, hi = mine ? box_ptr[b + 1] : 0;
+  unsigned todo = __ballot_sync(0xffffffffu, hi > lo);
+  auto place = [&](int64_t at, int64_t site) {
+    sorted[at] = site;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) sorted_x[3 * at + k] = site_x[3 * site + k];
+  };
+  while (todo) {
+    const int src = __ffs(int(todo)) - 1;
+    todo &= todo - 1;
+    const int64_t l = __shfl_sync(0xffffffffu, lo, src);
+    const int m = int(__shfl_sync(0xffffffffu, hi, src) - l);
+    for (int i0 = 0; i0 < m; i0 += 32) {
+      const bool has = i0 + lane < m;
+      const int64_t v = has ? binned[l + i0 + lane] : 0;
+      int rank = 0;
+      for (int j0 = 0; j0 < m; j0 += 32) {
+        const int n = min(32, m - j0);
+        const int64_t o = j0 == i0 ? v : (lane < n ? binned[l + j0 + lane] : 0);
+        for (int j = 0; j < n; ++j) rank += __shfl_sync(0xffffffffu, o, j) < v;
+      }
+      if (has) place(l + rank, v);
     }
-    sorted[j + 1] = v;
   }
-}
-
-__global__ void nl_pack_kernel(int64_t n_sites, const int64_t * __restrict__ sorted,
-                               const double * __restrict__ site_x, double * __restrict__ sorted_x,
-                               const int64_t * __restrict__ box_total) {
-  int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  // the binned sites (box_ptr's total): all sites unless some overflowed
-  if (i >= n_sites || (box_total && i >= *box_total)) return;
-  int64_t s = sorted[i];
-  sorted_x[3 * i + 0] = site_x[3 * s + 0];
-  sorted_x[3 * i + 1] = site_x[3 * s + 1];
-  sorted_x[3 * i + 2] = site_x[3 * s + 2];
 }
 
 struct GatherCtx {
@@ -346,7 +402,6 @@ __global__ void nl_gather_kernel(int64_t n_centers, GatherCtx c, int64_t * __res
       if (lane == 0) set_status(c.status, 104, s, int(ci));
       return;
     }
-    if (pair_off[ci + 1] > c.pair_cap && lane == 0) set_status(c.status, 104, s, int(ci));
     if (lane == 0) {
       center_atom[ci] = site_real[site];
       pair_j[base] = site_real[site];
@@ -441,14 +496,6 @@ __global__ void center_struct_kernel(int n_struct, const int64_t * __restrict__ 
     center_struct[i] = s;
 }
 
-// Capacity mode: offsets past the pair capacity are clamped to it, so that
-// every later per-centre loop stays inside the pair buffers even when the
-// list overflowed (status 104 then tells the caller to rebuild).
-__global__ void nl_clamp_offsets_kernel(int64_t n, int64_t * __restrict__ pair_off, int64_t cap) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n && pair_off[i] > cap) pair_off[i] = cap;
-}
-
 }  // namespace
 
 void neighbour_list_counts(const NlWork & w, int64_t & sites, int64_t & boxes) {
@@ -507,20 +554,20 @@ void build_neighbour_list(const NlInputs & in, double cutoff, NlWork & w, NlOutp
   w.counts64.ensure(sizeof(int64_t) * (S + 1));
   w.box_base.ensure(sizeof(int64_t) * (S + 1));
   NlGeom * geom = w.geom.as<NlGeom>();
-  nl_setup_kernel<<<div_up(S, 128), 128, 0, st>>>(S, in.atom_off, in.cells, in.pbc, in.n_centers,
-                                                  cutoff, geom, w.counts64.as<int64_t>(), status_dev);
+  nl_setup_kernel<<<std::max(1, div_up(S, kSetupBlock)), kSetupBlock, 0, st>>>(
+      S, in.atom_off, in.cells, in.pbc, in.n_centers, cutoff, geom, w.counts64.as<int64_t>(),
+      w.box_base.as<int64_t>(), status_dev);
   RGPU_LAUNCHED();
   if (!caps) check_status("setup");
-  nl_check_kernel<<<div_up(N, kThreads), kThreads, 0, st>>>(N, in.atom_struct, in.pos, in.types,
-                                                            geom, status_dev);
-  RGPU_LAUNCHED();
-  scan_exclusive_i64(w.counts64.as<int64_t>(), w.box_base.as<int64_t>(), S, w.scan_tmp, st);
+  if (S > kSetupBlock)
+    scan_exclusive_i64(w.counts64.as<int64_t>(), w.box_base.as<int64_t>(), S, w.scan_tmp, st);
 
-  // 2. ghost images
+  // 2. input checks and ghost images
   w.pair_count.ensure(sizeof(int32_t) * (N + 1));
   w.ghost_off.ensure(sizeof(int64_t) * (N + 1));
-  nl_ghost_count_kernel<<<div_up(N, kThreads), kThreads, 0, st>>>(
-      N, in.atom_struct, in.tag2idx, in.pos, geom, w.pair_count.as<int32_t>());
+  const int atoms_per_block = kThreads / kImageLanes;
+  nl_count_kernel<<<div_up(N, atoms_per_block), kThreads, 0, st>>>(
+      N, in.atom_struct, in.tag2idx, in.pos, in.types, geom, w.pair_count.as<int32_t>(), status_dev);
   RGPU_LAUNCHED();
   scan_exclusive_i32to64(w.pair_count.as<int32_t>(), w.ghost_off.as<int64_t>(), N, w.scan_tmp, st);
   int64_t n_sites = 0, n_boxes = 0;
@@ -550,29 +597,26 @@ void build_neighbour_list(const NlInputs & in, double cutoff, NlWork & w, NlOutp
   w.site_shift.ensure(sizeof(int32_t) * 3 * n_sites);
   w.site_box.ensure(sizeof(int64_t) * n_sites);
   w.box_count.ensure(sizeof(int32_t) * (n_boxes + 1));
-  w.box_fill.ensure(sizeof(int32_t) * (n_boxes + 1));
   w.box_ptr.ensure(sizeof(int64_t) * (n_boxes + 1));
   RGPU_CUDA(cudaMemsetAsync(w.box_count.p, 0, sizeof(int32_t) * (n_boxes + 1), st));
-  RGPU_CUDA(cudaMemsetAsync(w.box_fill.p, 0, sizeof(int32_t) * (n_boxes + 1), st));
-  nl_sites_kernel<<<div_up(N, kThreads), kThreads, 0, st>>>(
+  nl_sites_kernel<<<div_up(N, atoms_per_block), kThreads, 0, st>>>(
       N, in.atom_off, in.atom_struct, in.tag2idx, in.pos, in.types, geom, w.ghost_off.as<int64_t>(),
       w.box_base.as<int64_t>(), cutoff, w.site_x.as<double>(), w.site_type.as<int32_t>(),
       w.site_real.as<int32_t>(), w.site_shift.as<int32_t>(), w.site_box.as<int64_t>(),
       w.box_count.as<int32_t>(), status_dev, n_sites, n_boxes);
   RGPU_LAUNCHED();
   scan_exclusive_i32to64(w.box_count.as<int32_t>(), w.box_ptr.as<int64_t>(), n_boxes, w.scan_tmp, st);
+  w.binned.ensure(sizeof(int64_t) * n_sites);
   w.sorted.ensure(sizeof(int64_t) * n_sites);
   w.sorted_x.ensure(sizeof(double) * 3 * n_sites);
   nl_scatter_kernel<<<div_up(n_sites, kThreads), kThreads, 0, st>>>(
-      n_sites, w.site_box.as<int64_t>(), w.box_ptr.as<int64_t>(), w.box_fill.as<int32_t>(),
-      w.sorted.as<int64_t>(), ghosts_dev, N);
+      n_sites, w.site_box.as<int64_t>(), w.box_ptr.as<int64_t>(), w.box_count.as<int32_t>(),
+      w.binned.as<int64_t>(), ghosts_dev, N);
   RGPU_LAUNCHED();
-  nl_boxsort_kernel<<<div_up(n_boxes, kThreads), kThreads, 0, st>>>(n_boxes, w.box_ptr.as<int64_t>(),
-                                                                   w.sorted.as<int64_t>());
-  RGPU_LAUNCHED();
-  nl_pack_kernel<<<div_up(n_sites, kThreads), kThreads, 0, st>>>(
-      n_sites, w.sorted.as<int64_t>(), w.site_x.as<double>(), w.sorted_x.as<double>(),
-      caps ? w.box_ptr.as<int64_t>() + n_boxes : nullptr);
+  const int per = n_boxes <= 65536 ? 1 : 32;
+  nl_boxsort_kernel<<<div_up(div_up(n_boxes, per), kThreads / 32), kThreads, 0, st>>>(
+      n_boxes, per, w.box_ptr.as<int64_t>(), w.binned.as<int64_t>(), w.site_x.as<double>(), w.sorted.as<int64_t>(),
+      w.sorted_x.as<double>());
   RGPU_LAUNCHED();
   // The binning status (an atom outside every bin) is read with the pair
   // count below: the binning kernels clamp their box indices, so everything
@@ -580,16 +624,20 @@ void build_neighbour_list(const NlInputs & in, double cutoff, NlWork & w, NlOutp
 
   // 4. centres: structure of each centre row
   const int64_t n_centers = in.n_centers_total;
-  w.center_struct.ensure(sizeof(int32_t) * (n_centers + 1));
   w.center_atom.ensure(sizeof(int32_t) * (n_centers + 1));
-  center_struct_kernel<<<S, 128, 0, st>>>(S, in.center_off, w.center_struct.as<int32_t>());
-  RGPU_LAUNCHED();
+  const int32_t * center_struct = in.atom_struct;  // without a mask the centres are the atoms
+  if (in.tag2idx) {
+    w.center_struct.ensure(sizeof(int32_t) * (n_centers + 1));
+    center_struct_kernel<<<S, 128, 0, st>>>(S, in.center_off, w.center_struct.as<int32_t>());
+    RGPU_LAUNCHED();
+    center_struct = w.center_struct.as<int32_t>();
+  }
 
   // 5. count, scan, fill
   GatherCtx c;
   c.atom_off = in.atom_off;
   c.center_off = in.center_off;
-  c.center_struct_in = w.center_struct.as<int32_t>();
+  c.center_struct_in = center_struct;
   c.geom = geom;
   c.ghost_off = w.ghost_off.as<int64_t>();
   c.box_base = w.box_base.as<int64_t>();
@@ -612,7 +660,10 @@ void build_neighbour_list(const NlInputs & in, double cutoff, NlWork & w, NlOutp
                                                    nullptr, nullptr, nullptr, nullptr);
     RGPU_LAUNCHED();
   }
-  scan_exclusive_i64(w.counts64.as<int64_t>(), w.pair_off.as<int64_t>(), n_centers, w.scan_tmp, st);
+  // capacity mode: offsets past the pair capacity are clamped to it (and set
+  // status 104), so that every later per-centre loop stays inside the buffers
+  scan_exclusive_i64(w.counts64.as<int64_t>(), w.pair_off.as<int64_t>(), n_centers, w.scan_tmp, st,
+                     caps ? ScanCap{status_dev, caps->pairs} : ScanCap{});
   int64_t n_pairs = 0;
   if (caps) {
     n_pairs = caps->pairs;
@@ -635,15 +686,10 @@ void build_neighbour_list(const NlInputs & in, double cutoff, NlWork & w, NlOutp
         w.pair_dir.as<double>(), w.pair_center.as<int32_t>());
     RGPU_LAUNCHED();
   }
-  if (caps) {
-    nl_clamp_offsets_kernel<<<div_up(n_centers + 1, kThreads), kThreads, 0, st>>>(
-        n_centers + 1, w.pair_off.as<int64_t>(), n_pairs);
-    RGPU_LAUNCHED();
-  }
   out.n_centers = n_centers;
   out.n_pairs = n_pairs;
   out.center_atom = w.center_atom.as<int32_t>();
-  out.center_struct = w.center_struct.as<int32_t>();
+  out.center_struct = center_struct;
   out.pair_off = w.pair_off.as<int64_t>();
   out.pair_j = w.pair_j.as<int32_t>();
   out.pair_center = w.pair_center.as<int32_t>();

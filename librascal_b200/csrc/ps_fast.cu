@@ -567,14 +567,17 @@ void launch_ps_fwd_fast(const PsArgs & a, const float * C, float * X, __nv_bfloa
     launch_ps_fwd_fp32(a, C, X, Xh, Xl, row_scale, st);
 }
 
+void launch_chunk_map(const FeatureDims & fd, uint32_t * chunk_map, cudaStream_t st) {
+  chunk_map_kernel<<<div_up(fd.Dg / 4, 256), 256, 0, st>>>(fd, chunk_map);
+  RGPU_LAUNCHED();
+  RGPU_CUDA(cudaGetLastError());
+}
+
 void launch_ps_bwd_fp32(const PsArgs & a, const float * C, const __nv_bfloat16 * Xh, const __nv_bfloat16 * Xl,
-                        const float * row_scale, const float * dX, uint32_t * chunk_map, const uint32_t * present,
-                        float * dC, cudaStream_t st) {
+                        const float * row_scale, const float * dX, const uint32_t * chunk_map,
+                        const uint32_t * present, float * dC, cudaStream_t st) {
   if (a.n_centers == 0) return;
   if (a.fd.n > kMaxN) throw Error(RGPU_ERR_INVALID_ARGUMENT, "max_radial above 16 is not supported on the fast path");
-  const int nchunk = a.fd.Dg / 4;
-  chunk_map_kernel<<<div_up(nchunk, 256), 256, 0, st>>>(a.fd, chunk_map);
-  RGPU_LAUNCHED();
   constexpr size_t kMaxSmem = 227 * 1024 - 2048;
   const int threads = std::min(tile_config(a.fd.S, a.fd.n, a.fd.L).psb_threads, kBwdThreads);
 #define RGPU_PSB_CASE(LL)                                                                                     \

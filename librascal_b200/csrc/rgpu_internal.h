@@ -131,9 +131,15 @@ struct DevStatus {
 };
 
 // ------------------------------------------------------------------ scans
+// Largest value a scan may write (with a status word: larger ones are
+// clamped to it and set status 104).
+struct ScanCap {
+  DevStatus * status{nullptr};
+  int64_t limit{0};
+};
 // Exclusive prefix sum of n int64 values, out[n] = total. `tmp` scratch.
 void scan_exclusive_i64(const int64_t * in, int64_t * out, int64_t n, DevBuf & tmp,
-                        cudaStream_t st);
+                        cudaStream_t st, ScanCap cap = {});
 void scan_exclusive_i32to64(const int32_t * in, int64_t * out, int64_t n, DevBuf & tmp,
                             cudaStream_t st);
 
@@ -156,7 +162,7 @@ struct NlInputs {
 struct NlOutputs {
   int64_t n_centers{0}, n_pairs{0};
   int32_t * center_atom{nullptr};   // [n_centers] global original index
-  int32_t * center_struct{nullptr}; // [n_centers]
+  const int32_t * center_struct{nullptr}; // [n_centers]
   int64_t * pair_off{nullptr};      // [n_centers+1]
   int32_t * pair_j{nullptr};        // [n_pairs] global original index of the real atom
   int32_t * pair_center{nullptr};   // [n_pairs] centre row of each pair
@@ -166,7 +172,7 @@ struct NlOutputs {
 };
 struct NlWork {
   DevBuf geom, counts64, scan_tmp, ghost_off, site_x, site_type, site_real, site_shift,
-      site_box, box_base, box_count, box_ptr, box_fill, sorted, sorted_x, sorted_info,
+      site_box, box_base, box_count, box_ptr, binned, sorted, sorted_x,
       pair_count;
   int64_t last_sites{0}, last_boxes{0};
   DevBuf center_atom, center_struct, pair_off, pair_j, pair_shift, pair_dist, pair_dir, pair_center;
@@ -337,13 +343,13 @@ void launch_ps_grad_fp64(const PsArgs & a, const ExpansionArgs & e, int64_t c0, 
 // as dC[i][lm][s*n + n'] (lm = l^2 + m; the (species, radial) index is the
 // fastest so that the centre's 32 consecutive rows store coalesced).
 // x is read back as row_scale * (hi + lo) of the forward's BF16 split.
-// chunk_map: scratch of Dg/4 words (the launch fills it with the slot of
-// every 4-column chunk of a row in the kernel's per-l triangle order and its
-// species pair); present: the centres' species masks (the FP32 expansion's),
+// chunk_map: Dg/4 words (launch_chunk_map: the slot of every 4-column chunk of
+// a row in the kernel's per-l triangle order and its species pair); present: the centres' species masks (the FP32 expansion's),
 // whose absent pairs are taken as zero whatever dX holds there.
 void launch_ps_bwd_fp32(const PsArgs & a, const float * C, const __nv_bfloat16 * Xh,
-                        const __nv_bfloat16 * Xl, const float * row_scale, const float * dX, uint32_t * chunk_map,
-                        const uint32_t * present, float * dC, cudaStream_t st);
+                        const __nv_bfloat16 * Xl, const float * row_scale, const float * dX,
+                        const uint32_t * chunk_map, const uint32_t * present, float * dC, cudaStream_t st);
+void launch_chunk_map(const FeatureDims & fd, uint32_t * chunk_map, cudaStream_t st);
 
 // ------------------------------------------------------------------ GAP
 struct GapSpecies {
@@ -453,11 +459,17 @@ double measure_fma_peak(int precision);
 // hi/lo BF16 split of a row-major FP32 matrix (columns >= cols become 0).
 void split_bf16(const float * x, int64_t rows, int64_t cols, int64_t ldx, __nv_bfloat16 * hi,
                 __nv_bfloat16 * lo, int64_t ldo, cudaStream_t st);
-// energies[structure of centre(center_of_row[row0 + r])] += e(r), where e(r)
-// is e_row_fp64[r] or the sum of the n_parts FP32 partials e_part[t*ld + r].
-void launch_energy_reduce(int64_t rows, int n_parts, const float * e_part, int64_t ld,
-                          const double * e_row_fp64, int64_t row0, const int32_t * center_of_row,
-                          const int32_t * center_struct, double * energies, cudaStream_t st);
+// energies[structure of centre(center_of_row[r])] += e(r) for every row r of
+// the sorted features, where e(r) is e_row_fp64[r], or the sum of its species'
+// FP32 partials: species s has parts[s] planes of rows[s] values from ofs[s].
+struct EnergyParts {
+  int S{0};
+  int64_t row0[17]{}, ofs[16]{};
+  int parts[16]{};
+};
+void launch_energy_reduce(int64_t rows, const EnergyParts & parts, const float * e_part, const double * e_row_fp64,
+                          const int32_t * center_of_row, const int32_t * center_struct, double * energies,
+                          cudaStream_t st);
 
 // FP64 adjoint. dE/dc of every centre from the dE/dx rows t (reference order,
 // stride Dpad; ps.present: the FP64 expansion's species masks) into dC
@@ -524,26 +536,24 @@ void launch_pair_adjoint_fp32(const ExpansionArgs & a, const int32_t * pair_cent
                               double * stress = nullptr);
 
 // ------------------------------------------------------------------ helpers
-// Stable sort of centres by (species, presence mask): rows of one species
-// with the same neighbour species become neighbours, so 128-row GEMM tiles
-// share absent species. Replaces row_of_center / center_of_row.
-void launch_mask_sort(int64_t n, const int32_t * types, const int32_t * center_atom, const int8_t * lut,
-                      const uint32_t * present, int S, int32_t * row_of_center, int32_t * center_of_row, DevBuf & tmp,
-                      cudaStream_t st);
 // Per 128-row tile of each species' rows (species s: rows row0[s] ..
 // row0[s] + rows[s], tiles tile_off[s] .. tile_off[s+1]): the OR of the
 // presence masks of its rows.
 struct TileMaskArgs {
   static constexpr int kSpecies = 16;  // the largest species count of a dense layout
-  int S;
-  int64_t row0[kSpecies], rows[kSpecies], tile_off[kSpecies + 1];
+  int S{0};
+  int64_t row0[kSpecies]{}, rows[kSpecies]{}, tile_off[kSpecies + 1]{};
 };
-void launch_tile_masks(const TileMaskArgs & a, const int32_t * center_of_row, const uint32_t * present, uint32_t * out,
-                       cudaStream_t st);
-void launch_species_sort(int64_t n, const int32_t * types, const int32_t * center_atom,
-                         const int8_t * lut, int S, int64_t * species_count /*[S]*/,
-                         int32_t * row_of_center, int32_t * center_of_row, DevBuf & tmp,
-                         cudaStream_t st);
+// Stable sort of centres by (species, presence mask): rows of one species
+// with the same neighbour species become neighbours, so 128-row GEMM tiles
+// share absent species. Writes row_of_center / center_of_row and the tile
+// masks.
+void launch_mask_sort(int64_t n, const int32_t * types, const int32_t * center_atom, const int8_t * lut,
+                      const uint32_t * present, int S, const TileMaskArgs & tiles, int32_t * row_of_center,
+                      int32_t * center_of_row, uint32_t * tile_mask, DevBuf & tmp, cudaStream_t st);
+// Stable sort of centres by species.
+void launch_species_sort(int64_t n, const int32_t * types, const int32_t * center_atom, const int8_t * lut, int S,
+                         int32_t * row_of_center, int32_t * center_of_row, DevBuf & tmp, cudaStream_t st);
 void launch_round_tf32(float * x, int64_t n, cudaStream_t st);
 void launch_fill_f64(double * p, int64_t n, double v, cudaStream_t st);
 void launch_fill_f32(float * p, int64_t n, float v, cudaStream_t st);

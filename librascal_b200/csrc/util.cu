@@ -136,84 +136,118 @@ SphConst make_sph_constants() {
 
 namespace {
 
-constexpr int kScanBlock = 1024;
+// Exclusive scans. Up to kScanOne values one block scans them in one launch;
+// beyond, tiles of kScanTile values are scanned by themselves and a second
+// launch adds to each the sum of the tiles before it, which every block takes
+// from the tile sums itself. What bounds the small ones is the launch (about
+// 2 us each in a recorded graph; the recursive form took two to five nodes).
+constexpr int kScanBlock = 1024, kScanTile = 4 * kScanBlock, kScanOne = 2 * kScanTile;
 
-template <typename Tin>
-__global__ void scan_block_kernel(const Tin * __restrict__ in, int64_t * __restrict__ out, int64_t n,
-                                  int64_t * __restrict__ block_sums) {
-  __shared__ int64_t warp_tot[32];
-  int64_t i = int64_t(blockIdx.x) * kScanBlock + threadIdx.x;
-  int64_t v = (i < n) ? int64_t(in[i]) : 0;
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int64_t x = v;
+// Exclusive scan over the block of the four values each thread holds;
+// returns what precedes the thread's first value, `total` the block's sum.
+__device__ __forceinline__ int64_t block_scan4(const int64_t v[4], int64_t * warp_tot, int64_t & total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t own = v[0] + v[1] + v[2] + v[3];
+  int64_t x = own;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+    const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
     if (lane >= o) x += y;
   }
   if (lane == 31) warp_tot[wid] = x;
   __syncthreads();
-  if (wid == 0) {
-    int64_t t = warp_tot[lane];
+  int64_t t = warp_tot[lane];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int64_t y = __shfl_up_sync(0xffffffffu, t, o);
-      if (lane >= o) t += y;
-    }
-    warp_tot[lane] = t;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t y = __shfl_up_sync(0xffffffffu, t, o);
+    if (lane >= o) t += y;
   }
-  __syncthreads();
-  int64_t excl = x - v + (wid > 0 ? warp_tot[wid - 1] : 0);
-  if (i < n) out[i] = excl;
-  if (threadIdx.x == kScanBlock - 1) block_sums[blockIdx.x] = excl + v;
+  total = __shfl_sync(0xffffffffu, t, 31);
+  const int64_t before = __shfl_sync(0xffffffffu, t, wid > 0 ? wid - 1 : 0);
+  __syncthreads();  // warp_tot may be written again
+  return x - own + (wid > 0 ? before : 0);
 }
 
-__global__ void scan_add_kernel(int64_t * __restrict__ out, int64_t n,
-                                const int64_t * __restrict__ block_off) {
-  int64_t i = int64_t(blockIdx.x) * kScanBlock + threadIdx.x;
-  if (i < n) out[i] += block_off[blockIdx.x];
-}
-
-__global__ void scan_total_kernel(const int64_t * __restrict__ block_off, int nb,
-                                  int64_t * __restrict__ total) {
-  *total = block_off[nb];
+// ScanCap: the largest value that may be written (a buffer's capacity);
+// larger ones are clamped to it and set status 104.
+__device__ __forceinline__ int64_t scan_clamp(const ScanCap & cap, int64_t v) {
+  if (!cap.status || v <= cap.limit) return v;
+  set_status(cap.status, 104, 0, 0);
+  return cap.limit;
 }
 
 template <typename Tin>
-void scan_impl(const Tin * in, int64_t * out, int64_t n, DevBuf & tmp, size_t tmp_off,
-               cudaStream_t st) {
-  int nb = div_up(n, kScanBlock);
-  if (nb == 0) {
+__global__ void __launch_bounds__(kScanBlock)
+scan_one_kernel(const Tin * __restrict__ in, int64_t * __restrict__ out, int64_t n, ScanCap cap) {
+  __shared__ int64_t warp_tot[32];
+  int64_t carry = 0;
+  for (int64_t base = 0; base < n; base += kScanTile) {
+    const int64_t i = base + 4 * int64_t(threadIdx.x);
+    int64_t v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = i + k < n ? int64_t(in[i + k]) : 0;
+    int64_t total;
+    int64_t x = carry + block_scan4(v, warp_tot, total);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i + k < n) out[i + k] = scan_clamp(cap, x);
+      x += v[k];
+    }
+    carry += total;
+  }
+  if (threadIdx.x == 0) out[n] = scan_clamp(cap, carry);
+}
+
+template <typename Tin>
+__global__ void __launch_bounds__(kScanBlock)
+scan_tile_kernel(const Tin * __restrict__ in, int64_t * __restrict__ out, int64_t n, int64_t * __restrict__ sums) {
+  __shared__ int64_t warp_tot[32];
+  const int64_t i = int64_t(blockIdx.x) * kScanTile + 4 * int64_t(threadIdx.x);
+  int64_t v[4], total;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] = i + k < n ? int64_t(in[i + k]) : 0;
+  int64_t x = block_scan4(v, warp_tot, total);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (i + k < n) out[i + k] = x;
+    x += v[k];
+  }
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kScanBlock)
+scan_add_kernel(int64_t * __restrict__ out, int64_t n, const int64_t * __restrict__ sums, ScanCap cap) {
+  __shared__ int64_t warp_tot[32];
+  int64_t v[4] = {0, 0, 0, 0}, before;
+  for (unsigned k = threadIdx.x; k < blockIdx.x; k += kScanBlock) v[0] += sums[k];
+  block_scan4(v, warp_tot, before);
+  const int64_t base = int64_t(blockIdx.x) * kScanTile;
+  for (int k = threadIdx.x; k < kScanTile && base + k < n; k += kScanBlock)
+    out[base + k] = scan_clamp(cap, out[base + k] + before);
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = scan_clamp(cap, before + sums[blockIdx.x]);
+}
+
+template <typename Tin>
+void scan_impl(const Tin * in, int64_t * out, int64_t n, DevBuf & tmp, size_t tmp_off, cudaStream_t st,
+               ScanCap cap = {}) {
+  if (n <= 0) {
     cuda_check(cudaMemsetAsync(out, 0, sizeof(int64_t), st), "memset");
     return;
   }
-  int64_t * sums = reinterpret_cast<int64_t *>(static_cast<char *>(tmp.p) + tmp_off);
-  int64_t * sums_scan = sums + (nb + 1);
-  size_t used = tmp_off + sizeof(int64_t) * 2 * (nb + 1);
-  scan_block_kernel<Tin><<<nb, kScanBlock, 0, st>>>(in, out, n, sums);
-  RGPU_LAUNCHED();
-  if (nb == 1) {
-    // total = block sum
-    cuda_check(cudaMemcpyAsync(out + n, sums, sizeof(int64_t), cudaMemcpyDeviceToDevice, st), "copy");
+  if (n <= kScanOne) {
+    scan_one_kernel<Tin><<<1, kScanBlock, 0, st>>>(in, out, n, cap);
+    RGPU_LAUNCHED();
     return;
   }
-  scan_impl<int64_t>(sums, sums_scan, nb, tmp, used, st);
-  scan_add_kernel<<<nb, kScanBlock, 0, st>>>(out, n, sums_scan);
+  const int nb = div_up(n, kScanTile);
+  int64_t * sums = reinterpret_cast<int64_t *>(static_cast<char *>(tmp.p) + tmp_off);
+  scan_tile_kernel<Tin><<<nb, kScanBlock, 0, st>>>(in, out, n, sums);
   RGPU_LAUNCHED();
-  scan_total_kernel<<<1, 1, 0, st>>>(sums_scan, nb, out + n);
+  scan_add_kernel<<<nb, kScanBlock, 0, st>>>(out, n, sums, cap);
   RGPU_LAUNCHED();
 }
 
-size_t scan_tmp_bytes(int64_t n) {
-  size_t total = 0;
-  while (true) {
-    int64_t nb = (n + kScanBlock - 1) / kScanBlock;
-    total += sizeof(int64_t) * 2 * (nb + 1);
-    if (nb <= 1) break;
-    n = nb;
-  }
-  return total + 64;
-}
+size_t scan_tmp_bytes(int64_t n) { return sizeof(int64_t) * size_t((n + kScanTile - 1) / kScanTile + 1) + 64; }
 
 // ---- stable counting sort of centres by species
 constexpr int kSortBlock = 1024;
@@ -254,15 +288,6 @@ __global__ void species_rank_kernel(int64_t n, const int32_t * __restrict__ type
     row_of_center[i] = int32_t(r);
     center_of_row[r] = int32_t(i);
   }
-}
-
-__global__ void species_total_kernel(const int64_t * __restrict__ counts, int S, int nb,
-                                     int64_t * __restrict__ out) {
-  int s = threadIdx.x;
-  if (s >= S) return;
-  int64_t t = 0;
-  for (int b = 0; b < nb; ++b) t += counts[int64_t(s) * nb + b];
-  out[s] = t;
 }
 
 // ---- stable sort of centres by (species, species-presence mask): LSD
@@ -339,6 +364,87 @@ __global__ void tile_mask_kernel(TileMaskArgs a, const int32_t * __restrict__ ce
   if (lane == 0) out[t] = m;
 }
 
+// The stable sorts and the tile masks of up to kSmallSort centres in one
+// launch of one block: key = species << S | mask (the species alone without
+// `present`), 5-bit LSD passes with the order in shared memory, then the
+// permutation and, with `tiles`, the OR of the masks of each 128-row tile.
+// The multi-launch form takes ten to fourteen launches of one or a few blocks
+// each, about 2 us apiece; one block does 2 000 rows in about 10 us.
+constexpr int kSmallSort = 4096;
+__global__ void __launch_bounds__(kSortBlock)
+small_sort_kernel(int n, const int32_t * __restrict__ types, const int32_t * __restrict__ center_atom,
+                  const int8_t * __restrict__ lut, const uint32_t * __restrict__ present, int S, TileMaskArgs a,
+                  int32_t * __restrict__ row_of_center, int32_t * __restrict__ center_of_row,
+                  uint32_t * __restrict__ tiles) {
+  __shared__ uint32_t key[kSmallSort];
+  __shared__ uint16_t order[2][kSmallSort];
+  __shared__ int wcnt[32][33];  // [warp][digit]
+  __shared__ int start[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int shift0 = present ? S : 0;
+  for (int i = threadIdx.x; i < n; i += kSortBlock) {
+    const uint32_t m = present ? (S >= 32 ? present[i] : present[i] & ((1u << S) - 1u)) : 0u;
+    key[i] = (uint32_t(lut[types[center_atom[i]]]) << shift0) | m;
+    order[0][i] = uint16_t(i);
+  }
+  int cur = 0;
+  for (int shift = 0; shift < shift0 + 5; shift += 5, cur ^= 1) {
+    if (threadIdx.x < 32) start[threadIdx.x] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kSortBlock) atomicAdd(&start[(key[i] >> shift) & 31u], 1);
+    __syncthreads();
+    if (wid == 0) {  // exclusive scan of the digit counts
+      const int c = start[lane];
+      int x = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      start[lane] = x - c;
+    }
+    for (int base = 0; base < n; base += kSortBlock) {  // in order: the sort is stable
+      wcnt[wid][lane] = 0;
+      __syncthreads();
+      const int k = base + int(threadIdx.x);
+      const int c = k < n ? order[cur][k] : 0;
+      const int d = k < n ? int((key[c] >> shift) & 31u) : 32;
+      const unsigned same = __match_any_sync(0xffffffffu, d);
+      const int rank = __popc(same & lanemask_lt());
+      if (d < 32 && rank == 0) wcnt[wid][d] = __popc(same);
+      __syncthreads();
+      if (wid == 0) {  // where each warp's run of a digit starts
+        int at = start[lane];
+        for (int w = 0; w < 32; ++w) {
+          const int t = wcnt[w][lane];
+          wcnt[w][lane] = at;
+          at += t;
+        }
+        start[lane] = at;
+      }
+      __syncthreads();
+      if (k < n) order[cur ^ 1][wcnt[wid][d] + rank] = uint16_t(c);
+      __syncthreads();
+    }
+  }
+  for (int k = threadIdx.x; k < n; k += kSortBlock) {
+    const int c = order[cur][k];
+    row_of_center[c] = k;
+    center_of_row[k] = c;
+  }
+  if (!tiles) return;
+  const uint32_t mask = S >= 32 ? 0xffffffffu : (1u << S) - 1u;
+  for (int t = wid; t < int(a.tile_off[a.S]); t += 32) {
+    int s = 0;
+    while (t >= a.tile_off[s + 1]) ++s;
+    const int64_t r0 = a.row0[s] + (t - a.tile_off[s]) * 128, r1 = min(r0 + 128, a.row0[s] + a.rows[s]);
+    uint32_t m = 0;
+    for (int64_t r = r0 + lane; r < r1; r += 32) m |= key[order[cur][r]] & mask;
+    m = __reduce_or_sync(0xffffffffu, m);
+    if (lane == 0) tiles[t] = m;
+  }
+}
+
 __global__ void round_tf32_kernel(float * x, int64_t n) {
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n) x[i] = to_tf32(x[i]);
@@ -354,9 +460,9 @@ __global__ void fill_f32_kernel(float * p, int64_t n, float v) {
 
 }  // namespace
 
-void scan_exclusive_i64(const int64_t * in, int64_t * out, int64_t n, DevBuf & tmp, cudaStream_t st) {
+void scan_exclusive_i64(const int64_t * in, int64_t * out, int64_t n, DevBuf & tmp, cudaStream_t st, ScanCap cap) {
   tmp.ensure(scan_tmp_bytes(n));
-  scan_impl<int64_t>(in, out, n, tmp, 0, st);
+  scan_impl<int64_t>(in, out, n, tmp, 0, st, cap);
 }
 void scan_exclusive_i32to64(const int32_t * in, int64_t * out, int64_t n, DevBuf & tmp,
                             cudaStream_t st) {
@@ -365,9 +471,15 @@ void scan_exclusive_i32to64(const int32_t * in, int64_t * out, int64_t n, DevBuf
 }
 
 void launch_mask_sort(int64_t n, const int32_t * types, const int32_t * center_atom, const int8_t * lut,
-                      const uint32_t * present, int S, int32_t * row_of_center, int32_t * center_of_row, DevBuf & tmp,
-                      cudaStream_t st) {
+                      const uint32_t * present, int S, const TileMaskArgs & tiles, int32_t * row_of_center,
+                      int32_t * center_of_row, uint32_t * tile_mask, DevBuf & tmp, cudaStream_t st) {
   if (n <= 0) return;
+  if (n <= kSmallSort) {
+    small_sort_kernel<<<1, kSortBlock, 0, st>>>(int(n), types, center_atom, lut, present, S, tiles, row_of_center,
+                                                center_of_row, tile_mask);
+    RGPU_LAUNCHED();
+    return;
+  }
   const int nb = div_up(n, kSortBlock);
   const size_t cnt = size_t(32) * nb + 1;
   const size_t stmp = scan_tmp_bytes(int64_t(32) * nb);
@@ -392,32 +504,29 @@ void launch_mask_sort(int64_t n, const int32_t * types, const int32_t * center_a
   }
   rows_from_order_kernel<<<div_up(n, 256), 256, 0, st>>>(n, ord[cur], row_of_center, center_of_row);
   RGPU_LAUNCHED();
+  if (tiles.tile_off[tiles.S] > 0) {
+    tile_mask_kernel<<<div_up(tiles.tile_off[tiles.S] * 32, 256), 256, 0, st>>>(tiles, center_of_row, present,
+                                                                               tile_mask);
+    RGPU_LAUNCHED();
+  }
 }
 
-void launch_tile_masks(const TileMaskArgs & a, const int32_t * center_of_row, const uint32_t * present, uint32_t * out,
-                       cudaStream_t st) {
-  const int64_t tiles = a.tile_off[a.S];
-  if (tiles <= 0) return;
-  tile_mask_kernel<<<div_up(tiles * 32, 256), 256, 0, st>>>(a, center_of_row, present, out);
-  RGPU_LAUNCHED();
-}
-
-void launch_species_sort(int64_t n, const int32_t * types, const int32_t * center_atom,
-                         const int8_t * lut, int S, int64_t * species_count, int32_t * row_of_center,
-                         int32_t * center_of_row, DevBuf & tmp, cudaStream_t st) {
-  int nb = div_up(n, kSortBlock);
-  if (nb == 0) {
-    cuda_check(cudaMemsetAsync(species_count, 0, sizeof(int64_t) * S, st), "memset");
+void launch_species_sort(int64_t n, const int32_t * types, const int32_t * center_atom, const int8_t * lut, int S,
+                         int32_t * row_of_center, int32_t * center_of_row, DevBuf & tmp, cudaStream_t st) {
+  if (n <= 0) return;
+  if (n <= kSmallSort) {
+    small_sort_kernel<<<1, kSortBlock, 0, st>>>(int(n), types, center_atom, lut, nullptr, S, TileMaskArgs{},
+                                                row_of_center, center_of_row, nullptr);
+    RGPU_LAUNCHED();
     return;
   }
+  const int nb = div_up(n, kSortBlock);
   size_t cbytes = sizeof(int64_t) * (size_t(S) * nb + 1);
   size_t stmp = scan_tmp_bytes(int64_t(S) * nb);
   tmp.ensure(2 * cbytes + stmp + 256);
   int64_t * counts = tmp.as<int64_t>();
   int64_t * offs = counts + (size_t(S) * nb + 1);
   species_count_kernel<<<nb, kSortBlock, 0, st>>>(n, types, center_atom, lut, S, counts, nb);
-  RGPU_LAUNCHED();
-  species_total_kernel<<<1, 32, 0, st>>>(counts, S, nb, species_count);
   RGPU_LAUNCHED();
   // scan of counts in key-major order gives each (key, block) its first row
   scan_impl<int64_t>(counts, offs, int64_t(S) * nb, tmp, 2 * cbytes, st);
