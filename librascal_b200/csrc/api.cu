@@ -156,6 +156,22 @@ struct rgpu_calculator {
   SplineDev dev{};
 };
 
+// A part of a device buffer.
+struct DevView {
+  void * p{nullptr};
+  template <class T>
+  T * as() const {
+    return static_cast<T *>(p);
+  }
+};
+
+// Status words of a handle's kernels, copied to the host together.
+struct HandleStatus {
+  DevStatus nl;  // neighbour list
+  int tc[2];     // bounded waits of the tcgen05 kernels: gave up, stage
+  int pad[2];
+};
+
 struct GapLayout;
 
 // One FP32 prediction (rgpu_gap_predict / rgpu_gap_predict_stress) recorded
@@ -190,7 +206,8 @@ struct rgpu_structures {
   std::vector<uint8_t> mask;
   bool has_mask{false};
   std::vector<int64_t> center_off_h;
-  DevBuf atom_off_d, pos_d, types_d, cells_d, pbc_d, tag2idx_d, ncent_d, center_off_d, atom_struct_d;
+  DevBuf in_d;  // every input array, one after the other
+  DevView atom_off_d, pos_d, types_d, cells_d, pbc_d, tag2idx_d, ncent_d, center_off_d, atom_struct_d;
   // staging (pinned) for host inputs
   void * pinned{nullptr};
   size_t pinned_cap{0};
@@ -215,7 +232,8 @@ struct rgpu_structures {
   bool feat_gradients{false};
   bool feat_valid{false};
   // GAP work
-  DevBuf E_d, F_d, S_d, K64, t64, erow64, Wh, Wl, dX32, dC32, epart, Xh, Xl, chunk_map;
+  DevBuf out_d;  // energies, forces, stress sums, one after the other
+  DevBuf K64, t64, erow64, Wh, Wl, dX32, dC32, epart, Xh, Xl, chunk_map;
   int chunk_map_of[3]{0, 0, 0};  // the (S, n, L) that chunk_map holds
   bool feat_x32{false};  // FP32 features also kept unsplit (for export)
   DevBuf dCp, dCs, dXp;
@@ -246,8 +264,11 @@ struct rgpu_structures {
   const rgpu_gap_model * fwd_model{nullptr};
   DevBuf y0_d;  // per-structure energy baseline of fwd_model
   // status and timing
-  DevStatus * status_d{nullptr};
-  DevStatus * status_h{nullptr};
+  HandleStatus * status_d{nullptr};
+  HandleStatus * status_h{nullptr};
+  double * E() const { return out_d.as<double>(); }
+  double * F() const { return E() + n_struct; }
+  double * S() const { return F() + 3 * n_atoms; }
   cudaEvent_t ev[10]{};
   double stage_ms[10]{};
   bool timed{false};
@@ -318,9 +339,10 @@ void ensure_stream(rgpu_structures * s) {
   if (!s->st) {
     s->device = current_device();
     RGPU_CUDA(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking));
-    RGPU_CUDA(cudaMalloc(&s->status_d, sizeof(DevStatus)));
-    RGPU_CUDA(cudaMemset(s->status_d, 0, sizeof(DevStatus)));
-    RGPU_CUDA(cudaMallocHost(&s->status_h, sizeof(DevStatus)));
+    RGPU_CUDA(cudaMalloc(&s->status_d, sizeof(HandleStatus)));
+    RGPU_CUDA(cudaMemset(s->status_d, 0, sizeof(HandleStatus)));
+    RGPU_CUDA(cudaMallocHost(&s->status_h, sizeof(HandleStatus)));
+    *s->status_h = HandleStatus{};
     for (auto & e : s->ev) RGPU_CUDA(cudaEventCreate(&e));
   }
 }
@@ -348,27 +370,70 @@ void upload(rgpu_structures * s, DevBuf & dst, const void * src, size_t bytes) {
   RGPU_CUDA(cudaMemcpyAsync(dst.p, p, bytes, cudaMemcpyHostToDevice, s->st));
 }
 
-// Several host -> device copies through one pass of the staging buffer: a
-// single wait for the previous use of the buffer, then one copy per array.
+// The input arrays of a structure set through the staging buffer in one copy
+// into one device buffer, each view on a 256-byte boundary.
 struct Upload {
-  DevBuf * dst;
+  DevView * dst;
   const void * src;
   size_t bytes;
 };
-void upload_many(rgpu_structures * s, const std::vector<Upload> & ups) {
+void upload_inputs(rgpu_structures * s, const std::vector<Upload> & ups) {
   size_t total = 0;
   for (const Upload & u : ups) total += (u.bytes + 255) & ~size_t(255);
-  for (const Upload & u : ups) u.dst->ensure(u.bytes);
-  if (total == 0) return;
+  s->in_d.ensure(std::max<size_t>(total, 256));
   RGPU_CUDA(cudaStreamSynchronize(s->st));  // staging buffer reuse
-  unsigned char * base = static_cast<unsigned char *>(staging(s, total));
+  unsigned char * base = static_cast<unsigned char *>(staging(s, std::max<size_t>(total, 256)));
   size_t off = 0;
   for (const Upload & u : ups) {
-    if (u.bytes == 0) continue;
-    std::memcpy(base + off, u.src, u.bytes);
-    RGPU_CUDA(cudaMemcpyAsync(u.dst->p, base + off, u.bytes, cudaMemcpyHostToDevice, s->st));
+    u.dst->p = s->in_d.as<unsigned char>() + off;
+    if (u.bytes) std::memcpy(base + off, u.src, u.bytes);
     off += (u.bytes + 255) & ~size_t(255);
   }
+  if (total) RGPU_CUDA(cudaMemcpyAsync(s->in_d.p, base, total, cudaMemcpyHostToDevice, s->st));
+}
+
+// New positions into their place.
+void upload_positions(rgpu_structures * s, const double * positions) {
+  const size_t bytes = sizeof(double) * 3 * size_t(s->n_atoms);
+  if (bytes == 0) return;
+  RGPU_CUDA(cudaStreamSynchronize(s->st));  // staging buffer reuse
+  void * p = staging(s, bytes);
+  std::memcpy(p, positions, bytes);
+  RGPU_CUDA(cudaMemcpyAsync(s->pos_d.p, p, bytes, cudaMemcpyHostToDevice, s->st));
+}
+
+// The outputs' buffer, and zeros in the energies and what else is asked for.
+void zero_outputs(rgpu_structures * s, bool forces, bool stress) {
+  s->out_d.ensure(sizeof(double) * (7 * size_t(s->n_struct) + 3 * size_t(s->n_atoms) + 1));
+  const size_t n = stress ? size_t(s->S() - s->E()) + 6 * size_t(s->n_struct)
+                          : size_t(s->n_struct) + (forces ? 3 * size_t(s->n_atoms) : 0);
+  if (n) RGPU_CUDA(cudaMemsetAsync(s->E(), 0, sizeof(double) * n, s->st));
+}
+
+// The handle's status words to the host, in order on the stream, and what a
+// call that has waited for them makes of a tcgen05 wait that gave up.
+void fetch_status(rgpu_structures * s) {
+  RGPU_CUDA(cudaMemcpyAsync(s->status_h, s->status_d, sizeof(HandleStatus), cudaMemcpyDeviceToHost, s->st));
+}
+bool timed_out(rgpu_structures * s, int * where = nullptr) {
+  if (!s->status_h->tc[0]) return false;
+  if (where) *where = s->status_h->tc[1];
+  RGPU_CUDA(cudaMemsetAsync(s->status_d->tc, 0, sizeof(s->status_d->tc), s->st));
+  RGPU_CUDA(cudaStreamSynchronize(s->st));
+  s->status_h->tc[0] = s->status_h->tc[1] = 0;
+  return true;
+}
+void check_timeout(rgpu_structures * s) {
+  int where = 0;
+  if (timed_out(s, &where))
+    throw Error(RGPU_ERR_TIMEOUT, "tensor-core GEMM: a bounded pipeline wait gave up (stage " +
+                                      std::to_string(where) + ")");
+}
+// Clears the status words after a replay whose results were dropped.
+void reset_status(rgpu_structures * s) {
+  RGPU_CUDA(cudaMemsetAsync(s->status_d, 0, sizeof(HandleStatus), s->st));
+  RGPU_CUDA(cudaStreamSynchronize(s->st));
+  *s->status_h = HandleStatus{};
 }
 
 void mark(rgpu_structures * s, int i) {
@@ -436,7 +501,7 @@ void build_nl(rgpu_structures * s, double cutoff) {
   in.center_off = s->center_off_d.as<int64_t>();
   in.atom_struct = s->atom_struct_d.as<int32_t>();
   in.n_centers_total = s->center_off_h[s->n_struct];
-  build_neighbour_list(in, cutoff, s->nlw, s->nl, s->status_d, s->status_h, s->st);
+  build_neighbour_list(in, cutoff, s->nlw, s->nl, &s->status_d->nl, &s->status_h->nl, s->st);
   s->pair_off_h_valid = false;
   s->nl_valid = true;
   s->nl_cutoff = cutoff;
@@ -566,6 +631,7 @@ void compute_features(rgpu_calculator * c, rgpu_structures * s, int precision, b
       s->Xl.ensure(sizeof(uint16_t) * size_t(nc) * fd.Dg + 64);
       s->xscale32.ensure(sizeof(float) * (nc + 1));
       pa.present = s->present.as<uint32_t>();
+      pa.tc_status = s->status_d->tc;
       launch_ps_fwd_fast(pa, s->C32.as<float>(), need_x32 ? s->X32.as<float>() : nullptr,
                          s->Xh.as<__nv_bfloat16>(), s->Xl.as<__nv_bfloat16>(), s->xscale32.as<float>(), s->st);
     }
@@ -948,6 +1014,7 @@ void gap_fast_forward(rgpu_gap_model * m, rgpu_structures * s, double * E_d, boo
       a.zeta = m->zeta;
       a.e_part = s->epart.as<float>() + eofs[sI];
       a.row_scale = s->xscale32.as<float>() + row0;  // k = (p . t) / |p|
+      a.status = s->status_d->tc;
       set_segments(a, s, tm, sI, 1);  // K blocks of species pairs absent from a tile are skipped
       fwd.push_back(a);
     }
@@ -1015,6 +1082,7 @@ void gap_fast_backward(rgpu_gap_model * m, rgpu_structures * s, double * F_d, do
       a.ldc = fd.Dg;
       // N tiles of species pairs absent from a tile are not computed; the
       // power-spectrum backward reads zeros for them (chunk map)
+      a.status = s->status_d->tc;
       set_segments(a, s, tile_mask_args(s), sI, 2);
       bwd.push_back(a);
     } else if (rows > 0) {
@@ -1111,42 +1179,29 @@ static void gap_predict_impl(rgpu_gap_model * m, rgpu_structures * s, int precis
     compute_features(m->calc, s, precision, want_forces, m->species, /*need_x32=*/false);
     model_layout(m, s, precision == RGPU_PRECISION_FP32);
     const int64_t na = s->n_atoms;
-    s->E_d.ensure(sizeof(double) * (s->n_struct + 1));
-    s->F_d.ensure(sizeof(double) * 3 * (na + 1));
-    RGPU_CUDA(cudaMemsetAsync(s->E_d.p, 0, sizeof(double) * s->n_struct, s->st));
-    if (want_forces) RGPU_CUDA(cudaMemsetAsync(s->F_d.p, 0, sizeof(double) * 3 * na, s->st));
-    double * stress_d = nullptr;
-    if (neg_stress) {
-      s->S_d.ensure(sizeof(double) * 6 * (s->n_struct + 1));
-      RGPU_CUDA(cudaMemsetAsync(s->S_d.p, 0, sizeof(double) * 6 * s->n_struct, s->st));
-      stress_d = s->S_d.as<double>();
-    }
+    zero_outputs(s, want_forces, neg_stress != nullptr);
+    double * stress_d = neg_stress ? s->S() : nullptr;
     if (precision == RGPU_PRECISION_FP64)
-      gap_plain(m, s, s->E_d.as<double>(), s->F_d.as<double>(), want_forces, stress_d);
+      gap_plain(m, s, s->E(), s->F(), want_forces, stress_d);
     else
-      gap_fast(m, s, s->E_d.as<double>(), s->F_d.as<double>(), want_forces, stress_d);
+      gap_fast(m, s, s->E(), s->F(), want_forces, stress_d);
     mark(s, 8);
-    // outputs through the pinned staging buffer: a device-to-host copy into
-    // the caller's pageable memory is staged by the driver at a fraction of
-    // the bandwidth
-    const size_t eb = energies ? sizeof(double) * s->n_struct : 0, fb = forces ? sizeof(double) * 3 * na : 0,
-                 sb = neg_stress ? sizeof(double) * 6 * s->n_struct : 0;
-    const size_t need = eb + fb + sb + 64;
+    // outputs in one copy through the pinned staging buffer: a device-to-host
+    // copy into the caller's pageable memory is staged by the driver at a
+    // fraction of the bandwidth
+    const size_t ns = size_t(s->n_struct), lo = energies ? 0 : (forces ? ns : ns + 3 * size_t(na)),
+                 hi = neg_stress ? 7 * ns + 3 * size_t(na) : (forces ? ns + 3 * size_t(na) : (energies ? ns : lo));
+    const size_t need = sizeof(double) * (hi - lo) + 64;
     if (need > s->pinned_cap) RGPU_CUDA(cudaStreamSynchronize(s->st));  // no copy may use the old buffer
-    unsigned char * pin = static_cast<unsigned char *>(staging(s, need));
-    if (eb) RGPU_CUDA(cudaMemcpyAsync(pin, s->E_d.p, eb, cudaMemcpyDeviceToHost, s->st));
-    if (fb) RGPU_CUDA(cudaMemcpyAsync(pin + eb, s->F_d.p, fb, cudaMemcpyDeviceToHost, s->st));
-    if (sb) RGPU_CUDA(cudaMemcpyAsync(pin + eb + fb, s->S_d.p, sb, cudaMemcpyDeviceToHost, s->st));
+    double * pin = static_cast<double *>(staging(s, need)) - lo;
+    if (hi > lo)
+      RGPU_CUDA(cudaMemcpyAsync(pin + lo, s->E() + lo, sizeof(double) * (hi - lo), cudaMemcpyDeviceToHost, s->st));
+    if (precision == RGPU_PRECISION_FP32) fetch_status(s);
     RGPU_CUDA(cudaStreamSynchronize(s->st));
-    if (eb) std::memcpy(energies, pin, eb);
-    if (fb) std::memcpy(forces, pin + eb, fb);
-    if (sb) std::memcpy(neg_stress, pin + eb + fb, sb);
-    if (precision == RGPU_PRECISION_FP32) {
-      const int where = gemm_tc_timeout(true);
-      if (where)
-        throw Error(RGPU_ERR_TIMEOUT, "tensor-core GEMM: a bounded pipeline wait gave up (stage " +
-                                          std::to_string(where) + ")");
-    }
+    if (energies) std::memcpy(energies, pin, sizeof(double) * ns);
+    if (forces) std::memcpy(forces, pin + ns, sizeof(double) * 3 * size_t(na));
+    if (neg_stress) std::memcpy(neg_stress, pin + ns + 3 * size_t(na), sizeof(double) * 6 * ns);
+    if (precision == RGPU_PRECISION_FP32) check_timeout(s);
     if (energies) {
       const std::vector<double> y0 = structure_baselines(m, s);
       for (int st = 0; st < s->n_struct; ++st) energies[st] += y0[st];
@@ -1172,6 +1227,9 @@ static void gap_forward_dev_impl(rgpu_gap_model * m, rgpu_structures * s, const 
                 RGPU_EXC_LOGIC_ERROR);
   calculator_to_device(m->calc);
   s->timed = false;
+  // the baselines go up before the stream has work: the upload waits for it
+  const std::vector<double> y0 = structure_baselines(m, s);
+  upload(s, s->y0_d, y0.data(), sizeof(double) * y0.size());
   if (positions_dev) {
     RGPU_CUDA(cudaMemcpyAsync(s->pos_d.p, positions_dev, sizeof(double) * 3 * s->n_atoms,
                               cudaMemcpyDeviceToDevice, s->st));
@@ -1181,17 +1239,12 @@ static void gap_forward_dev_impl(rgpu_gap_model * m, rgpu_structures * s, const 
   build_nl(s, m->calc->hy.cutoff);
   compute_features(m->calc, s, RGPU_PRECISION_FP32, true, m->species, /*need_x32=*/false);
   model_layout(m, s, true);
-  s->E_d.ensure(sizeof(double) * (s->n_struct + 1));
-  RGPU_CUDA(cudaMemsetAsync(s->E_d.p, 0, sizeof(double) * s->n_struct, s->st));
-  gap_fast_forward(m, s, s->E_d.as<double>());
-  const std::vector<double> y0 = structure_baselines(m, s);
-  upload(s, s->y0_d, y0.data(), sizeof(double) * y0.size());
-  launch_add_f64(s->E_d.as<double>(), s->y0_d.as<double>(), energies_dev, s->n_struct, s->st);
+  zero_outputs(s, false, false);
+  gap_fast_forward(m, s, s->E());
+  launch_add_f64(s->E(), s->y0_d.as<double>(), energies_dev, s->n_struct, s->st);
+  fetch_status(s);
   RGPU_CUDA(cudaStreamSynchronize(s->st));
-  const int where = gemm_tc_timeout(true);
-  if (where)
-    throw Error(RGPU_ERR_TIMEOUT, "tensor-core GEMM: a bounded pipeline wait gave up (stage " +
-                                      std::to_string(where) + ")");
+  check_timeout(s);
   s->fwd_model = m;
 }
 
@@ -1206,16 +1259,13 @@ static void gap_backward_dev_impl(rgpu_gap_model * m, rgpu_structures * s, const
                                        "no other call on the structures in between");
   s->timed = false;
   const int64_t na = s->n_atoms;
-  s->F_d.ensure(sizeof(double) * 3 * (na + 1));
-  RGPU_CUDA(cudaMemsetAsync(s->F_d.p, 0, sizeof(double) * 3 * na, s->st));
-  gap_fast_backward(m, s, s->F_d.as<double>(), nullptr, energies_grad_dev);
+  zero_outputs(s, true, false);
+  gap_fast_backward(m, s, s->F(), nullptr, energies_grad_dev);
   // the adjoint accumulates forces, -dE/dr
-  launch_scale_f64(s->F_d.as<double>(), -1.0, grad_dev, 3 * na, s->st);
+  launch_scale_f64(s->F(), -1.0, grad_dev, 3 * na, s->st);
+  fetch_status(s);
   RGPU_CUDA(cudaStreamSynchronize(s->st));
-  const int where = gemm_tc_timeout(true);
-  if (where)
-    throw Error(RGPU_ERR_TIMEOUT, "tensor-core GEMM: a bounded pipeline wait gave up (stage " +
-                                      std::to_string(where) + ")");
+  check_timeout(s);
 }
 
 // ---------------------------------------------------------------- training
@@ -1407,11 +1457,13 @@ static void sparse_kernel_mm_impl(rgpu_gap_model * m, double * out) {
 // calculator. The recording is replayed only while none of them moved.
 static std::vector<const void *> md_buffers(const rgpu_gap_model * m, const rgpu_structures * s) {
   std::vector<const void *> v;
-  for (const DevBuf * b : {&s->atom_off_d, &s->pos_d, &s->types_d, &s->cells_d, &s->pbc_d, &s->tag2idx_d,
-                           &s->ncent_d, &s->center_off_d, &s->atom_struct_d, &s->lut, &s->row_of_center,
+  for (const DevView * b : {&s->atom_off_d, &s->pos_d, &s->types_d, &s->cells_d, &s->pbc_d, &s->ncent_d,
+                            &s->center_off_d, &s->atom_struct_d})
+    v.push_back(b->p);
+  for (const DevBuf * b : {&s->lut, &s->row_of_center,
                            &s->center_of_row, &s->sort_tmp, &s->present, &s->tile_mask,
                            &s->C64, &s->X64,
-                           &s->invn64, &s->dC64, &s->C32, &s->X32, &s->xscale32, &s->E_d, &s->F_d, &s->S_d, &s->K64,
+                           &s->invn64, &s->dC64, &s->C32, &s->X32, &s->xscale32, &s->out_d, &s->K64,
                            &s->t64, &s->erow64, &s->Wh, &s->Wl, &s->dX32, &s->dC32, &s->epart, &s->Xh, &s->Xl,
                            &s->chunk_map, &s->dCp, &s->dCs, &s->dXp, &s->knm, &s->plist, &s->Tq})
     v.push_back(b->p);
@@ -1461,7 +1513,7 @@ static void graph_enqueue(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   in.center_off = s->center_off_d.as<int64_t>();
   in.atom_struct = s->atom_struct_d.as<int32_t>();
   in.n_centers_total = s->center_off_h[s->n_struct];
-  build_neighbour_list(in, c->hy.cutoff, s->nlw, s->nl, s->status_d, s->status_h, st, &caps);
+  build_neighbour_list(in, c->hy.cutoff, s->nlw, s->nl, &s->status_d->nl, &s->status_h->nl, st, &caps);
   // features (the FP32 branch of compute_features, layout unchanged)
   const bool by_mask = sorts_by_mask(c, s);
   sort_rows(s, by_mask);
@@ -1476,21 +1528,16 @@ static void graph_enqueue(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   launch_expansion_fp32(ea, s->C32.as<float>(), s->present.as<uint32_t>(), st);
   if (by_mask) sort_rows_by_mask(s);
   pa.present = s->present.as<uint32_t>();
+  pa.tc_status = s->status_d->tc;
   launch_ps_fwd_fast(pa, s->C32.as<float>(), nullptr, s->Xh.as<__nv_bfloat16>(), s->Xl.as<__nv_bfloat16>(),
                      s->xscale32.as<float>(), st);
-  RGPU_CUDA(cudaMemsetAsync(s->E_d.p, 0, sizeof(double) * s->n_struct, st));
-  if (forces) RGPU_CUDA(cudaMemsetAsync(s->F_d.p, 0, sizeof(double) * 3 * na, st));
-  if (stress) RGPU_CUDA(cudaMemsetAsync(s->S_d.p, 0, sizeof(double) * 6 * s->n_struct, st));
-  gap_fast(m, s, s->E_d.as<double>(), s->F_d.as<double>(), forces, stress ? s->S_d.as<double>() : nullptr);
-  if (double * out = out_h) {
-    RGPU_CUDA(cudaMemcpyAsync(out, s->E_d.p, sizeof(double) * s->n_struct, cudaMemcpyDeviceToHost, st));
-    if (forces)
-      RGPU_CUDA(cudaMemcpyAsync(out + s->n_struct, s->F_d.p, sizeof(double) * 3 * na, cudaMemcpyDeviceToHost, st));
-    if (stress)
-      RGPU_CUDA(cudaMemcpyAsync(out + s->n_struct + 3 * na, s->S_d.p, sizeof(double) * 6 * s->n_struct,
-                                cudaMemcpyDeviceToHost, st));
+  zero_outputs(s, forces, stress);
+  gap_fast(m, s, s->E(), s->F(), forces, stress ? s->S() : nullptr);
+  if (out_h) {
+    const size_t n = size_t(s->n_struct) * (stress ? 7 : 1) + (forces ? 3 * size_t(na) : 0);
+    if (n) RGPU_CUDA(cudaMemcpyAsync(out_h, s->E(), sizeof(double) * n, cudaMemcpyDeviceToHost, st));
   }
-  RGPU_CUDA(cudaMemcpyAsync(s->status_h, s->status_d, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
+  fetch_status(s);
 }
 
 // The step's work on the structures' stream, positions from s->md_pos_h.
@@ -1558,24 +1605,19 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
     RGPU_CUDA(cudaGraphLaunch(s->md_exec, s->st));
     RGPU_CUDA(cudaStreamSynchronize(s->st));
     ++s->md_replays;
-    const int where = gemm_tc_timeout(true);
-    if (where)
-      throw Error(RGPU_ERR_TIMEOUT, "tensor-core GEMM: a bounded pipeline wait gave up (stage " +
-                                        std::to_string(where) + ")");
-    if (s->status_h->code == 0) {
+    check_timeout(s);
+    if (s->status_h->nl.code == 0) {
       md_finish(m, s, energies, forces, neg_stress);
       return;
     }
     // outgrown capacities or an input error: the ordinary path below
     // rebuilds, or reports the error with its message
-    s->md_reason = 100 + s->status_h->code;
-    RGPU_CUDA(cudaMemsetAsync(s->status_d, 0, sizeof(DevStatus), s->st));
-    RGPU_CUDA(cudaStreamSynchronize(s->st));
-    s->status_h->code = 0;
+    s->md_reason = 100 + s->status_h->nl.code;
+    reset_status(s);
   }
   md_drop(s);
   // the ordinary path: checks the input, sizes every buffer, gives this step's results
-  upload(s, s->pos_d, positions, sizeof(double) * 3 * na);
+  upload_positions(s, positions);
   s->nl_valid = false;
   s->feat_valid = false;
   gap_predict_impl(m, s, RGPU_PRECISION_FP32, energies, forces, neg_stress);
@@ -1597,19 +1639,16 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
     RGPU_CUDA(cudaMallocHost(&s->md_out_h, sizeof(double) * std::max<size_t>(nout, 1)));
     s->md_out_cap = nout;
   }
-  if (stress) s->S_d.ensure(sizeof(double) * 6 * (s->n_struct + 1));
   std::memcpy(s->md_pos_h, positions, sizeof(double) * 3 * na);
   // one run without recording sizes the capacity buffers (no allocation may
   // happen while recording) and checks that the step fits them
   s->timed = false;
   md_enqueue(m, s, stress);
   RGPU_CUDA(cudaStreamSynchronize(s->st));
-  if (s->status_h->code != 0 || gemm_tc_timeout(true)) {
+  if (s->status_h->nl.code != 0 || timed_out(s)) {
     // cannot happen with fresh capacities unless something is off: leave
     // the step to the ordinary path next time
-    RGPU_CUDA(cudaMemsetAsync(s->status_d, 0, sizeof(DevStatus), s->st));
-    RGPU_CUDA(cudaStreamSynchronize(s->st));
-    s->status_h->code = 0;
+    reset_status(s);
     return;
   }
   // record; a step that cannot be recorded keeps the ordinary path
@@ -1711,14 +1750,9 @@ static bool pgraph_replay(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
     s->nl_valid = false;
     s->feat_valid = false;
     s->fwd_model = nullptr;
-    const int where = gemm_tc_timeout(true);
-    if (where)
-      throw Error(RGPU_ERR_TIMEOUT, "tensor-core GEMM: a bounded pipeline wait gave up (stage " +
-                                        std::to_string(where) + ")");
-    if (s->status_h->code != 0) {
-      RGPU_CUDA(cudaMemsetAsync(s->status_d, 0, sizeof(DevStatus), s->st));
-      RGPU_CUDA(cudaStreamSynchronize(s->st));
-      s->status_h->code = 0;
+    check_timeout(s);
+    if (s->status_h->nl.code != 0) {
+      reset_status(s);
       pgraph_release(g);
       s->pgraphs.erase(s->pgraphs.begin() + (&g - s->pgraphs.data()));
       return false;
@@ -1757,13 +1791,12 @@ static void pgraph_record(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
     const size_t nout = size_t(s->n_struct) * 7 + 3 * size_t(s->n_atoms) + 1;
     RGPU_CUDA(cudaMallocHost(&g.out_h, sizeof(double) * nout));
   }
-  if (stress) s->S_d.ensure(sizeof(double) * 6 * (s->n_struct + 1));
   s->timed = false;
   bool ok = true;
   try {
     graph_enqueue(m, s, stress, nullptr, g.out_h, g.caps, forces);
     RGPU_CUDA(cudaStreamSynchronize(s->st));
-    ok = s->status_h->code == 0 && gemm_tc_timeout(true) == 0;
+    ok = s->status_h->nl.code == 0 && !timed_out(s);
   } catch (...) {
     ok = false;
   }
@@ -1787,9 +1820,7 @@ static void pgraph_record(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   s->fwd_model = nullptr;
   if (!ok) {
     (void)cudaGetLastError();
-    RGPU_CUDA(cudaMemsetAsync(s->status_d, 0, sizeof(DevStatus), s->st));
-    RGPU_CUDA(cudaStreamSynchronize(s->st));
-    s->status_h->code = 0;
+    reset_status(s);
     pgraph_release(g);
     return;
   }
@@ -2009,7 +2040,7 @@ rgpu_status rgpu_structures_set(rgpu_structures * s, int32_t n_structures, const
         {&s->center_off_d, s->center_off_h.data(), sizeof(int64_t) * (n_structures + 1)},
         {&s->atom_struct_d, astruct.data(), sizeof(int32_t) * s->n_atoms}};
     if (s->has_mask) ups.push_back({&s->tag2idx_d, tag2idx.data(), sizeof(int32_t) * s->n_atoms});
-    upload_many(s, ups);
+    upload_inputs(s, ups);
     s->nl_valid = false;
     s->feat_valid = false;
     s->fwd_model = nullptr;
@@ -2019,7 +2050,7 @@ rgpu_status rgpu_structures_set(rgpu_structures * s, int32_t n_structures, const
 rgpu_status rgpu_structures_update_positions(rgpu_structures * s, const double * positions) {
   return guard([&] {
     OnDevice on_dev(s);
-    upload(s, s->pos_d, positions, sizeof(double) * 3 * s->n_atoms);
+    upload_positions(s, positions);
     s->nl_valid = false;
     s->feat_valid = false;
     s->fwd_model = nullptr;

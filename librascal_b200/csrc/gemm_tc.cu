@@ -793,7 +793,7 @@ void grouped_launch(const Bf16x3Gemm * gs, int n, cudaStream_t st) {
   if (ng == 0) return;
   p.n_groups = ng;
   p.n_tiles = tiles;
-  p.status = tc_status();
+  p.status = gs[0].status ? reinterpret_cast<TcStatus *>(gs[0].status) : tc_status();
   p.mma_wait_limit = g_mma_wait_limit.load();
   int dev = 0, sms = 0;
   cuda_check(cudaGetDevice(&dev), "cudaGetDevice");

@@ -332,7 +332,7 @@ void launch_ps_fwd_tc(const PsArgs & a, const float * C, __nv_bfloat16 * Xh, __n
   RGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int64_t tiles = (a.n_centers + plan.T - 1) / plan.T;
   const int grid = int(std::min<int64_t>(tiles, int64_t(sms) * 2));
-  TcStatus * status = tc_status_word();
+  TcStatus * status = a.tc_status ? reinterpret_cast<TcStatus *>(a.tc_status) : tc_status_word();
 #define RGPU_PSTC_CASE(LL)                                                                                      \
   case LL:                                                                                                      \
     RGPU_CUDA(cudaFuncSetAttribute(ps_fwd_tc_kernel<LL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))); \

@@ -314,6 +314,8 @@ struct PsArgs {
   // FP32 forward: the centres' species masks (the FP32 expansion's); tiles of
   // pairs a centre lacks are written as zeros. Null: every pair computed.
   const uint32_t * present = nullptr;
+  // timeout word pair of the tcgen05 forward (null: the device's own)
+  int * tc_status = nullptr;
 };
 // X rows (normalised) and inverse norms.
 void launch_ps_fwd_fp64(const PsArgs & a, const double * C, double * X, double * inv_norm,
@@ -431,6 +433,9 @@ struct Bf16x3Gemm {
   const uint32_t * tile_mask = nullptr;
   int seg_mode = 0;
   int seg_G = 0, seg_LD = 0, seg_LO = 0;
+  // grouped launches: where a bounded wait that gives up reports (timeout
+  // flag, stage); null: the device's own word pair
+  int * status = nullptr;
 };
 constexpr int kTcTileN = 256;
 void gemm_bf16x3(const Bf16x3Gemm & g, cudaStream_t st);
