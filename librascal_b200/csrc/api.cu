@@ -237,6 +237,7 @@ struct rgpu_structures {
   int chunk_map_of[3]{0, 0, 0};  // the (S, n, L) that chunk_map holds
   bool feat_x32{false};  // FP32 features also kept unsplit (for export)
   DevBuf dCp, dCs, dXp;
+  DevBuf export_d;               // rows of rgpu_get_features on their way out
   DevBuf knm, plist, Tq;  // sparse kernel matrices for training
   // MD step recorded as a CUDA graph (rgpu_md_step)
   cudaGraph_t md_graph{nullptr};
@@ -2157,50 +2158,35 @@ rgpu_status rgpu_get_features(const rgpu_calculator * calc, const rgpu_structure
     const FeatureDims & fd = s->fd;
     const int64_t nc = s->nl.n_centers;
     const bool ps = calc->hy.kind == "sphericalinvariants";
-    const int inner = ps ? fd.n * fd.n * (fd.L + 1) : fd.nK;
-    const int row_len = ps ? fd.Dpad : fd.S * fd.nK;
-    std::vector<int32_t> row_of(nc);
-    RGPU_CUDA(cudaMemcpyAsync(row_of.data(), s->row_of_center.p, sizeof(int32_t) * nc, cudaMemcpyDeviceToHost, s->st));
-    std::vector<double> dense(size_t(nc) * row_len);
-    if (s->feat_precision == RGPU_PRECISION_FP64) {
-      const void * src = ps ? s->X64.p : s->C64.p;
-      RGPU_CUDA(cudaMemcpyAsync(dense.data(), src, sizeof(double) * dense.size(), cudaMemcpyDeviceToHost, s->st));
-      RGPU_CUDA(cudaStreamSynchronize(s->st));
-    } else {
-      // FP32 expansion rows are padded ([S*n][row_stride(L)])
-      const size_t rs = size_t(row_stride(fd.L));
-      std::vector<float> tmp(ps ? size_t(nc) * fd.Dg : size_t(nc) * fd.S * fd.n * rs);
-      const void * src = ps ? s->X32.p : s->C32.p;
-      RGPU_CUDA(cudaMemcpyAsync(tmp.data(), src, sizeof(float) * tmp.size(), cudaMemcpyDeviceToHost, s->st));
-      RGPU_CUDA(cudaStreamSynchronize(s->st));
-      if (ps) {
-        // FP32 rows hold the unnormalised p in the packed layout: scale by
-        // 1/|p| and unfold into the reference's column order
-        std::vector<float> scale(nc);
-        RGPU_CUDA(cudaMemcpyAsync(scale.data(), s->xscale32.p, sizeof(float) * nc, cudaMemcpyDeviceToHost, s->st));
-        RGPU_CUDA(cudaStreamSynchronize(s->st));
-        for (int64_t r = 0; r < nc; ++r)
-          unpack_to_reference(fd, &tmp[size_t(r) * fd.Dg], scale[r], &dense[size_t(r) * row_len]);
-      } else {
-        for (int64_t r = 0; r < nc; ++r)
-          for (int row = 0; row < fd.S * fd.n; ++row)
-            for (int l = 0; l <= fd.L; ++l)
-              for (int m = 0; m < 2 * l + 1; ++m)
-                dense[size_t(r) * row_len + size_t(row) * fd.K + l * l + m] =
-                    tmp[(size_t(r) * fd.S * fd.n + row) * rs + offp(l) + m];
-      }
+    const int64_t row = int64_t(n_keys) * (ps ? fd.n * fd.n * (fd.L + 1) : fd.nK);
+    if (nc == 0 || row == 0) return;
+    if (ps && s->feat_precision != RGPU_PRECISION_FP64 && !s->feat_x32)
+      throw Error(RGPU_ERR_NOT_COMPUTED, "the last FP32 prediction kept no features to export");
+    // selected and rearranged on the device, then straight into the caller's
+    // array, a bounded number of rows at a time
+    const std::vector<int> blocks = key_blocks(calc, s, n_keys, keys);
+    DevBuf & buf = const_cast<rgpu_structures *>(s)->export_d;
+    const int64_t rows = std::min<int64_t>(nc, std::max<int64_t>(1, (int64_t(256) << 20) / int64_t(sizeof(double)) / row));
+    const size_t head = (sizeof(int32_t) * size_t(n_keys) + 255) & ~size_t(255);
+    buf.ensure(head + sizeof(double) * size_t(rows) * row);
+    RGPU_CUDA(cudaMemcpyAsync(buf.p, blocks.data(), sizeof(int32_t) * n_keys, cudaMemcpyHostToDevice, s->st));
+    FeatureExport a;
+    a.fd = fd;
+    a.power_spectrum = ps;
+    a.fp64 = s->feat_precision == RGPU_PRECISION_FP64;
+    a.src = a.fp64 ? (ps ? s->X64.p : s->C64.p) : (ps ? s->X32.p : s->C32.p);
+    a.row_of_center = s->row_of_center.as<int32_t>();
+    a.row_scale = s->xscale32.as<float>();
+    a.blocks = buf.as<int32_t>();
+    a.n_keys = n_keys;
+    a.out = reinterpret_cast<double *>(buf.as<unsigned char>() + head);
+    for (a.c0 = 0; a.c0 < nc; a.c0 = a.c1) {
+      a.c1 = std::min(nc, a.c0 + rows);
+      launch_feature_export(a, s->st);
+      RGPU_CUDA(cudaMemcpyAsync(out + a.c0 * row, a.out, sizeof(double) * size_t(a.c1 - a.c0) * row,
+                                cudaMemcpyDeviceToHost, s->st));
     }
-    auto blocks = key_blocks(calc, s, n_keys, keys);
-    for (int64_t ci = 0; ci < nc; ++ci) {
-      const double * src = &dense[size_t(ps ? row_of[ci] : ci) * row_len];
-      double * dst = out + size_t(ci) * n_keys * inner;
-      for (int k = 0; k < n_keys; ++k) {
-        if (blocks[k] < 0)
-          std::memset(dst + size_t(k) * inner, 0, sizeof(double) * inner);
-        else
-          std::memcpy(dst + size_t(k) * inner, src + size_t(blocks[k]) * inner, sizeof(double) * inner);
-      }
-    }
+    RGPU_CUDA(cudaStreamSynchronize(s->st));
   });
 }
 

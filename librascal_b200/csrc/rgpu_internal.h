@@ -290,7 +290,7 @@ __host__ __device__ inline void tile_column(const FeatureDims & fd, int i, int j
   base = segment_offset(fd, A, B) + 4 * t;
   lstep = 4 * (A < B ? fd.TO : fd.TD);
 }
-inline int packed_column(const FeatureDims & fd, int l, int I, int J) {
+__host__ __device__ inline int packed_column(const FeatureDims & fd, int l, int I, int J) {
   int base, lstep;
   tile_column(fd, I >> 1, J >> 1, base, lstep);
   return base + (fd.L - l) * lstep + (I & 1) + 2 * (J & 1);
@@ -300,6 +300,21 @@ inline int reference_column(const FeatureDims & fd, int a, int n1, int b, int n2
   const int key = a * fd.S - a * (a - 1) / 2 + (b - a);
   return ((key * fd.n + n1) * fd.n + n2) * (fd.L + 1) + l;
 }
+// Dense FP64 export rows [c0, c1) of the centres: out[c - c0][k][e], the block
+// blocks[k] (-1: zeros) of each requested key, from whichever of the four
+// feature stores `src` is (power spectrum or expansion, FP64 or FP32).
+struct FeatureExport {
+  FeatureDims fd;
+  bool power_spectrum, fp64;
+  const void * src;
+  const int32_t * row_of_center;
+  const float * row_scale;  // FP32 power spectrum
+  const int32_t * blocks;
+  int n_keys;
+  int64_t c0, c1;
+  double * out;
+};
+void launch_feature_export(const FeatureExport & a, cudaStream_t st);
 // A row in the reference's dense order (D values) to the packed layout (Dg
 // values, zeros in the padding).
 void pack_reference_row(const FeatureDims & fd, const double * ref, double * packed);

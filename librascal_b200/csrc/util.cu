@@ -589,6 +589,57 @@ void launch_scale_rows_by_group(float * x, int64_t rows, int64_t cols, const int
 // ------------------------------------------------------------ packed layout
 namespace {
 constexpr double kSqrt2 = 1.41421356237309504880;
+
+// One thread per exported value, consecutive threads along a row. Bound by the
+// copy to the host that follows; doing the key selection (and, for FP32, the
+// unfolding below) here leaves the host nothing to rearrange.
+__global__ void feature_export_kernel(FeatureExport a, int inner, int64_t n) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const FeatureDims & fd = a.fd;
+  const int64_t ck = i / inner;
+  const int e = int(i - ck * inner), k = int(ck % a.n_keys);
+  const int64_t c = a.c0 + ck / a.n_keys;
+  const int b = a.blocks[k];
+  double v = 0.;
+  if (b >= 0 && a.fp64) {
+    const double * src = static_cast<const double *>(a.src);
+    v = a.power_spectrum ? src[int64_t(a.row_of_center[c]) * fd.Dpad + int64_t(b) * inner + e]
+                         : src[(c * fd.S + b) * fd.nK + e];
+  } else if (b >= 0 && a.power_spectrum) {
+    int sa = 0, r = b;  // key b is the species pair (sa, sa + r)
+    while (r >= fd.S - sa) r -= fd.S - sa++;
+    const int sb = sa + r, l = e % (fd.L + 1), q = e / (fd.L + 1);
+    int n1 = q / fd.n, n2 = q - n1 * fd.n;
+    const bool fold = sa == sb && n1 != n2;
+    if (fold && n1 > n2) {
+      const int t = n1;
+      n1 = n2;
+      n2 = t;
+    }
+    const int64_t row = a.row_of_center[c];
+    float x = static_cast<const float *>(a.src)[row * fd.Dg + packed_column(fd, l, sa * fd.n + n1, sb * fd.n + n2)] *
+              a.row_scale[row];
+    if (fold) x *= float(1. / kSqrt2);  // the packed entry is sqrt2 p(n1 n2)
+    v = double(x);
+  } else if (b >= 0) {
+    const int nn = e / fd.K, lm = e - nn * fd.K;
+    int l = 0;
+    while ((l + 1) * (l + 1) <= lm) ++l;
+    v = double(static_cast<const float *>(
+        a.src)[(c * fd.Sn + b * fd.n + nn) * row_stride(fd.L) + offp_rt(l) + (lm - l * l)]);
+  }
+  a.out[i] = v;
+}
+}  // namespace
+
+void launch_feature_export(const FeatureExport & a, cudaStream_t st) {
+  const int inner = a.power_spectrum ? a.fd.n * a.fd.n * (a.fd.L + 1) : a.fd.nK;
+  const int64_t n = (a.c1 - a.c0) * a.n_keys * inner;
+  if (n <= 0) return;
+  feature_export_kernel<<<unsigned((n + 255) / 256), 256, 0, st>>>(a, inner, n);
+  RGPU_LAUNCHED();
+  RGPU_CUDA(cudaGetLastError());
 }
 
 void pack_reference_row(const FeatureDims & fd, const double * ref, double * packed) {
