@@ -52,14 +52,18 @@ constexpr int kMaxN = 16;  // largest max_radial of the register-staged path
 // dE/dc of the pair's centre is read as dC[i][lm][s*n + n'], n contiguous
 // values per lm (float4 loads when n == NV). With STRESS, the pair's
 // r_ji (x) g_ij (Voigt xx yy zz yz xz xy, the reference's
-// sparse_kernel_predict.hh:355-366) is summed per structure as well.
+// sparse_kernel_predict.hh:355-366) is summed per structure as well. With
+// `scale`, each structure's contributions are multiplied by scale[structure]
+// (an upstream gradient; a pass of its own over dE/dc took 114 us for 16 000
+// atoms).
 template <int L, int NV, bool STRESS>
 // 5 resident blocks per SM (96 registers, a few bytes of spills at L = 6)
 // measured faster than 4 (128 registers) or 6 (more spills)
 __global__ void __launch_bounds__(kThreads, 5)
 pair_adjoint_kernel(ExpansionArgs a, const int32_t * __restrict__ pair_center, int64_t n_pairs,
                     const float * __restrict__ dC, double * __restrict__ F,
-                    const int32_t * __restrict__ center_struct, double * __restrict__ stress) {
+                    const int32_t * __restrict__ center_struct, double * __restrict__ stress,
+                    const double * __restrict__ scale) {
   constexpr int K = (L + 1) * (L + 1);
   constexpr int L1 = L + 1;
   const int W = a.fd.W, n = a.fd.n, Sn = a.fd.S * a.fd.n;
@@ -166,9 +170,10 @@ pair_adjoint_kernel(ExpansionArgs a, const int32_t * __restrict__ pair_center, i
             }
           });
       const float fr = fc / float(r);
-      g0 = dx * sY + fr * sd0;
-      g1 = dy * sY + fr * sd1;
-      g2 = dz * sY + fr * sd2;
+      const float up = scale ? float(scale[center_struct[ci]]) : 1.f;
+      g0 = up * (dx * sY + fr * sd0);
+      g1 = up * (dy * sY + fr * sd1);
+      g2 = up * (dz * sY + fr * sd2);
       if constexpr (STRESS) {
         const float rf = float(r), rx = -rf * dx, ry = -rf * dy, rz = -rf * dz;
         t6[0] = rx * g0;
@@ -232,23 +237,23 @@ pair_adjoint_kernel(ExpansionArgs a, const int32_t * __restrict__ pair_center, i
 // each instantiation unrolls the spherical-harmonics recurrence).
 template <int L>
 void adjoint_launch(const ExpansionArgs & a, const int32_t * pair_center, int64_t n_pairs, const float * dC,
-                    double * forces, cudaStream_t st, const int32_t * center_struct, double * stress, int grid,
-                    int threads) {
+                    double * forces, cudaStream_t st, const int32_t * center_struct, double * stress,
+                    const double * scale, int grid, int threads) {
   sph_constants_tu();  // this translation unit's copy of the constants
   if (a.fd.n <= 8) {
     if (stress)
-      pair_adjoint_kernel<L, 8, true><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces, center_struct,
-                                                              stress);
+      pair_adjoint_kernel<L, 8, true><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces,
+                                                               center_struct, stress, scale);
     else
-      pair_adjoint_kernel<L, 8, false><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces, nullptr,
-                                                               nullptr);
+      pair_adjoint_kernel<L, 8, false><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces, center_struct,
+                                                               nullptr, scale);
   } else {
     if (stress)
       pair_adjoint_kernel<L, 16, true><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces,
-                                                               center_struct, stress);
+                                                               center_struct, stress, scale);
     else
-      pair_adjoint_kernel<L, 16, false><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces, nullptr,
-                                                                nullptr);
+      pair_adjoint_kernel<L, 16, false><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces, center_struct,
+                                                                nullptr, scale);
   }
 }
 
@@ -259,13 +264,13 @@ void adjoint_launch(const ExpansionArgs & a, const int32_t * pair_center, int64_
 // dispatch refers to the others through extern declarations.
 template <int L>
 void adjoint_launch_l(const ExpansionArgs & a, const int32_t * pc, int64_t np, const float * dC, double * F,
-                      cudaStream_t st, const int32_t * cs, double * S, int grid, int threads) {
-  adjoint_launch<L>(a, pc, np, dC, F, st, cs, S, grid, threads);
+                      cudaStream_t st, const int32_t * cs, double * S, const double * scale, int grid, int threads) {
+  adjoint_launch<L>(a, pc, np, dC, F, st, cs, S, scale, grid, threads);
 }
 
 #define RGPU_ADJ_SIG(LL)                                                                                  \
   void adjoint_launch_l<LL>(const ExpansionArgs &, const int32_t *, int64_t, const float *, double *,     \
-                            cudaStream_t, const int32_t *, double *, int, int)
+                            cudaStream_t, const int32_t *, double *, const double *, int, int)
 #define RGPU_ADJ_INST(LL)                                             \
   template RGPU_ADJ_SIG(LL);
 #define RGPU_ADJ_EXTERN(LL)                                           \
@@ -342,7 +347,7 @@ RGPU_ADJ_EXTERN(12)
 #ifdef RGPU_ADJ_DISPATCH
 void launch_pair_adjoint_fp32(const ExpansionArgs & a, const int32_t * pair_center, int64_t n_pairs,
                               const float * dC, double * forces, cudaStream_t st,
-                              const int32_t * center_struct, double * stress) {
+                              const int32_t * center_struct, double * stress, const double * scale) {
   if (a.n_centers == 0 || n_pairs == 0) return;
   if (a.fd.n > kMaxN) throw Error(RGPU_ERR_INVALID_ARGUMENT, "max_radial above 16 is not supported on the fast path");
   const TileConfig cfg = tile_config(a.fd.S, a.fd.n, a.fd.L);
@@ -354,7 +359,7 @@ void launch_pair_adjoint_fp32(const ExpansionArgs & a, const int32_t * pair_cent
       int(std::min<int64_t>((n_pairs + threads - 1) / threads, int64_t(sms) * cfg.adj_blocks_per_sm));
 #define RGPU_ADJ_CASE(LL)                                                                        \
   case LL:                                                                                       \
-    adjoint_launch_l<LL>(a, pair_center, n_pairs, dC, forces, st, center_struct, stress, grid, threads); \
+    adjoint_launch_l<LL>(a, pair_center, n_pairs, dC, forces, st, center_struct, stress, scale, grid, threads); \
     break;
   switch (a.fd.L) {
     RGPU_ADJ_CASE(0)

@@ -1102,13 +1102,10 @@ void gap_fast_backward(rgpu_gap_model * m, rgpu_structures * s, double * F_d, do
   ensure_chunk_map(s, fd);
   launch_ps_bwd_fp32(pa, s->C32.as<float>(), Xh, Xl, s->xscale32.as<float>(), s->dX32.as<float>(),
                      s->chunk_map.as<uint32_t>(), s->present.as<uint32_t>(), s->dC32.as<float>(), st);
-  if (struct_scale)
-    launch_scale_rows_by_group(s->dC32.as<float>(), nc, int64_t(fd.S) * fd.nK, s->nl.center_struct, struct_scale,
-                               st);
   mark(s, 7);
   ExpansionArgs ea = exp_args(c, s);
   launch_pair_adjoint_fp32(ea, s->nl.pair_center, s->nl.n_pairs, s->dC32.as<float>(), F_d, st,
-                           s->nl.center_struct, stress_d);
+                           s->nl.center_struct, stress_d, struct_scale);
 }
 
 void gap_fast(rgpu_gap_model * m, rgpu_structures * s, double * E_d, double * F_d, bool forces,

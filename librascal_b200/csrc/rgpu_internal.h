@@ -549,11 +549,12 @@ void launch_knm_gradient(const KnmGradArgs & a, DevBuf & list, DevBuf & scratch,
 
 // Adjoint pair kernel: forces from dE/dC (FP32, the layout written by
 // launch_ps_bwd_fp32) and recomputed dC/dr. With stress, also the unscaled
-// negative stress sum_pairs r_ji (x) g_ij per structure (6 Voigt values).
+// negative stress sum_pairs r_ji (x) g_ij per structure (6 Voigt values). With
+// scale, everything times scale[structure].
 void launch_pair_adjoint_fp32(const ExpansionArgs & a, const int32_t * pair_center, int64_t n_pairs,
                               const float * dC, double * forces,
                               cudaStream_t st, const int32_t * center_struct = nullptr,
-                              double * stress = nullptr);
+                              double * stress = nullptr, const double * scale = nullptr);
 
 // ------------------------------------------------------------------ helpers
 // Per 128-row tile of each species' rows (species s: rows row0[s] ..
@@ -580,8 +581,4 @@ void launch_fill_f32(float * p, int64_t n, float v, cudaStream_t st);
 // out = a + b; out = a x (n doubles, device)
 void launch_add_f64(const double * a, const double * b, double * out, int64_t n, cudaStream_t st);
 void launch_scale_f64(const double * x, double a, double * out, int64_t n, cudaStream_t st);
-// x[r][c] *= scale[group[r]] for a row-major rows x cols FP32 matrix
-void launch_scale_rows_by_group(float * x, int64_t rows, int64_t cols, const int32_t * group,
-                                const double * scale, cudaStream_t st);
-
 }  // namespace rgpu

@@ -561,12 +561,6 @@ __global__ void scale_f64_kernel(const double * __restrict__ x, double a, double
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n) out[i] = a * x[i];
 }
-__global__ void scale_rows_by_group_kernel(float * __restrict__ x, int64_t rows, int64_t cols,
-                                           const int32_t * __restrict__ group, const double * __restrict__ scale) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= rows * cols) return;
-  x[i] *= float(scale[group[i / cols]]);
-}
 }  // namespace
 
 void launch_add_f64(const double * a, const double * b, double * out, int64_t n, cudaStream_t st) {
@@ -577,12 +571,6 @@ void launch_add_f64(const double * a, const double * b, double * out, int64_t n,
 void launch_scale_f64(const double * x, double a, double * out, int64_t n, cudaStream_t st) {
   if (n <= 0) return;
   scale_f64_kernel<<<div_up(n, 256), 256, 0, st>>>(x, a, out, n);
-  RGPU_LAUNCHED();
-}
-void launch_scale_rows_by_group(float * x, int64_t rows, int64_t cols, const int32_t * group,
-                                const double * scale, cudaStream_t st) {
-  if (rows * cols <= 0) return;
-  scale_rows_by_group_kernel<<<div_up(rows * cols, 256), 256, 0, st>>>(x, rows, cols, group, scale);
   RGPU_LAUNCHED();
 }
 
