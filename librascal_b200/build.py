@@ -25,8 +25,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 SOURCES = [
     ("nl.cu", ["--fmad=false"], "nl"),
     ("util.cu", [], "util"),
-    ("expansion.cu", ["--fmad=false", "-DRGPU_PART_FP64"], "expansion_f64"),
-    ("expansion.cu", ["-DRGPU_PART_FP32"], "expansion_f32"),
+    ("expansion.cu", ["--fmad=false"], "expansion_f64"),
+    ("expansion_f32.cu", [], "expansion_f32"),
     ("powerspectrum.cu", ["--fmad=false", "-DRGPU_PART_FP64"], "powerspectrum_f64"),
     ("ps_fast.cu", [], "ps_fast"),
     ("ps_tc.cu", [], "ps_tc"),

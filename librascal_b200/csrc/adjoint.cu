@@ -65,7 +65,6 @@ pair_adjoint_kernel(ExpansionArgs a, const int32_t * __restrict__ pair_center, i
                     const int32_t * __restrict__ center_struct, double * __restrict__ stress,
                     const double * __restrict__ scale) {
   constexpr int K = (L + 1) * (L + 1);
-  constexpr int L1 = L + 1;
   const int W = a.fd.W, n = a.fd.n, Sn = a.fd.S * a.fd.n;
   const bool vec = (n & 3) == 0;  // dE/dc rows of n floats as 16-byte loads
   const int lane = threadIdx.x & 31;
@@ -158,7 +157,7 @@ pair_adjoint_kernel(ExpansionArgs a, const int32_t * __restrict__ pair_center, i
 #pragma unroll
             for (int nn = 0; nn < NV; ++nn) {
               if (nn < n) {
-                const float4 t = __ldg(q4 + nn * L1 + l);
+                const float4 t = __ldg(q4 + l * n + nn);
                 const float ri = aa * (t.x + ca * t.y) + bb * (t.z + cb * t.w);
                 const float dri = (t.z - t.x - ea * t.y + eb * t.w) * ih;
                 rl[nn] = ri;

@@ -152,7 +152,7 @@ struct rgpu_calculator {
   int device{-1};  // device of the uploaded tables (-1: not uploaded yet)
   Hypers hy;
   RadialSpline spline;
-  DevBuf grid, y, y2h, yf, y2hf, q4f, center;
+  DevBuf grid, y, y2h, q4f, center;
   SplineDev dev{};
 };
 
@@ -216,6 +216,7 @@ struct rgpu_structures {
   double nl_cutoff{-1};
   NlWork nlw;
   NlOutputs nl;
+  int64_t exact_pairs{0};  // pairs of the last list built with synchronisation (nl.n_pairs may be a capacity)
   std::vector<int64_t> pair_off_h;  // host copy of nl.pair_off, made on demand
   bool pair_off_h_valid{false};
   std::vector<int> batch_species;   // sorted atom types present in the batch
@@ -503,6 +504,7 @@ void build_nl(rgpu_structures * s, double cutoff) {
   in.atom_struct = s->atom_struct_d.as<int32_t>();
   in.n_centers_total = s->center_off_h[s->n_struct];
   build_neighbour_list(in, cutoff, s->nlw, s->nl, &s->status_d->nl, &s->status_h->nl, s->st);
+  s->exact_pairs = s->nl.n_pairs;
   s->pair_off_h_valid = false;
   s->nl_valid = true;
   s->nl_cutoff = cutoff;
@@ -535,6 +537,7 @@ ExpansionArgs exp_args(const rgpu_calculator * c, const rgpu_structures * s) {
   a.rs.exponent = c->hy.rs_exponent;
   a.rs.scale = c->hy.rs_scale;
   a.n_centers = s->nl.n_centers;
+  a.n_pairs = s->exact_pairs;
   a.center_atom = s->nl.center_atom;
   a.pair_off = s->nl.pair_off;
   a.pair_j = s->nl.pair_j;
@@ -1475,7 +1478,7 @@ static std::vector<const void *> md_buffers(const rgpu_gap_model * m, const rgpu
   for (const DevBuf * b : {&m->T64, &m->alpha64, &m->Th, &m->Tl, &m->Tth, &m->Ttl, &m->alpha32, &m->ucol})
     v.push_back(b->p);
   const rgpu_calculator * c = m->calc;
-  for (const DevBuf * b : {&c->grid, &c->y, &c->y2h, &c->yf, &c->y2hf, &c->q4f, &c->center}) v.push_back(b->p);
+  for (const DevBuf * b : {&c->grid, &c->y, &c->y2h, &c->q4f, &c->center}) v.push_back(b->p);
   return v;
 }
 
@@ -1883,12 +1886,14 @@ static void calculator_to_device(rgpu_calculator * c) {
       yf[i] = float(sp.y[i]);
       y2hf[i] = float(sp.y2h[i]);
     }
-    // interval table of the FP32 path: one 16-byte load per channel
-    const size_t W = size_t(sp.width);
+    // interval table of the FP32 path: one 16-byte load per channel, the
+    // channels of one l side by side
+    const size_t W = size_t(sp.width), L1 = size_t(c->hy.max_angular) + 1, n = W / L1;
     std::vector<float> q4(size_t(std::max(sp.grid_size - 1, 1)) * W * 4, 0.f);
     for (int k = 0; k + 1 < sp.grid_size; ++k)
-      for (size_t c = 0; c < W; ++c) {
-        float * o = &q4[(size_t(k) * W + c) * 4];
+      for (size_t ch = 0; ch < W; ++ch) {
+        float * o = &q4[(size_t(k) * W + ch) * 4];
+        const size_t c = ch % n * L1 + ch / n;
         o[0] = yf[size_t(k) * W + c];
         o[1] = y2hf[size_t(k) * W + c];
         o[2] = yf[size_t(k + 1) * W + c];
@@ -1903,15 +1908,11 @@ static void calculator_to_device(rgpu_calculator * c) {
     put(c->grid, sp.grid.data(), sizeof(double) * sp.grid.size());
     put(c->y, sp.y.data(), sizeof(double) * GW);
     put(c->y2h, sp.y2h.data(), sizeof(double) * GW);
-    put(c->yf, yf.data(), sizeof(float) * GW);
-    put(c->y2hf, y2hf.data(), sizeof(float) * GW);
     put(c->q4f, q4.data(), sizeof(float) * q4.size());
     put(c->center, center.data(), sizeof(double) * center.size());
     c->dev.grid = c->grid.as<double>();
     c->dev.y = c->y.as<double>();
     c->dev.y2h = c->y2h.as<double>();
-    c->dev.yf = c->yf.as<float>();
-    c->dev.y2hf = c->y2hf.as<float>();
     c->dev.q4f = c->q4f.as<float4>();
     c->dev.x1 = sp.x1;
     c->dev.h = sp.h;

@@ -21,34 +21,14 @@ namespace {
 
 constexpr int kWarps = 4;
 constexpr int kPad = 33;  // shared row stride of the per-pair tiles
-// The FP32 kernel takes pairs CH at a time (8, 16 or 32; 16 by default, as
-// most centres of the molecular benchmark have fewer than 16 pairs, which
-// keeps the per-warp tiles small and the resident warps many) with one
-// centre per warp and up to kMaxWarpsF warps per block, both chosen per
-// feature shape by the tile configuration.
-constexpr int kMaxWarpsF = 8;
-
-template <typename T>
-struct Tab;
-template <>
-struct Tab<double> {
-  static __device__ __forceinline__ const double * y(const SplineDev & s) { return s.y; }
-  static __device__ __forceinline__ const double * d(const SplineDev & s) { return s.y2h; }
-};
-template <>
-struct Tab<float> {
-  static __device__ __forceinline__ const float * y(const SplineDev & s) { return s.yf; }
-  static __device__ __forceinline__ const float * d(const SplineDev & s) { return s.y2hf; }
-};
-
 // Evaluate RI (and optionally dRI) of all W channels at r into smem columns.
 template <typename T, bool DER>
 __device__ __forceinline__ void spline_eval(const SplineDev & sp, double r, T * RI, T * dRI,
                                             int stride) {
   SplinePos q = spline_pos(sp, r);
   const T a = T(q.a), b = T(q.b);
-  const T * y0 = Tab<T>::y(sp) + size_t(q.k) * sp.W;
-  const T * d0 = Tab<T>::d(sp) + size_t(q.k) * sp.W;
+  const T * y0 = sp.y + size_t(q.k) * sp.W;
+  const T * d0 = sp.y2h + size_t(q.k) * sp.W;
   const T * y1 = y0 + sp.W;
   const T * d1 = d0 + sp.W;
   const T ca = a * a - T(1), cb = b * b - T(1);
@@ -157,174 +137,6 @@ expansion_kernel(ExpansionArgs a, T * __restrict__ C, uint32_t * __restrict__ pr
   }
 }
 
-
-#ifndef RGPU_PART_FP64
-// FP32 fast path. The same sums, organised for throughput instead of the
-// reference's accumulation order (the FP64 kernel above keeps that order):
-//   (a) lanes = pairs: f_c, the spline interval and Y_lm of one pair each;
-//   (b) lanes = radial channels: f_c RI_c(r_p) for the chunk's pairs one
-//       after the other, one 16-byte load of the interval table per channel;
-//   (c) lanes = (l, four columns m of the padded l-block, four radial
-//       channels): 16 accumulators per lane; per pair of a species one
-//       16-byte load of Y and four loads of f_c RI feed 16 products; the
-//       sums are written once, as 16-byte stores, into the padded row
-//       layout [S*n][row_stride(L)] (Y is zero in the padding columns, so
-//       the padding of every l-block is written as zero).
-template <int L, int CH>
-__global__ void __launch_bounds__(kMaxWarpsF * 32)
-expansion_f32_kernel(ExpansionArgs a, float * __restrict__ C, uint32_t * __restrict__ present) {
-  constexpr int K = (L + 1) * (L + 1);
-  constexpr int L1 = L + 1;
-  constexpr int RS = row_stride(L), OL = offp(L + 1), NG = OL / 4;
-  constexpr int kChunkF = CH, kPadF = CH + 1;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nw = blockDim.x >> 5;  // centres per block
-  const int W = a.fd.W, S = a.fd.S, n = a.fd.n;
-  const int wpad = (W * kPadF + 3) & ~3;  // keeps Yp 16-byte aligned
-  float * RIf = reinterpret_cast<float *>(smem_raw) + size_t(wid) * (wpad + CH * RS);  // [W][kPadF]
-  float * Yp = RIf + wpad;  // [CH][RS]: Y_lm of each pair in the padded column layout
-  __shared__ float pa_s[kMaxWarpsF][32], pb_s[kMaxWarpsF][32], fc_s[kMaxWarpsF][32];
-  __shared__ int pk_s[kMaxWarpsF][32];
-  __shared__ uint8_t order_s[kMaxWarpsF][32];
-  __shared__ int16_t colk[K];  // padded column of lm: offp(l) + m
-  __shared__ uint8_t grp_l[NG];
-  for (int lm = threadIdx.x; lm < K; lm += blockDim.x) {
-    int l = 0;
-    while ((l + 1) * (l + 1) <= lm) ++l;
-    colk[lm] = int16_t(offp_rt(l) + (lm - l * l));
-  }
-  for (int g = threadIdx.x; g < NG; g += blockDim.x) {
-    int l = 0;
-    while (4 * g >= offp_rt(l + 1)) ++l;
-    grp_l[g] = uint8_t(l);
-  }
-  for (int e = lane; e < CH * RS; e += 32) Yp[e] = 0.f;  // padding columns stay zero
-  __syncthreads();
-  const int nblk = (n + 3) >> 2;  // blocks of four radial channels
-  for (int64_t ci = int64_t(blockIdx.x) * nw + wid; ci < a.n_centers; ci += int64_t(gridDim.x) * nw) {
-    float * Ci = C + size_t(ci) * S * n * RS;
-    const int64_t p_lo = a.pair_off[ci] + 1, p_hi = a.pair_off[ci + 1];
-    const int ti = a.species_lut[a.types[a.center_atom[ci]]];
-    uint32_t mask_all = 1u << ti;
-    // the columns after the last l-block
-    for (int j = lane; j < S * n * (RS - OL); j += 32) {
-      const int row = j / (RS - OL), c = OL + (j - row * (RS - OL));
-      Ci[row * RS + c] = 0.f;
-    }
-    bool first = true;
-    for (int64_t p0 = p_lo; p0 < p_hi || first; p0 += kChunkF) {
-      const int np = int(max(int64_t(0), min(int64_t(kChunkF), p_hi - p0)));
-      int my_sp = 31;
-      if (lane < np) {
-        const int64_t p = p0 + lane;
-        const double r = a.pair_dist[p];
-        my_sp = a.species_lut[a.types[a.pair_j[p]]];
-        const SplinePos q = spline_pos(a.sp, r);
-        pk_s[wid][lane] = q.k;
-        pa_s[wid][lane] = float(q.a);
-        pb_s[wid][lane] = float(q.b);
-        fc_s[wid][lane] = float(cutoff_fc(a, r));
-        const float dx = float(a.pair_dir[3 * p]), dy = float(a.pair_dir[3 * p + 1]),
-                    dz = float(a.pair_dir[3 * p + 2]);
-        float * yrow = Yp + lane * RS;
-        spherical_harmonics<L, false, float>(dx, dy, dz, [&](int lm, float y, float, float, float) {
-          yrow[colk[lm]] = y;
-        });
-      }
-      // stable order of the chunk's pairs by species
-      int before = 0;
-      unsigned my_mask = 0;
-      for (int s = 0; s < S; ++s) {
-        unsigned m = __ballot_sync(0xffffffffu, my_sp == s);
-        if (my_sp == s) my_mask = m;
-        if (s < my_sp) before += __popc(m);
-        if (m) mask_all |= 1u << s;
-      }
-      if (lane < np) order_s[wid][before + __popc(my_mask & lanemask_lt())] = uint8_t(lane);
-      __syncwarp();
-      // lanes = radial channels c and c + 32 (then c + 64, ... when W is
-      // larger); four pairs per step, so that their table loads are in
-      // flight together
-      const bool c1_ok = lane + 32 < W, c0_ok = lane < W;
-#pragma unroll 4
-      for (int q = 0; q < np; ++q) {
-        const float fa = pa_s[wid][q], fb = pb_s[wid][q], f = fc_s[wid][q];
-        const float ca = fa * fa - 1.f, cb = fb * fb - 1.f;
-        const float4 * row = a.sp.q4f + size_t(pk_s[wid][q]) * W;
-        if (c0_ok) {
-          const float4 t = __ldg(row + lane);
-          RIf[lane * kPadF + q] = f * (fa * (t.x + ca * t.y) + fb * (t.z + cb * t.w));
-        }
-        if (c1_ok) {
-          const float4 t = __ldg(row + lane + 32);
-          RIf[(lane + 32) * kPadF + q] = f * (fa * (t.x + ca * t.y) + fb * (t.z + cb * t.w));
-        }
-        for (int c = lane + 64; c < W; c += 32) {
-          const float4 t = __ldg(row + c);
-          RIf[c * kPadF + q] = f * (fa * (t.x + ca * t.y) + fb * (t.z + cb * t.w));
-        }
-      }
-      __syncwarp();
-      int start = 0;
-      for (int s = 0; s < S; ++s) {
-        const int cnt = __popc(__ballot_sync(0xffffffffu, my_sp == s));
-        if (cnt > 0 || first) {
-          float * Cs = Ci + size_t(s) * n * RS;
-          for (int t = lane; t < NG * nblk; t += 32) {
-            const int g = t % NG, n0 = 4 * (t / NG);
-            const int l = grp_l[g], col = 4 * g;
-            const float * ri = RIf + (n0 * L1 + l) * kPadF;  // channel (n0 + k) L1 + l at + k L1 kPadF
-            float acc[4][4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-#pragma unroll
-              for (int e = 0; e < 4; ++e) acc[k][e] = 0.f;
-            for (int q = 0; q < cnt; ++q) {
-              const int pl = order_s[wid][start + q];
-              const float4 y = *reinterpret_cast<const float4 *>(Yp + pl * RS + col);
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                if (n0 + k < n) {
-                  const float rv = ri[k * L1 * kPadF + pl];
-                  acc[k][0] += rv * y.x;
-                  acc[k][1] += rv * y.y;
-                  acc[k][2] += rv * y.z;
-                  acc[k][3] += rv * y.w;
-                }
-              }
-            }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const int nn = n0 + k;
-              if (nn < n) {
-                float4 * dst = reinterpret_cast<float4 *>(Cs + nn * RS + col);
-                if (first) {
-                  // centre contribution (calculator_spherical_expansion.hh:2244-2247)
-                  if (s == ti && col == 0) acc[k][0] += float(a.center_contrib[nn]);
-                  *dst = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
-                } else {
-                  float4 o = *dst;
-                  o.x += acc[k][0];
-                  o.y += acc[k][1];
-                  o.z += acc[k][2];
-                  o.w += acc[k][3];
-                  *dst = o;
-                }
-              }
-            }
-          }
-        }
-        start += cnt;
-      }
-      __syncwarp();
-      first = false;
-    }
-    if (lane == 0) present[ci] = mask_all;
-    __syncwarp();
-  }
-}
-#endif
 
 // Plain path: grad_j c^i for every non-self pair of centres [c0, c1); each
 // lane streams its pair's 3 x n x K block.
@@ -451,80 +263,13 @@ void launch_exp(const ExpansionArgs & a, T * C, uint32_t * present, cudaStream_t
   RGPU_CUDA(cudaGetLastError());
 }
 
-#ifndef RGPU_PART_FP64
-void launch_exp_f32(const ExpansionArgs & a, float * C, uint32_t * present, cudaStream_t st) {
-  if (a.n_centers == 0) return;
-  if (a.fd.n > 16) throw Error(RGPU_ERR_INVALID_ARGUMENT, "max_radial above 16 is not supported on the fast path");
-  sph_constants_tu();
-  const TileConfig cfg = tile_config(a.fd.S, a.fd.n, a.fd.L);
-  const int CH = cfg.exp_chunk;
-  int dev = 0, sms = 148, optin = 0;
-  RGPU_CUDA(cudaGetDevice(&dev));
-  RGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  RGPU_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const size_t per_warp =
-      ((size_t(a.fd.W) * (CH + 1) + 3) / 4 * 4 + size_t(CH) * row_stride(a.fd.L)) * sizeof(float);
-  const int warps = int(std::max<size_t>(1, std::min<size_t>(size_t(cfg.exp_warps), (size_t(optin) - 8192) / per_warp)));
-  const size_t smem = size_t(warps) * per_warp;
-  int grid = int(std::min<int64_t>((a.n_centers + warps - 1) / warps, int64_t(sms) * 16 * (4 / std::min(warps, 4))));
-#define RGPU_EXPF_NV(LL, CHH)                                                                       \
-  {                                                                                                 \
-    RGPU_CUDA(cudaFuncSetAttribute(expansion_f32_kernel<LL, CHH>,                                   \
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));        \
-    expansion_f32_kernel<LL, CHH><<<grid, warps * 32, smem, st>>>(a, C, present);                   \
-  }
-#define RGPU_EXP_CASE(LL)              \
-  case LL:                             \
-    if (CH == 8) {                     \
-      RGPU_EXPF_NV(LL, 8)              \
-    } else if (CH == 32) {             \
-      RGPU_EXPF_NV(LL, 32)             \
-    } else {                           \
-      RGPU_EXPF_NV(LL, 16)             \
-    }                                  \
-    break;
-  switch (a.fd.L) {
-    RGPU_EXP_CASE(0)
-    RGPU_EXP_CASE(1)
-    RGPU_EXP_CASE(2)
-    RGPU_EXP_CASE(3)
-    RGPU_EXP_CASE(4)
-    RGPU_EXP_CASE(5)
-    RGPU_EXP_CASE(6)
-    RGPU_EXP_CASE(7)
-    RGPU_EXP_CASE(8)
-    RGPU_EXP_CASE(9)
-    RGPU_EXP_CASE(10)
-    RGPU_EXP_CASE(11)
-    RGPU_EXP_CASE(12)
-    default:
-      throw Error(RGPU_ERR_INVALID_ARGUMENT, "max_angular above 12 is not supported on the GPU");
-  }
-#undef RGPU_EXP_CASE
-#undef RGPU_EXPF_NV
-  RGPU_LAUNCHED();
-  RGPU_CUDA(cudaGetLastError());
-}
-#endif
-
 }  // namespace
 
-// The library compiles this file twice: RGPU_PART_FP64 (with --fmad=false, so
-// the FP64 arithmetic rounds like the CPU restatement) and RGPU_PART_FP32.
-#ifndef RGPU_PART_FP32
 void launch_expansion_fp64(const ExpansionArgs & a, double * C, uint32_t * present,
                            cudaStream_t st) {
   launch_exp<double>(a, C, present, st);
 }
-#endif
-#ifndef RGPU_PART_FP64
-void launch_expansion_fp32(const ExpansionArgs & a, float * C, uint32_t * present,
-                           cudaStream_t st) {
-  launch_exp_f32(a, C, present, st);
-}
-#endif
 
-#ifndef RGPU_PART_FP32
 void launch_expansion_grad_fp64(const ExpansionArgs & a, int64_t c0, int64_t c1, int64_t p_base,
                                 double * dCp, cudaStream_t st) {
   if (c1 <= c0) return;
@@ -569,6 +314,5 @@ void launch_expansion_selfgrad_fp64(const ExpansionArgs & a, int64_t c0, int64_t
   RGPU_LAUNCHED();
   RGPU_CUDA(cudaGetLastError());
 }
-#endif
 
 }  // namespace rgpu

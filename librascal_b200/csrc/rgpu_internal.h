@@ -105,9 +105,7 @@ struct SplineDev {
   const double * grid;
   const double * y;    // [G][W]
   const double * y2h;  // [G][W]
-  const float * yf;
-  const float * y2hf;
-  const float4 * q4f;  // [G-1][W]: (y_k, y2h_k, y_k+1, y2h_k+1) of interval k, FP32
+  const float4 * q4f;  // [G-1][W]: (y_k, y2h_k, y_k+1, y2h_k+1) of interval k, FP32, channels ordered [l][n]
   double x1, h, inv_h, ppu;
   int search_size, W;
 };
@@ -222,6 +220,7 @@ struct ExpansionArgs {
   const int8_t * species_lut;     // [130] -> species index or -1
   double rc, sw;
   int64_t n_centers;
+  int64_t n_pairs;  // of the last list built with synchronisation: picks kernels, bounds nothing
   const int32_t * center_atom;
   const int64_t * pair_off;
   const int32_t * pair_j;
