@@ -284,12 +284,6 @@ struct SegWalk {
     }
     return A >= sg.G || on;
   }
-  // whether any unit of [u0, u0 + n) is needed
-  __device__ __forceinline__ bool any(int u0, int n) {
-    bool r = false;
-    for (int u = u0; u < u0 + n; ++u) r |= need(u);
-    return r;
-  }
 };
 
 struct TcGroupedArgs {
@@ -334,6 +328,53 @@ __device__ __forceinline__ TileSpan tile_span(const TcGroupedArgs & p, const TcG
     u1 = last + 1;
   }
   return {u0, u1 - u0};
+}
+
+// The K blocks of an M-tile, in order: all of them, or under K-mode skipping
+// those that overlap a segment whose two groups the tile holds. f(kb) returns
+// false to stop. Segments are walked, not asked block by block: the producer
+// and the MMA issuer are one thread each, and what they execute per block
+// bounds the pipeline once a block's MMAs take less (forward of 100 clusters,
+// 64 columns: 76 -> 65 us with this walk and ready-made descriptors).
+template <int BK, class F>
+__device__ __forceinline__ bool for_k_blocks(const SegGeom & sg, bool skip, uint32_t mask, int nk, F && f) {
+  if (!skip) {
+    for (int kb = 0; kb < nk; ++kb)
+      if (!f(kb)) return false;
+    return true;
+  }
+  if (mask == 0) mask = 0xFFFFFFFFu;  // a tile always holds its rows' own species
+  int u = 0, next = 0;                // first unit of the segment; first block not visited yet
+  for (int A = 0; A < sg.G; ++A)
+    for (int B = A; B < sg.G; ++B) {
+      const int end = u + (A == B ? sg.LD : sg.LO);
+      if (((mask >> A) & (mask >> B) & 1u) != 0u) {
+        const int last = (end - 1) / (BK / 32);
+        for (int kb = max(next, u / (BK / 32)); kb <= last; ++kb)
+          if (!f(kb)) return false;
+        next = last + 1;
+      }
+      u = end;
+    }
+  return true;
+}
+// Their number.
+template <int BK>
+__device__ __forceinline__ int count_k_blocks(const SegGeom & sg, bool skip, uint32_t mask, int nk) {
+  if (!skip) return nk;
+  if (mask == 0) mask = 0xFFFFFFFFu;
+  int u = 0, next = 0, n = 0;
+  for (int A = 0; A < sg.G; ++A)
+    for (int B = A; B < sg.G; ++B) {
+      const int end = u + (A == B ? sg.LD : sg.LO);
+      if (((mask >> A) & (mask >> B) & 1u) != 0u) {
+        const int last = (end - 1) / (BK / 32);
+        n += last + 1 - max(next, u / (BK / 32));
+        next = last + 1;
+      }
+      u = end;
+    }
+  return n;
 }
 
 __device__ __forceinline__ int find_group(const TcGroupedArgs & p, int64_t t) {
@@ -383,6 +424,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_grouped_kernel(const __gr
   if (warp == 0) {
     if (lane == 0) {
       uint32_t it = 0;  // K blocks issued by this CTA
+      int s = 0;        // its ring stage and the stage's phase
+      uint32_t ph = 0;
       bool ok = true;
       for (int64_t t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
         const int g = find_group(p, t);
@@ -393,27 +436,25 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_grouped_kernel(const __gr
         const int m0 = int(mt * kBM), n0 = 32 * sp.u0;
         const int nk = int((G.K + BK - 1) / BK);
         const bool kskip = p.seg.mode == 1 && G.tile_mask;
-        SegWalk w;
-        if (kskip) w.start(p.seg, G.tile_mask[mt]);
-        for (int kb = 0; kb < nk; ++kb) {
-          if (kskip && !w.any(kb * (BK / 32), BK / 32)) continue;
-          const int s = int(it % STAGES);
-          const uint32_t ph = (it / STAGES) & 1u;
-          if (!mbar_wait(&empty[s], ph ^ 1u, status, 1)) {
-            ok = false;
-            break;
-          }
+        const CUtensorMap *ma_hi = &p.a_hi[g], *ma_lo = &p.a_lo[g], *mb_hi = &p.b_hi[g], *mb_lo = &p.b_lo[g];
+        ok = for_k_blocks<BK>(p.seg, kskip, kskip ? G.tile_mask[mt] : 0u, nk, [&](int kb) {
+          if (!mbar_wait(&empty[s], ph ^ 1u, status, 1)) return false;
           unsigned char * st = base + s * SM::STAGE_BYTES;
           mbar_expect_tx(&full[s], SM::STAGE_BYTES);
           const int kx = kb * BK;
-          tma_load_2d(st, &p.a_hi[g], &full[s], kx, m0);
-          tma_load_2d(st + SM::A_BYTES, &p.a_lo[g], &full[s], kx, m0);
+          tma_load_2d(st, ma_hi, &full[s], kx, m0);
+          tma_load_2d(st + SM::A_BYTES, ma_lo, &full[s], kx, m0);
           // B as one box of BN rows from the span's first column (rows past
           // the span or past N are loaded or zero-filled but not multiplied)
-          tma_load_2d(st + 2 * SM::A_BYTES, &p.b_hi[g], &full[s], kx, n0);
-          tma_load_2d(st + 2 * SM::A_BYTES + SM::B_BYTES, &p.b_lo[g], &full[s], kx, n0);
+          tma_load_2d(st + 2 * SM::A_BYTES, mb_hi, &full[s], kx, n0);
+          tma_load_2d(st + 2 * SM::A_BYTES + SM::B_BYTES, mb_lo, &full[s], kx, n0);
           ++it;
-        }
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1u;
+          }
+          return true;
+        });
       }
       // the last copies must have landed before the CTA releases its shared
       // memory (they normally have; this matters after a timeout)
@@ -422,7 +463,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_grouped_kernel(const __gr
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      uint32_t it = 0;
+      const uint64_t d0 = smem_desc_k<BK>(smem_u32(base));  // A_hi of stage 0
+      int s = 0;  // ring stage and its phase
+      uint32_t ph = 0;
       int i = 0;
       bool ok = true;
       for (int64_t t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
@@ -442,32 +485,30 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_grouped_kernel(const __gr
         tc_fence_after();
         const uint32_t acc = tmem + uint32_t(b * BN);
         const bool kskip = p.seg.mode == 1 && G.tile_mask;
-        SegWalk w;
-        if (kskip) w.start(p.seg, G.tile_mask[mt]);
-        bool first = true;  // the tile's first MMA overwrites the accumulator
-        for (int kb = 0; kb < nk; ++kb) {
-          if (kskip && !w.any(kb * (BK / 32), BK / 32)) continue;
-          const int s = int(it % STAGES);
-          const uint32_t ph = (it / STAGES) & 1u;
+        const int blocks = count_k_blocks<BK>(p.seg, kskip, kskip ? G.tile_mask[mt] : 0u, nk);
+        uint32_t acc0 = 0u;  // the tile's first MMA overwrites the accumulator
+        for (int kb = 0; kb < blocks; ++kb) {
           if (!mbar_wait(&full[s], ph, status, 2, p.mma_wait_limit)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          unsigned char * st = base + s * SM::STAGE_BYTES;
-          const uint32_t a_hi = smem_u32(st), a_lo = smem_u32(st + SM::A_BYTES);
-          const uint32_t b_hi = smem_u32(st + 2 * SM::A_BYTES), b_lo = smem_u32(st + 2 * SM::A_BYTES + SM::B_BYTES);
+          // descriptors differ in their address field alone (16-byte units)
+          const uint32_t so = uint32_t(s) * (SM::STAGE_BYTES >> 4);
+          const uint64_t a_hi = d0 + so, a_lo = a_hi + (SM::A_BYTES >> 4), b_hi = a_hi + (2 * SM::A_BYTES >> 4),
+                         b_lo = b_hi + (SM::B_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
-            const uint32_t off = uint32_t(k) * 32u;
-            const uint32_t acc0 = (first && k == 0) ? 0u : 1u;
-            mma_bf16(acc, smem_desc_k<BK>(a_lo + off), smem_desc_k<BK>(b_hi + off), idesc, acc0);
-            mma_bf16(acc, smem_desc_k<BK>(a_hi + off), smem_desc_k<BK>(b_lo + off), idesc, 1u);
-            mma_bf16(acc, smem_desc_k<BK>(a_hi + off), smem_desc_k<BK>(b_hi + off), idesc, 1u);
+            mma_bf16(acc, a_lo + 2 * k, b_hi + 2 * k, idesc, acc0);
+            mma_bf16(acc, a_hi + 2 * k, b_lo + 2 * k, idesc, 1u);
+            mma_bf16(acc, a_hi + 2 * k, b_hi + 2 * k, idesc, 1u);
+            acc0 = 1u;
           }
           mma_commit(&empty[s]);
-          ++it;
-          first = false;
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
         mma_commit(&tfull[b]);  // also after a failed wait, so the epilogue moves on
         ++i;
@@ -811,16 +852,17 @@ void grouped_launch(const Bf16x3Gemm * gs, int n, cudaStream_t st) {
 // Width of the forward's tiles. 256 columns load the least per product (48 KB
 // per 32 k against 24 KB for 64) and stay as soon as the tiles fill the SMs;
 // below that the narrower tiles put more SMs to work on a chain that is K
-// blocks long. Per 32 k a tile took about 0.52 us at 256 columns and 0.39 at
-// 64 (what bounds it there is the issue of copies and MMAs by one thread
-// each, hence K blocks of 64 for the narrow tiles: 0.48 with blocks of 32),
-// plus about 2 us and 6 us per 256 columns of epilogue. At 100 clusters with
-// 1 000 sparse points (22 tiles of 256, 185 K blocks) 64 columns took 76 us
-// instead of 103; at 84 tiles and 32 K blocks 256 columns remain the choice.
+// blocks long. Per 32 k a tile takes about 0.53 us at 256 columns (MMAs and
+// copies share the shared memory: 0.42 us of either alone) and 0.30 at 64
+// (K blocks of 64 for the narrow tiles: their MMAs and copies are issued by
+// one thread each, and that issue bounds a block of 32), plus about 2 us and
+// 6 us per 256 columns of epilogue. At 100 clusters with 1 000 sparse points
+// (22 tiles of 256, 185 K blocks) 64 columns took 65 us instead of 103; at
+// 84 tiles and 32 K blocks 256 columns remain the choice.
 int gemm_forward_tile(const int64_t * rows, const int * M, int n, int64_t K) {
   constexpr int kSms = 148;
   const int widths[3] = {256, 128, 64};
-  const double per_block[3] = {0.52, 0.44, 0.39};
+  const double per_block[3] = {0.53, 0.33, 0.30};
   int best = widths[0];
   double best_us = 0.;
   for (int w = 0; w < 3; ++w) {
