@@ -29,159 +29,207 @@ namespace rgpu {
 namespace {
 
 constexpr int kThreads = 128;
-
-__device__ __forceinline__ float fc_cos_f(double r, double rc, double sw) {
-  if (r <= (rc - sw)) return 1.f;
-  if (r > rc) return 0.f;
-  double rs = 3.14159265358979323846264338327950288 * (r - rc + sw) / sw;
-  return float(0.5 * (1. + cos(rs)));
-}
-__device__ __forceinline__ float dfc_cos_f(double r, double rc, double sw) {
-  if (r <= (rc - sw)) return 0.f;
-  if (r > rc) return 0.f;
-  double rs = 3.14159265358979323846264338327950288 * (r - rc + sw) / sw;
-  return float(-0.5 * 3.14159265358979323846264338327950288 / sw * sin(rs));
-}
-
 constexpr int kMaxN = 16;  // largest max_radial of the register-staged path
+// Shared memory a block may take for dE/dc rows: four blocks of 128 threads
+// stay resident.
+constexpr size_t kStageBytes = 52 * 1024;
 
 // One thread per pair (pairs of many centres share a warp, so no lane idles
 // when centres have few neighbours). Per l, the n radial values RI and
-// p1 = dRI f_c + RI df_c are staged in registers (NV >= n of them); the
-// spherical-harmonics recurrence then streams (Y, grad Y) for that l.
+// p1 = dRI f_c + RI df_c are staged in registers (NV >= n of them) and the
+// harmonics of that l stream past them: polynomials q_lm(z) (x + iy)^m of the
+// unit vector, whose z derivative is the next order's q, and whose plain
+// gradient sum is projected onto the sphere once per pair at the end.
+//
 // dE/dc of the pair's centre is read as dC[i][lm][s*n + n'], n contiguous
-// values per lm (float4 loads when n == NV). With STRESS, the pair's
-// r_ji (x) g_ij (Voigt xx yy zz yz xz xy, the reference's
-// sparse_kernel_predict.hh:355-366) is summed per structure as well. With
-// `scale`, each structure's contributions are multiplied by scale[structure]
-// (an upstream gradient; a pass of its own over dE/dc took 114 us for 16 000
-// atoms).
-template <int L, int NV, bool STRESS>
-// 5 resident blocks per SM (96 registers, a few bytes of spills at L = 6)
-// measured faster than 4 (128 registers) or 6 (more spills)
-__global__ void __launch_bounds__(kThreads, 5)
+// values per lm (16-byte loads when n is a multiple of 4). These reads bound
+// the kernel: n (l+1)^2 values per pair, one lm at a time, each waiting on L1
+// or L2 with about 20 warps per SM to hide it (9.6 of the 16 cycles between a
+// warp's instructions at 46 neighbours, n = 12, l = 9). With STAGE the rows of
+// the block's centres (`rows` at a time) are therefore copied to shared memory
+// first, every copy in flight at once: 100 000 atoms with 46 neighbours at
+// n = 12, l = 9 take 3.5 ms instead of 4.2, 150 atoms with 60 neighbours at
+// n = 8, l = 6 16 us instead of 26. Blocks that span too many centres for
+// that (10 000 clusters, 12 neighbours, 7.8 KB rows: 1.0 ms) prefetch their
+// rows to L2 and read them there.
+//
+// With `stress`, the pair's r_ji (x) g_ij (Voigt xx yy zz yz xz xy, the
+// reference's sparse_kernel_predict.hh:355-366) is summed per structure as
+// well. With `scale`, each structure's contributions are multiplied by
+// scale[structure] (an upstream gradient; a pass of its own over dE/dc took
+// 114 us for 16 000 atoms).
+template <int L, int NV, bool STAGE>
+__global__ void __launch_bounds__(kThreads, NV <= 8 ? 5 : 4)
 pair_adjoint_kernel(ExpansionArgs a, const int32_t * __restrict__ pair_center, int64_t n_pairs,
                     const float * __restrict__ dC, double * __restrict__ F,
                     const int32_t * __restrict__ center_struct, double * __restrict__ stress,
-                    const double * __restrict__ scale) {
-  constexpr int K = (L + 1) * (L + 1);
+                    const double * __restrict__ scale, int rows) {
+  constexpr int L1 = L + 1, K = L1 * L1, SL = kMaxL + 2;
+  extern __shared__ __align__(16) float staged[];
   const int W = a.fd.W, n = a.fd.n, Sn = a.fd.S * a.fd.n;
   const bool vec = (n & 3) == 0;  // dE/dc rows of n floats as 16-byte loads
   const int lane = threadIdx.x & 31;
-  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+  const int row_len = Sn * K, row_step = ((row_len + 3) & ~3) + 4;  // staged rows start in different banks
+  const float ih = float(a.sp.inv_h);
   // the list's own total bounds the loop (below n_pairs when the list was
   // built to a capacity)
   {
     const int64_t listed = a.pair_off[a.n_centers];
     if (listed < n_pairs) n_pairs = listed;
   }
-  // the loop bound is warp-uniform: the F_i sums below shuffle across lanes
-  for (int64_t base = int64_t(blockIdx.x) * blockDim.x + threadIdx.x - lane; base < n_pairs; base += stride) {
-    const int64_t p = base + lane;
+  // the loop bound is uniform over the block: its warps stage rows together
+  // and their lanes shuffle below
+  for (int64_t base = int64_t(blockIdx.x) * blockDim.x; base < n_pairs; base += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t p = base + threadIdx.x;
     const int32_t ci = p < n_pairs ? pair_center[p] : -1;
-    {
+    int32_t c_first = 0, c_last = 0;  // the block's centres
+    if (STAGE) {
+      c_first = pair_center[base];
+      c_last = pair_center[min(base + int64_t(blockDim.x), n_pairs) - 1];
+    } else {
       // the lanes of one centre bring its dE/dc row (Sn K floats, read
       // below one lm at a time) towards L2 together, before the spline and
       // Y_lm work, so that the reads below wait on L2 rather than DRAM
       const unsigned same = __match_any_sync(0xffffffffu, ci);
       if (ci >= 0) {
         const int rank = __popc(same & lanemask_lt()), run = __popc(same);
-        const char * row = reinterpret_cast<const char *>(dC + size_t(ci) * Sn * K);
-        const int lines = (Sn * K * 4 + 127) >> 7;
+        const char * line = reinterpret_cast<const char *>(dC + size_t(ci) * row_len);
+        const int lines = (row_len * 4 + 127) >> 7;
         for (int k = rank; k < lines; k += run)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(row + (size_t(k) << 7)));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(line + (size_t(k) << 7)));
       }
     }
-    float g0 = 0.f, g1 = 0.f, g2 = 0.f;
-    float t6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float g0 = 0.f, g1 = 0.f, g2 = 0.f, x = 0.f, y = 0.f, z = 0.f, rf = 0.f;
     int32_t j = -1, self_atom = -1;
-    // the self pair carries no force of its own: the other pairs' F_i terms do
-    if (ci >= 0 && p != a.pair_off[ci]) {
+    for (int32_t c_lo = c_first; c_lo <= c_last; c_lo += STAGE ? rows : 1) {
+      const int32_t c_hi = STAGE ? min(c_last + 1, c_lo + rows) : 1;
+      if (STAGE) {
+        __syncthreads();  // the rows staged before are read no more
+        for (int32_t c = c_lo; c < c_hi; ++c) {
+          const float * src = dC + size_t(c) * row_len;
+          const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(staged + (c - c_lo) * row_step));
+          if ((row_len & 3) == 0) {
+            for (int e = threadIdx.x; e < row_len / 4; e += blockDim.x)
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * e), "l"(src + 4 * e) : "memory");
+          } else {
+            for (int e = threadIdx.x; e < row_len; e += blockDim.x)
+              asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4 * e), "l"(src + e) : "memory");
+          }
+        }
+        asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+      }
+      // the self pair carries no force of its own: the other pairs' F_i terms do
+      if (ci < 0 || p == a.pair_off[ci] || (STAGE && (ci < c_lo || ci >= c_hi))) continue;
       self_atom = a.center_atom[ci];
       const double r = a.pair_dist[p];
       j = a.pair_j[p];
       const int s = a.species_lut[a.types[j]];
-      float fc = fc_cos_f(r, a.rc, a.sw), dfc = dfc_cos_f(r, a.rc, a.sw);
-      if (a.rs.on) {
-        const double u = rs_value(a.rs, r);
-        const double cosw = 0.5 * (1. + cos(3.14159265358979323846264338327950288 * (r - a.rc + a.sw) / a.sw));
-        const double sr = (r <= a.rc - a.sw) ? 1.0 : (r > a.rc ? 0.0 : cosw);
-        dfc = float(rs_grad(a.rs, r) * sr + u * double(dfc));
-        fc = float(u * sr);
-      }
+      double fcd, dfcd;
+      cutoff_fc_dfc(a, r, fcd, dfcd);
+      const float fc = float(fcd), dfc = float(dfcd);
       const SplinePos q = spline_pos(a.sp, r);
       const float aa = float(q.a), bb = float(q.b);
       const float ca = aa * aa - 1.f, cb = bb * bb - 1.f;
       const float ea = 3.f * aa * aa - 1.f, eb = 3.f * bb * bb - 1.f;
-      const float ih = float(a.sp.inv_h);
       // interval k of the spline: (y_k, y2h_k, y_k+1, y2h_k+1) per channel
       const float4 * q4 = a.sp.q4f + size_t(q.k) * W;
-      const float * E = dC + size_t(ci) * Sn * K + s * n;
-      float rl[NV], pl[NV];
-      float sY = 0.f, sd0 = 0.f, sd1 = 0.f, sd2 = 0.f;
-      const float dx = float(a.pair_dir[3 * p]), dy = float(a.pair_dir[3 * p + 1]),
-                  dz = float(a.pair_dir[3 * p + 2]);
-      spherical_harmonics<L, true, float>(
-          dx, dy, dz,
-          [&](int lm, float y, float gx, float gy, float gz) {
-            float A = 0.f, B = 0.f;
-            const float * El = E + lm * Sn;
-            if (vec) {
-              const float4 * E4 = reinterpret_cast<const float4 *>(El);
+      const float * E = (STAGE ? staged + (ci - c_lo) * row_step : dC + size_t(ci) * row_len) + s * n;
+      x = float(a.pair_dir[3 * p]);
+      y = float(a.pair_dir[3 * p + 1]);
+      z = float(a.pair_dir[3 * p + 2]);
+      rf = float(r);
+      float re[L1], im[L1];  // (x + iy)^m
+      re[0] = 1.f;
+      im[0] = 0.f;
 #pragma unroll
-              for (int qq = 0; qq < NV / 4; ++qq) {
-                if (4 * qq < n) {
-                  const float4 ev = __ldg(E4 + qq);
-                  A = fmaf(ev.w, pl[4 * qq + 3],
-                           fmaf(ev.z, pl[4 * qq + 2], fmaf(ev.y, pl[4 * qq + 1], fmaf(ev.x, pl[4 * qq], A))));
-                  B = fmaf(ev.w, rl[4 * qq + 3],
-                           fmaf(ev.z, rl[4 * qq + 2], fmaf(ev.y, rl[4 * qq + 1], fmaf(ev.x, rl[4 * qq], B))));
-                }
-              }
-            } else {
-#pragma unroll
-              for (int nn = 0; nn < NV; ++nn) {
-                if (nn < n) {
-                  const float ev = __ldg(El + nn);
-                  A += ev * pl[nn];
-                  B += ev * rl[nn];
-                }
-              }
-            }
-            sY += A * y;
-            sd0 += B * gx;
-            sd1 += B * gy;
-            sd2 += B * gz;
-          },
-          [&](int l) {
-#pragma unroll
-            for (int nn = 0; nn < NV; ++nn) {
-              if (nn < n) {
-                const float4 t = __ldg(q4 + l * n + nn);
-                const float ri = aa * (t.x + ca * t.y) + bb * (t.z + cb * t.w);
-                const float dri = (t.z - t.x - ea * t.y + eb * t.w) * ih;
-                rl[nn] = ri;
-                pl[nn] = dri * fc + ri * dfc;
-              } else {
-                rl[nn] = 0.f;
-                pl[nn] = 0.f;
-              }
-            }
-          });
-      const float fr = fc / float(r);
-      const float up = scale ? float(scale[center_struct[ci]]) : 1.f;
-      g0 = up * (dx * sY + fr * sd0);
-      g1 = up * (dy * sY + fr * sd1);
-      g2 = up * (dz * sY + fr * sd2);
-      if constexpr (STRESS) {
-        const float rf = float(r), rx = -rf * dx, ry = -rf * dy, rz = -rf * dz;
-        t6[0] = rx * g0;
-        t6[1] = ry * g1;
-        t6[2] = rz * g2;
-        t6[3] = ry * g2;
-        t6[4] = rz * g0;
-        t6[5] = rx * g1;
+      for (int m = 1; m <= L; ++m) {
+        re[m] = re[m - 1] * x - im[m - 1] * y;
+        im[m] = re[m - 1] * y + im[m - 1] * x;
       }
+      float q1[L1], q0[L1 + 1];  // q of l - 1 and l
+      float sY = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
+      float cmm = 0.398942280401432677939946059934381868f;  // sqrt(1/(2 pi))
+#pragma unroll
+      for (int l = 0; l <= L; ++l) {
+        float rl[NV], pl[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+          rl[k] = pl[k] = 0.f;
+          if (k < n) {
+            const float4 t = __ldg(q4 + l * n + k);
+            const float ri = aa * (t.x + ca * t.y) + bb * (t.z + cb * t.w);
+            const float dri = (t.z - t.x - ea * t.y + eb * t.w) * ih;
+            rl[k] = ri;
+            pl[k] = dri * fc + ri * dfc;
+          }
+        }
+        // q_lm: q_mm, then the recursion in l (math/spherical_harmonics.cc:54-91)
+#pragma unroll
+        for (int m = 0; m < l; ++m) {
+          float v;
+          if (m == l - 1)
+            v = SphC<float>::c1(l) * z * q0[m];
+          else
+            v = (z * q0[m] + SphC<float>::b(l * SL + m) * q1[m]) * SphC<float>::a(l * SL + m);
+          q1[m] = q0[m];
+          q0[m] = v;
+        }
+        if (l > 0) cmm *= SphC<float>::c2(l);
+        q0[l] = cmm;
+        q1[l] = 0.f;
+        q0[l + 1] = 0.f;
+        auto dots = [&](int lm, float & A, float & B) {
+          const float * El = E + lm * Sn;
+          A = 0.f;
+          B = 0.f;
+          if (vec) {
+            const float4 * E4 = reinterpret_cast<const float4 *>(El);
+#pragma unroll
+            for (int k = 0; k < NV / 4; ++k)
+              if (4 * k < n) {
+                const float4 e = STAGE ? E4[k] : __ldg(E4 + k);
+                A = fmaf(e.w, pl[4 * k + 3], fmaf(e.z, pl[4 * k + 2], fmaf(e.y, pl[4 * k + 1], fmaf(e.x, pl[4 * k], A))));
+                B = fmaf(e.w, rl[4 * k + 3], fmaf(e.z, rl[4 * k + 2], fmaf(e.y, rl[4 * k + 1], fmaf(e.x, rl[4 * k], B))));
+              }
+          } else {
+#pragma unroll
+            for (int k = 0; k < NV; ++k)
+              if (k < n) {
+                const float e = STAGE ? El[k] : __ldg(El + k);
+                A = fmaf(e, pl[k], A);
+                B = fmaf(e, rl[k], B);
+              }
+          }
+        };
+        const int o = l * l + l;
+#pragma unroll
+        for (int m = 0; m <= l; ++m) {
+          // dq_lm/dz = -sqrt((l - m)(l + m + 1)) q_l,m+1
+          const float dq = m < l ? -SphC<float>::plm(l * SL + m) * q0[m + 1] : 0.f;
+          float A, B;
+          dots(o + m, A, B);
+          if (m == 0) {
+            constexpr float kInvSqrt2 = 0.707106781186547524400844362104849039f;
+            sY = fmaf(A, q0[0] * kInvSqrt2, sY);
+            sz = fmaf(B, dq * kInvSqrt2, sz);
+          } else {
+            float A2, B2;
+            dots(o - m, A2, B2);
+            const float tq = q0[m] * float(m), c = tq * re[m - 1], d = tq * im[m - 1];
+            sY = fmaf(q0[m], fmaf(A, re[m], A2 * im[m]), sY);
+            sx += fmaf(B, c, B2 * d);
+            sy += fmaf(B2, c, -B * d);
+            sz = fmaf(dq, fmaf(B, re[m], B2 * im[m]), sz);
+          }
+        }
+      }
+      // the tangential part of the gradient sum
+      const float radial = x * sx + y * sy + z * sz, fr = fc / rf;
+      const float up = scale ? float(scale[center_struct[ci]]) : 1.f;
+      g0 = up * (x * sY + fr * (sx - x * radial));
+      g1 = up * (y * sY + fr * (sy - y * radial));
+      g2 = up * (z * sY + fr * (sz - z * radial));
       atomicAdd(&F[3 * size_t(j) + 0], -double(g0));
       atomicAdd(&F[3 * size_t(j) + 1], -double(g1));
       atomicAdd(&F[3 * size_t(j) + 2], -double(g2));
@@ -189,9 +237,8 @@ pair_adjoint_kernel(ExpansionArgs a, const int32_t * __restrict__ pair_center, i
     // F_i += g unless j is a periodic image of i: the centre's pairs are
     // consecutive lanes, so a segmented warp scan leaves each run's sum in
     // its last lane and one atomic per run and component remains.
-    float h0 = (j >= 0 && j != self_atom) ? g0 : 0.f;
-    float h1 = (j >= 0 && j != self_atom) ? g1 : 0.f;
-    float h2 = (j >= 0 && j != self_atom) ? g2 : 0.f;
+    const bool other = j >= 0 && j != self_atom;
+    float h0 = other ? g0 : 0.f, h1 = other ? g1 : 0.f, h2 = other ? g2 : 0.f;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const float u0 = __shfl_up_sync(0xffffffffu, h0, off);
@@ -211,7 +258,9 @@ pair_adjoint_kernel(ExpansionArgs a, const int32_t * __restrict__ pair_center, i
       atomicAdd(&F[3 * size_t(ia) + 1], double(h1));
       atomicAdd(&F[3 * size_t(ia) + 2], double(h2));
     }
-    if constexpr (STRESS) {
+    if (stress) {
+      const float rx = -rf * x, ry = -rf * y, rz = -rf * z;  // zero without a pair of its own
+      float t6[6] = {rx * g0, ry * g1, rz * g2, ry * g2, rz * g0, rx * g1};
       // structures are consecutive runs of centres, hence of lanes
       const int32_t sid = ci >= 0 ? center_struct[ci] : -1;
 #pragma unroll
@@ -234,26 +283,36 @@ pair_adjoint_kernel(ExpansionArgs a, const int32_t * __restrict__ pair_center, i
 // One instantiation per (L, NV): compiled in the translation unit that owns
 // L (the library builds this file once per range of L, in parallel, since
 // each instantiation unrolls the spherical-harmonics recurrence).
+template <int L, int NV>
+void adjoint_launch_nv(const ExpansionArgs & a, const int32_t * pair_center, int64_t n_pairs, const float * dC,
+                       double * forces, cudaStream_t st, const int32_t * center_struct, double * stress,
+                       const double * scale, int grid, int threads) {
+  // rows of the centres a block of pairs spans on average, and two more; a
+  // block that spans others takes them in turn
+  const size_t row = sizeof(float) * (((size_t(a.fd.Sn) * a.fd.K + 3) & ~size_t(3)) + 4);
+  const int64_t per_centre = std::max<int64_t>(1, a.n_pairs / a.n_centers);
+  const int rows = int(threads / per_centre) + 2;
+  if (rows * row <= kStageBytes) {
+    auto kernel = pair_adjoint_kernel<L, NV, true>;
+    RGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kStageBytes)));
+    kernel<<<grid, threads, rows * row, st>>>(a, pair_center, n_pairs, dC, forces, center_struct, stress, scale, rows);
+  } else {
+    pair_adjoint_kernel<L, NV, false><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces, center_struct,
+                                                              stress, scale, 0);
+  }
+}
+
 template <int L>
 void adjoint_launch(const ExpansionArgs & a, const int32_t * pair_center, int64_t n_pairs, const float * dC,
                     double * forces, cudaStream_t st, const int32_t * center_struct, double * stress,
                     const double * scale, int grid, int threads) {
   sph_constants_tu();  // this translation unit's copy of the constants
-  if (a.fd.n <= 8) {
-    if (stress)
-      pair_adjoint_kernel<L, 8, true><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces,
-                                                               center_struct, stress, scale);
-    else
-      pair_adjoint_kernel<L, 8, false><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces, center_struct,
-                                                               nullptr, scale);
-  } else {
-    if (stress)
-      pair_adjoint_kernel<L, 16, true><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces,
-                                                               center_struct, stress, scale);
-    else
-      pair_adjoint_kernel<L, 16, false><<<grid, threads, 0, st>>>(a, pair_center, n_pairs, dC, forces, center_struct,
-                                                                nullptr, scale);
-  }
+  if (a.fd.n <= 8)
+    adjoint_launch_nv<L, 8>(a, pair_center, n_pairs, dC, forces, st, center_struct, stress, scale, grid, threads);
+  else if (a.fd.n <= 12)
+    adjoint_launch_nv<L, 12>(a, pair_center, n_pairs, dC, forces, st, center_struct, stress, scale, grid, threads);
+  else
+    adjoint_launch_nv<L, 16>(a, pair_center, n_pairs, dC, forces, st, center_struct, stress, scale, grid, threads);
 }
 
 }  // namespace
