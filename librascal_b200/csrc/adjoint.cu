@@ -61,7 +61,7 @@ __host__ __device__ constexpr int staged_row(int row_len) { return ((row_len + 3
 // the channel loops and the strides of 16-byte reads out of it.
 // Before and now: 100 000 atoms with 46 neighbours at n = 12, l = 9, 4.2 and
 // 1.9 ms; 10 000 clusters (n = 8, l = 6, 5 species) 1.04 and 0.64 ms; a box of
-// 150 atoms with 60 neighbours (n = 8, l = 6) 26 and 13.6 us; 97 cells at
+// 150 atoms with 34 neighbours (n = 8, l = 6) 26 and 13.6 us; 97 cells at
 // n = 7, l = 5, 384 and 254 us.
 //
 // With `stress`, the pair's r_ji (x) g_ij (Voigt xx yy zz yz xz xy, the

@@ -26,6 +26,11 @@ constexpr int kMaxWarps = 8;
 // 1.11 ms against 0.84 per 161 000 centres (its sums are written species by
 // species), and at 34 neighbours of 2 species 37 us against 33 per 2 000.
 constexpr int64_t kFewPairs = 40;
+// Centres per SM up to which a centre gets a block rather than a warp (warp
+// and block, us): 1 000 centres of a box 30 and 22, 1 600 of 100 clusters 26
+// and 22, 1 728 of a box at n = 12, l = 9 76 and 61; 2 000 of a box 33.5 and
+// 33.6, 3 200 of 200 clusters 30 and 38.
+constexpr int64_t kFewCentres = 12;
 
 template <int L, int NV>
 struct ExpSmem {
@@ -350,6 +355,172 @@ expansion_few_kernel(ExpansionArgs a, float * __restrict__ C, uint32_t * __restr
   }
 }
 
+// Few centres (see launch_expansion_fp32): a block of four warps per centre,
+// its pairs up to `chunk` at a time (more than one chunk adds to the
+// coefficients in global memory):
+//   (a) threads = pairs: distance, direction, spline weights, and the pair's
+//       place in the chunk's order by species;
+//   (b) threads = (pair, two orders m): Y_lm (pairs_f32.cuh); warps = pairs,
+//       lanes = radial channels: f_c RI, the table rows read whole;
+//   (c) threads = (species, four columns m of an l-block, four radial
+//       channels): per pair of the species two 16-byte loads from shared
+//       memory feed 16 products; the sums are written once, as 16-byte stores
+//       into the padded row layout [S*n][row_stride(L)] (Y is zero in the
+//       padding columns, so the padding of every l-block is written as zero).
+// A small system waits for one centre's chain of these steps, which four warps
+// shorten (150 centres, 34 neighbours, n = 8, l = 6: 29 -> 12.7 us; 216 with 46,
+// n = 12, l = 9: 69 -> 28); with many centres their barriers and idle lanes
+// cost more.
+constexpr int kBlockThreads = 128;
+template <int L>
+__global__ void __launch_bounds__(kBlockThreads)
+expansion_block_kernel(ExpansionArgs a, float * __restrict__ C, uint32_t * __restrict__ present, int chunk) {
+  using P = PairShape<L>;
+  constexpr int L1 = P::L1, NL = P::NL, RS = row_stride(L), OL = offp(L + 1), NG = OL / 4;
+  constexpr int kWarps = kBlockThreads / 32, kMaxChunk = kBlockThreads;
+  extern __shared__ __align__(16) float smf[];
+  __shared__ HarmonicConstants<L> hc;
+  __shared__ float4 wt[kMaxChunk];                // the spline's weights of each pair's nodes
+  __shared__ float geo[3][kMaxChunk];             // its direction
+  __shared__ int gk[kMaxChunk];                   // its spline interval
+  __shared__ int16_t dst_s[L1 * 16];              // channel (l, n) of the table -> place in a radial row
+  __shared__ int16_t counts[kMaxSpecies][kWarps];  // pairs of each species by warp
+  __shared__ int16_t first_s[kMaxSpecies + 1];    // first slot of each species
+  __shared__ uint8_t grp_l[NG];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int W = a.fd.W, S = a.fd.S, n = a.fd.n, nb = (n + 3) >> 2;  // blocks of four radial channels
+  const int RW = L1 * 4 * nb;
+  float * Y = smf;              // [chunk][RS]: padded columns of each pair, by species
+  float * R = smf + chunk * RS;  // [chunk][l][n rounded up to 4]
+  hc.fill();
+  for (int c = threadIdx.x; c < W; c += kBlockThreads) dst_s[c] = int16_t(c / n * 4 * nb + c % n);
+  for (int g = threadIdx.x; g < NG; g += kBlockThreads) {
+    int l = 0;
+    while (4 * g >= offp_rt(l + 1)) ++l;
+    grp_l[g] = uint8_t(l);
+  }
+  // padding columns of Y and channels past n stay zero
+  for (int e = threadIdx.x; e < chunk * (RS + RW); e += kBlockThreads) smf[e] = 0.f;
+  __syncthreads();
+  const int tasks = NG * nb;
+  for (int64_t ci = blockIdx.x; ci < a.n_centers; ci += gridDim.x) {
+    float * Ci = C + size_t(ci) * S * n * RS;
+    const int64_t p_lo = a.pair_off[ci] + 1, p_hi = a.pair_off[ci + 1];
+    const int ti = a.species_lut[a.types[a.center_atom[ci]]];
+    uint32_t mask = 1u << ti;
+    // the columns after the last l-block
+    for (int e = threadIdx.x; e < S * n * (RS - OL); e += kBlockThreads)
+      Ci[e / (RS - OL) * RS + OL + e % (RS - OL)] = 0.f;
+    bool first = true;
+    for (int64_t p0 = p_lo; p0 < p_hi || first; p0 += chunk, first = false) {
+      const int np = int(max(int64_t(0), min(int64_t(chunk), p_hi - p0)));
+      const int64_t p = p0 + threadIdx.x;
+      const bool own = int(threadIdx.x) < np;
+      const int sp = own ? a.species_lut[a.types[a.pair_j[p]]] : -1;
+      int rank = 0;  // among the warp's pairs of the same species
+      for (int s = 0; s < S; ++s) {
+        const unsigned m = __ballot_sync(0xffffffffu, sp == s);
+        if (lane == s) counts[s][wid] = int16_t(__popc(m));
+        if (sp == s) rank = __popc(m & lanemask_lt());
+      }
+      __syncthreads();
+      if (wid == 0) {
+        int mine = 0;
+        if (lane < S)
+          for (int w = 0; w < kWarps; ++w) mine += counts[lane][w];
+        mask |= __ballot_sync(0xffffffffu, mine > 0);
+        int upto = mine;
+#pragma unroll
+        for (int o = 1; o < kMaxSpecies; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, upto, o);
+          if (lane >= o) upto += u;
+        }
+        if (lane < S) first_s[lane + 1] = int16_t(upto);
+        if (lane == 0) first_s[0] = 0;
+      }
+      __syncthreads();
+      if (own) {
+        int slot = first_s[sp] + rank;
+        for (int w = 0; w < wid; ++w) slot += counts[sp][w];
+        const double r = a.pair_dist[p];
+        const SplinePos q = spline_pos(a.sp, r);
+        // f_c RI = w.x y_k + w.y y''_k + w.z y_k+1 + w.w y''_k+1
+        const float f = float(cutoff_fc(a, r)), fa = float(q.a), fb = float(q.b);
+        wt[slot] = make_float4(f * fa, f * fa * (fa * fa - 1.f), f * fb, f * fb * (fb * fb - 1.f));
+        gk[slot] = q.k;
+        for (int d = 0; d < 3; ++d) geo[d][slot] = float(a.pair_dir[3 * p + d]);
+      }
+      __syncthreads();
+      for (int q = threadIdx.x / NL; q < np && threadIdx.x < kBlockThreads / NL * NL; q += kBlockThreads / NL) {
+        float * y = Y + q * RS;
+        pair_harmonics<L>(hc, geo[0][q], geo[1][q], geo[2][q], threadIdx.x % NL,
+                          [&](int l, int m, float v, float, float re, float im, float, float) {
+                            float * o = y + offp_rt(l) + l;
+                            if (m == 0) {
+                              *o = v * 0.707106781186547524400844362104849039f;
+                            } else {
+                              o[m] = v * re;
+                              o[-m] = v * im;
+                            }
+                          });
+      }
+      for (int c = lane; c < W; c += 32) {
+        float * o = R + dst_s[c];
+        const float4 * table = a.sp.q4f + c;
+#pragma unroll 4
+        for (int q = wid; q < np; q += kWarps) {
+          const float4 t = __ldg(table + size_t(gk[q]) * W), w = wt[q];
+          o[q * RW] = fmaf(w.w, t.w, fmaf(w.z, t.z, fmaf(w.y, t.y, w.x * t.x)));
+        }
+      }
+      __syncthreads();
+      for (int t = threadIdx.x; t < S * tasks; t += kBlockThreads) {
+        const int s = t / tasks, u = t - s * tasks, b = u / NG, g = u - b * NG;
+        const int q0 = first_s[s], q1 = first_s[s + 1];
+        if (q0 == q1 && !first) continue;
+        const float * yp = Y + 4 * g;
+        const float * rp = R + grp_l[g] * 4 * nb + 4 * b;
+        float acc[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[k][e] = 0.f;
+#pragma unroll 2
+        for (int q = q0; q < q1; ++q) {
+          const float4 y = *reinterpret_cast<const float4 *>(yp + q * RS);
+          const float4 r = *reinterpret_cast<const float4 *>(rp + q * RW);
+          const float rv[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            acc[k][0] = fmaf(rv[k], y.x, acc[k][0]);
+            acc[k][1] = fmaf(rv[k], y.y, acc[k][1]);
+            acc[k][2] = fmaf(rv[k], y.z, acc[k][2]);
+            acc[k][3] = fmaf(rv[k], y.w, acc[k][3]);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int nn = 4 * b + k;
+          if (nn < n) {
+            float4 * o = reinterpret_cast<float4 *>(Ci + (s * n + nn) * RS + 4 * g);
+            float4 v = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+            if (first) {
+              // centre contribution (calculator_spherical_expansion.hh:2244-2247)
+              if (s == ti && g == 0) v.x += float(a.center_contrib[nn]);
+            } else {
+              const float4 before = *o;
+              v = make_float4(before.x + v.x, before.y + v.y, before.z + v.z, before.w + v.w);
+            }
+            *o = v;
+          }
+        }
+      }
+      __syncthreads();  // Y, R and the counts are read no more
+    }
+    if (threadIdx.x == 0) present[ci] = mask;
+  }
+}
+
 template <int L, int NV>
 void launch_nv(const ExpansionArgs & a, float * C, uint32_t * present, cudaStream_t st) {
   const TileConfig cfg = tile_config(a.fd.S, a.fd.n, a.fd.L);
@@ -416,13 +587,34 @@ void launch_few(const ExpansionArgs & a, float * C, uint32_t * present, cudaStre
 #undef RGPU_EXPF_NV
 }
 
+template <int L>
+void launch_block(const ExpansionArgs & a, float * C, uint32_t * present, cudaStream_t st) {
+  const size_t per_pair = (row_stride(L) + size_t(L + 1) * ((a.fd.n + 3) / 4 * 4)) * sizeof(float);
+  // pairs at a time: a warp's number on each of the four, while five blocks fit on an SM
+  int chunk = 4 * tile_config(a.fd.S, a.fd.n, a.fd.L).exp_chunk;
+  while (chunk > 16 && chunk * per_pair > 44 * 1024) chunk /= 2;
+  const size_t smem = chunk * per_pair;
+  auto kernel = expansion_block_kernel<L>;
+  RGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  int dev = 0, sms = 148, per_sm = 1;
+  RGPU_CUDA(cudaGetDevice(&dev));
+  RGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  RGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlockThreads, smem));
+  const int grid = int(std::min<int64_t>(a.n_centers, int64_t(sms) * std::max(per_sm, 1) * 4));
+  kernel<<<grid, kBlockThreads, smem, st>>>(a, C, present, chunk);
+}
+
 }  // namespace
 
 void launch_expansion_fp32(const ExpansionArgs & a, float * C, uint32_t * present, cudaStream_t st) {
   if (a.n_centers == 0) return;
   if (a.fd.n > 16) throw Error(RGPU_ERR_INVALID_ARGUMENT, "max_radial above 16 is not supported on the fast path");
   sph_constants_tu();
-  if (a.n_pairs < kFewPairs * a.n_centers) {
+  int dev = 0, sms = 148;
+  RGPU_CUDA(cudaGetDevice(&dev));
+  RGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const bool block = a.n_centers <= kFewCentres * sms;
+  if (!block && a.n_pairs < kFewPairs * a.n_centers) {
     launch_few(a, C, present, st);
     RGPU_LAUNCHED();
     RGPU_CUDA(cudaGetLastError());
@@ -430,7 +622,9 @@ void launch_expansion_fp32(const ExpansionArgs & a, float * C, uint32_t * presen
   }
 #define RGPU_CASE(LL)                            \
   case LL:                                       \
-    if (a.fd.n <= 8)                             \
+    if (block)                                   \
+      launch_block<LL>(a, C, present, st);       \
+    else if (a.fd.n <= 8)                        \
       launch_nv<LL, 8>(a, C, present, st);       \
     else if (a.fd.n <= 12)                       \
       launch_nv<LL, 12>(a, C, present, st);      \
