@@ -27,8 +27,8 @@ Reported for the gap-like workloads:
             structures are copied host->device and the energies and forces
             device->host inside the timed region;
   plain_fp64_ms_per_step, speedup_vs_plain_fp64
-            the plain FP64 GPU path (the reference's algorithm with the
-            materialised dX/dr) on the same batch, timed the same way;
+            the FP64 GPU path (features, kernel and adjoint forces in double
+            precision) on the same batch, timed the same way;
   force_err, energy_err
             max|F32 - F64| / max|F64| and max|E32 - E64| / max|E64| over the
             whole batch, and both GPU paths against the CPU oracle on the
@@ -401,11 +401,13 @@ def run_training(args):
             wall.append(time.perf_counter() - t)
             dev_ms.append(st.stage_times()[0])
     launches = int(lib.rgpu_kernel_launches(0) - l0)
-    # FP64 flops of the gradient block's GEMM: 2 * 3 * pairs_s * D * M_s per species
+    # FP64 flops of the gradient block's GEMM: 2 * 3 * pairs_s * D_b * M_s per
+    # species, D_b the columns of the neighbour's own species pairs (the
+    # others' derivatives are zero): S of the S (S + 1) / 2 pairs
     nl = st.neighbour_list()
     npc = np.diff(nl["pair_offsets"])
     zc = batch["numbers"][nl["center_atom"]]
-    D = T_sel.shape[1]
+    D = T_sel.shape[1] * 2.0 / (len(species) + 1)
     msp = {int(z): int(np.sum(np.asarray(sp.species) == z)) for z in set(sp.species)}
     flops = sum(2.0 * 3 * float(npc[zc == z].sum()) * D * m for z, m in msp.items())
     ms = float(np.mean(dev_ms))
@@ -438,9 +440,9 @@ def run_training(args):
                                      "l 6, GTO spline, %d sparse points, zeta 2; K_NM energy rows + 3 gradient "
                                      "rows per atom" % (n_struct, M),
                             n_atoms=n_atoms, output_gb=K_g.nbytes / 1e9,
-                            l2="inputs larger than L2: dX/dr chunks of up to 24 GB"),
-                roofline=dict(bound="fp64", kernel="gathered FP64 tile GEMM of the gradient block (dgemm.cuh), "
-                              "with the materialised dX/dr chunks in the same timed stage",
+                            l2="inputs larger than L2: feature rows of %.1f GB" % (8e-9 * n_atoms * T_sel.shape[1])),
+                roofline=dict(bound="fp64", kernel="FP64 tensor-core GEMM of the gradient block (dgemm.cuh), "
+                              "with its short pair rows in the same timed stage",
                               achieved=achieved, peak=fp64_peak, unit="TFLOP/s",
                               frac=achieved / fp64_peak, traffic=None, peak_kind=fp64_kind,
                               flops_per_step=flops),

@@ -71,7 +71,7 @@ void build_radial_spline(const Hypers & hy, RadialSpline & out);
 // candidates with CUDA events and commits its choices as a table that the
 // package loads into the library; shapes without an entry use the defaults.
 struct TileConfig {
-  int exp_chunk = 16;          // neighbour pairs per chunk of the FP32 expansion: 8, 16 or 32
+  int exp_chunk = 16;          // pairs per warp and chunk of the FP32 expansion: 8, 16 or 32 (unused where a warp keeps its sums in registers)
   int exp_warps = 4;           // centres (one warp each) per block of the FP32 expansion: 1..8
   int adj_threads = 128;       // threads per block of the pair adjoint: 32..128, multiple of 32
   int adj_blocks_per_sm = 64;  // grid cap of the pair adjoint, in blocks per SM: 1..256
