@@ -2,7 +2,9 @@
 // order, is expansion.cu): C[i][S n][row_stride(L)], each l-block padded to
 // four floats, and the mask of the species among the centre's neighbours.
 //
-// One warp per centre, pairs by species (pairs_f32.cuh). The coefficients of
+// Three kernels, by neighbours per centre and by the number of centres (see
+// launch_expansion_fp32 and the constants below). With many neighbours: one
+// warp per centre, pairs by species (pairs_f32.cuh). The coefficients of
 // one species stay in registers, lanes over lm and n per lane, while its pairs
 // pass: per pair and 32 lm one value of Y and n/4 broadcast loads of f_c RI
 // feed n products. They are written once per species. The previous kernel kept

@@ -1,14 +1,10 @@
-// What the FP32 expansion and the FP32 pair adjoint share: one warp works on
-// one centre, its pairs sorted by neighbour species, a few at a time.
-//   * geometry (lanes = pairs): distance, direction, spline interval, cutoff;
+// What the FP32 expansion kernels share:
 //   * harmonics (lanes = (pair, two orders m)): each lane runs the recursions
 //     in l of the orders m = j and m = L - j, L + 2 steps together whatever j,
 //     so a warp evaluates 32 / ceil((L + 1) / 2) pairs (8 at L = 6) at once
 //     with few lanes idle; one lane per pair left 24 of 32 idle for the eight
 //     pairs a centre and species has at a time;
-//   * radial table (lanes = channels): rows of the table are read whole, one
-//     8-byte node per lane. A lane per pair touches one 128-byte line per
-//     channel and lane instead, which bounded the adjoint.
+//   * the order of a centre's pairs by neighbour species, a window at a time.
 #pragma once
 
 #include "common.cuh"
