@@ -350,6 +350,7 @@ __global__ void nl_boxsort_kernel(int64_t n_boxes, int per, const int64_t * __re
 
 struct GatherCtx {
   const int64_t * atom_off;
+  const int32_t * tag2idx;  // null: atoms in tag order
   const int64_t * center_off;
   const int32_t * center_struct_in;  // structure of each centre row
   const NlGeom * geom;
@@ -360,7 +361,7 @@ struct GatherCtx {
   const double * sorted_x;
   const double * site_x;
   double cutoff, rc2;
-  int64_t box_cap, pair_cap;  // capacities (the exact counts when synchronised)
+  int64_t site_cap, box_cap, pair_cap;  // capacities (the exact counts when synchronised)
   DevStatus * status;
 };
 
@@ -381,36 +382,47 @@ __global__ void nl_gather_kernel(int64_t n_centers, GatherCtx c, int64_t * __res
   const int s = c.center_struct_in[ci];
   const NlGeom & g = c.geom[s];
   const int64_t a0 = c.atom_off[s];
-  const int64_t site = a0 + c.ghost_off[a0] + (ci - c.center_off[s]);
-  const double xi[3] = {c.site_x[3 * site], c.site_x[3 * site + 1], c.site_x[3 * site + 2]};
-  int b[3];
-  box_of(g, xi, c.cutoff, b);
-  b[0] = min(b[0], g.nboxes[0] - 2);
-  b[1] = min(b[1], g.nboxes[1] - 2);
-  b[2] = min(b[2], g.nboxes[2] - 2);
-  // a structure whose mesh reaches past the box capacity is skipped (capacity mode)
-  if (c.box_base[s] + int64_t(g.nboxes[0]) * g.nboxes[1] * g.nboxes[2] > c.box_cap) {
-    if (lane == 0) set_status(c.status, 104, s, 0);
-    if (MODE == 0 && lane == 0) count[ci] = 1;
-    return;
-  }
-  int64_t out = 0;
+  const int64_t tag = a0 + (ci - c.center_off[s]), site = tag + c.ghost_off[a0];
   int64_t base = 0;
   if (MODE == 1) {
+    // The centre and its self pair come first and from the atom itself, so
+    // that every centre and every pair slot below the list's total is written
+    // whatever the capacities cut off below: the kernels that follow index
+    // with them before the host has read the status.
+    const int32_t atom = c.tag2idx ? c.tag2idx[tag] : int32_t(tag);
     base = pair_off[ci];
-    if (base + 1 + 0 > c.pair_cap) {  // not even the self pair fits
+    if (lane == 0) center_atom[ci] = atom;
+    if (base >= c.pair_cap) {  // not even the self pair fits
       if (lane == 0) set_status(c.status, 104, s, int(ci));
       return;
     }
     if (lane == 0) {
-      center_atom[ci] = site_real[site];
-      pair_j[base] = site_real[site];
+      pair_j[base] = atom;
+      pair_center[base] = int32_t(ci);
       pair_shift[3 * base] = pair_shift[3 * base + 1] = pair_shift[3 * base + 2] = 0;
       pair_dist[base] = 0.;
       pair_dir[3 * base] = pair_dir[3 * base + 1] = pair_dir[3 * base + 2] = 0.;
     }
     base += 1;
   }
+  // Capacity mode: a centre past the site capacity has no site to read, and a
+  // structure whose mesh reaches past the box capacity has no box offsets;
+  // both keep their self pair alone.
+  if (site >= c.site_cap ||
+      c.box_base[s] + int64_t(g.nboxes[0]) * g.nboxes[1] * g.nboxes[2] > c.box_cap) {
+    if (lane == 0) {
+      set_status(c.status, 104, s, int(ci));
+      if (MODE == 0) count[ci] = 1;
+    }
+    return;
+  }
+  const double xi[3] = {c.site_x[3 * site], c.site_x[3 * site + 1], c.site_x[3 * site + 2]};
+  int b[3];
+  box_of(g, xi, c.cutoff, b);
+  b[0] = min(b[0], g.nboxes[0] - 2);
+  b[1] = min(b[1], g.nboxes[1] - 2);
+  b[2] = min(b[2], g.nboxes[2] - 2);
+  int64_t out = 0;
   // The stencil's 9 box rows (dx, dy; 3 boxes along z each) are runs of the
   // box-sorted sites; lanes 0..8 read one run's bounds each, all at once.
   int64_t run_lo = 0, run_len = 0;
@@ -483,7 +495,7 @@ __global__ void nl_gather_kernel(int64_t n_centers, GatherCtx c, int64_t * __res
   }
   if (MODE == 0 && lane == 0) count[ci] = out + 1;
   if (MODE == 1)
-    for (int64_t p = base - 1 + lane; p < base + out && p < c.pair_cap; p += 32) pair_center[p] = int32_t(ci);
+    for (int64_t p = base + lane; p < base + out && p < c.pair_cap; p += 32) pair_center[p] = int32_t(ci);
   (void)site_type;
 }
 
@@ -636,6 +648,7 @@ void build_neighbour_list(const NlInputs & in, double cutoff, NlWork & w, NlOutp
   // 5. count, scan, fill
   GatherCtx c;
   c.atom_off = in.atom_off;
+  c.tag2idx = in.tag2idx;
   c.center_off = in.center_off;
   c.center_struct_in = center_struct;
   c.geom = geom;
@@ -647,6 +660,7 @@ void build_neighbour_list(const NlInputs & in, double cutoff, NlWork & w, NlOutp
   c.site_x = w.site_x.as<double>();
   c.cutoff = cutoff;
   c.rc2 = cutoff * cutoff;
+  c.site_cap = n_sites;
   c.box_cap = n_boxes;
   c.pair_cap = INT64_MAX;  // set below, once the pair count or capacity is known
   c.status = status_dev;
