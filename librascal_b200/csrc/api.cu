@@ -438,6 +438,14 @@ void reset_status(rgpu_structures * s) {
   *s->status_h = HandleStatus{};
 }
 
+// Nothing computed so far is reused by a later call: the list, the features
+// and what a forward left for its backward.
+void drop_results(rgpu_structures * s) {
+  s->nl_valid = false;
+  s->feat_valid = false;
+  s->fwd_model = nullptr;
+}
+
 void mark(rgpu_structures * s, int i) {
   if (s->timed) RGPU_CUDA(cudaEventRecord(s->ev[i], s->st));
 }
@@ -1603,6 +1611,7 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
   if (replay) {
     std::memcpy(s->md_pos_h, positions, sizeof(double) * 3 * na);
     ensure_chunk_map(s, make_dims(m->calc->hy, int(s->species.size())));
+    drop_results(s);  // the replay overwrites positions, list and features
     RGPU_CUDA(cudaGraphLaunch(s->md_exec, s->st));
     RGPU_CUDA(cudaStreamSynchronize(s->st));
     ++s->md_replays;
@@ -1618,9 +1627,8 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
   }
   md_drop(s);
   // the ordinary path: checks the input, sizes every buffer, gives this step's results
+  drop_results(s);
   upload_positions(s, positions);
-  s->nl_valid = false;
-  s->feat_valid = false;
   gap_predict_impl(m, s, RGPU_PRECISION_FP32, energies, forces, neg_stress);
   if (s->md_no_graph) return;
   // capacities 25 % above this step's counts
@@ -1644,6 +1652,7 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
   // one run without recording sizes the capacity buffers (no allocation may
   // happen while recording) and checks that the step fits them
   s->timed = false;
+  drop_results(s);  // the list becomes the capacity-bound one
   md_enqueue(m, s, stress);
   RGPU_CUDA(cudaStreamSynchronize(s->st));
   if (s->status_h->nl.code != 0 || timed_out(s)) {
@@ -1674,8 +1683,6 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
     (void)cudaGetLastError();
     md_drop(s);
     s->md_no_graph = true;
-    s->nl_valid = false;
-    s->feat_valid = false;
     return;
   }
   s->md_model = m;
@@ -1686,8 +1693,6 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
   s->md_replays = 0;
   // the ordinary step above already produced this call's results; the
   // positions of the next step arrive in md_pos_h
-  s->nl_valid = false;
-  s->feat_valid = false;
 }
 
 // ------------------------------------------------- predictions as CUDA graphs
@@ -1744,13 +1749,9 @@ static bool pgraph_replay(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
     if (g.buffers != bufs) continue;
     s->timed = false;
     if (g.forces) ensure_chunk_map(s, s->fd);
+    drop_results(s);  // the list becomes the capacity-bound one
     RGPU_CUDA(cudaGraphLaunch(g.exec, s->st));
     RGPU_CUDA(cudaStreamSynchronize(s->st));
-    // the list on the device is the capacity-bound one: nothing computed here
-    // is reused by a later call
-    s->nl_valid = false;
-    s->feat_valid = false;
-    s->fwd_model = nullptr;
     check_timeout(s);
     if (s->status_h->nl.code != 0) {
       reset_status(s);
