@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -148,7 +149,20 @@ void parse_hypers(const std::string & kind, const std::string & text, Hypers & h
 }  // namespace rgpu
 
 // ------------------------------------------------------------------ handles
+// What a structure set keeps of a calculator or model (features, recorded
+// calls) is tied to its serial number: an address may be that of a later
+// object, whose buffers may lie where the former's did.
+static uint64_t next_serial() {
+  static std::atomic<uint64_t> n{0};
+  return ++n;
+}
+template <class Handle>
+static uint64_t serial_of(const Handle * h) {
+  return h ? h->serial : 0;
+}
+
 struct rgpu_calculator {
+  const uint64_t serial{next_serial()};
   int device{-1};  // device of the uploaded tables (-1: not uploaded yet)
   Hypers hy;
   RadialSpline spline;
@@ -182,7 +196,7 @@ struct GapLayout;
 struct PredictGraph {
   cudaGraph_t graph{nullptr};
   cudaGraphExec_t exec{nullptr};
-  const rgpu_gap_model * model{nullptr};
+  uint64_t model{0};  // serial
   bool stress{false}, outputs{false}, forces{true};
   int n_struct{0};
   int64_t n_atoms{0};
@@ -229,7 +243,7 @@ struct rgpu_structures {
   DevBuf row_of_center, center_of_row, sort_tmp, present, tile_mask;
   DevBuf C64, X64, invn64, dC64, C32, X32, xscale32;  // xscale32[row] = 1/|p| (FP32 path)
   int feat_precision{-1};
-  const rgpu_calculator * feat_calc{nullptr};
+  uint64_t feat_calc{0};  // serial
   bool feat_gradients{false};
   bool feat_valid{false};
   // GAP work
@@ -243,7 +257,7 @@ struct rgpu_structures {
   // MD step recorded as a CUDA graph (rgpu_md_step)
   cudaGraph_t md_graph{nullptr};
   cudaGraphExec_t md_exec{nullptr};
-  const rgpu_gap_model * md_model{nullptr};
+  uint64_t md_model{0};  // serial
   bool md_stress{false};
   NlCaps md_caps{};
   std::vector<const void *> md_buffers;  // device buffer addresses at recording
@@ -261,9 +275,10 @@ struct rgpu_structures {
   bool use_graphs{true};
   uint64_t pgraph_clock{0};
   int64_t pgraph_replays{0}, pgraph_records{0}, pgraph_last_kernels{0};
-  // autograd: the model whose forward (rgpu_gap_forward_dev) left W, the
-  // features and the list in place for rgpu_gap_backward_dev (null: none)
-  const rgpu_gap_model * fwd_model{nullptr};
+  // autograd: the serial of the model whose forward (rgpu_gap_forward_dev)
+  // left W, the features and the list in place for rgpu_gap_backward_dev (0:
+  // none)
+  uint64_t fwd_model{0};
   DevBuf y0_d;  // per-structure energy baseline of fwd_model
   // status and timing
   HandleStatus * status_d{nullptr};
@@ -277,6 +292,7 @@ struct rgpu_structures {
 };
 
 struct rgpu_gap_model {
+  const uint64_t serial{next_serial()};
   int device{-1};  // device of the model's buffers (-1: none allocated yet)
   rgpu_calculator * calc{nullptr};
   std::vector<int> species;  // model layout species (sorted)
@@ -443,7 +459,7 @@ void reset_status(rgpu_structures * s) {
 void drop_results(rgpu_structures * s) {
   s->nl_valid = false;
   s->feat_valid = false;
-  s->fwd_model = nullptr;
+  s->fwd_model = 0;
 }
 
 void mark(rgpu_structures * s, int i) {
@@ -497,7 +513,7 @@ void set_layout(rgpu_structures * s, const Hypers & hy, const std::vector<int> &
 
 void build_nl(rgpu_structures * s, double cutoff) {
   if (s->nl_valid && s->nl_cutoff == cutoff) return;
-  s->fwd_model = nullptr;
+  s->fwd_model = 0;
   NlInputs in;
   in.n_struct = s->n_struct;
   in.n_atoms = s->n_atoms;
@@ -605,12 +621,12 @@ void compute_features(rgpu_calculator * c, rgpu_structures * s, int precision, b
                       const std::vector<int> & extra_species, bool need_x32 = true) {
   build_nl(s, c->hy.cutoff);
   set_layout(s, c->hy, extra_species);
-  if (s->feat_valid && s->feat_calc == c && s->feat_precision == precision &&
+  if (s->feat_valid && s->feat_calc == c->serial && s->feat_precision == precision &&
       (precision == RGPU_PRECISION_FP64 || s->feat_x32 || !need_x32)) {
     s->feat_gradients = s->feat_gradients || grads;
     return;
   }
-  s->fwd_model = nullptr;
+  s->fwd_model = 0;
   mark(s, 2);
   const bool by_mask = precision == RGPU_PRECISION_FP32 && sorts_by_mask(c, s);
   sort_rows(s, by_mask);
@@ -650,7 +666,7 @@ void compute_features(rgpu_calculator * c, rgpu_structures * s, int precision, b
     s->feat_x32 = need_x32;
   }
   s->feat_valid = true;
-  s->feat_calc = c;
+  s->feat_calc = c->serial;
   s->feat_precision = precision;
   s->feat_gradients = grads;
 }
@@ -980,7 +996,7 @@ void gap_fast_forward(rgpu_gap_model * m, rgpu_structures * s, double * E_d, boo
   const FeatureDims & fd = s->fd;
   const int64_t nc = s->nl.n_centers;
   cudaStream_t st = s->st;
-  s->fwd_model = nullptr;
+  s->fwd_model = 0;
   mark(s, 4);
   // per-species W (BF16 hi/lo) and energy partials ([tiles along M][rows])
   int points[kMaxSpecies];
@@ -1254,7 +1270,7 @@ static void gap_forward_dev_impl(rgpu_gap_model * m, rgpu_structures * s, const 
   fetch_status(s);
   RGPU_CUDA(cudaStreamSynchronize(s->st));
   check_timeout(s);
-  s->fwd_model = m;
+  s->fwd_model = m->serial;
 }
 
 // Backward half: grad_dev[a][c] = sum_A energies_grad_dev[A] dE_A/dr_a[c]
@@ -1263,7 +1279,7 @@ static void gap_forward_dev_impl(rgpu_gap_model * m, rgpu_structures * s, const 
 static void gap_backward_dev_impl(rgpu_gap_model * m, rgpu_structures * s, const double * energies_grad_dev,
                                   double * grad_dev) {
   if (!m || !s || !energies_grad_dev || !grad_dev) throw Error(RGPU_ERR_INVALID_ARGUMENT, "null argument");
-  if (s->fwd_model != m || !s->feat_valid || !s->nl_valid)
+  if (s->fwd_model != m->serial || !s->feat_valid || !s->nl_valid)
     throw Error(RGPU_ERR_NOT_COMPUTED, "the backward needs the forward of the same model and structures, with "
                                        "no other call on the structures in between");
   s->timed = false;
@@ -1495,7 +1511,7 @@ static void md_drop(rgpu_structures * s) {
   if (s->md_graph) cudaGraphDestroy(s->md_graph);
   s->md_exec = nullptr;
   s->md_graph = nullptr;
-  s->md_model = nullptr;
+  s->md_model = 0;
 }
 
 // The FP32 prediction on the structures' stream with no host
@@ -1600,7 +1616,7 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
   ensure_stream(s);
   bool replay = false;
   if (s->md_exec) {
-    if (s->md_model != m || s->md_stress != stress || m->layout_species != s->species ||
+    if (s->md_model != m->serial || s->md_stress != stress || m->layout_species != s->species ||
         s->md_species != s->species)
       s->md_reason = 3;
     else if (md_buffers(m, s) != s->md_buffers)
@@ -1685,7 +1701,7 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
     s->md_no_graph = true;
     return;
   }
-  s->md_model = m;
+  s->md_model = m->serial;
   s->md_stress = stress;
   s->md_buffers = md_buffers(m, s);
   s->md_species = s->species;
@@ -1742,7 +1758,7 @@ static bool pgraph_replay(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   const std::vector<int64_t> cnt = centres_per_species(s);
   std::vector<const void *> bufs;
   for (PredictGraph & g : s->pgraphs) {
-    if (g.model != m || g.stress != stress || g.outputs != outputs || g.forces != want_forces ||
+    if (g.model != m->serial || g.stress != stress || g.outputs != outputs || g.forces != want_forces ||
         g.n_struct != s->n_struct || g.n_atoms != s->n_atoms || g.species != s->species || g.species_count != cnt)
       continue;
     if (bufs.empty()) bufs = md_buffers(m, s);
@@ -1781,7 +1797,7 @@ static void pgraph_record(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   g.caps.sites = sites + sites / 8 + 64;
   g.caps.boxes = boxes + boxes / 8 + 64;
   g.caps.pairs = s->nl.n_pairs + s->nl.n_pairs / 8 + 256;
-  g.model = m;
+  g.model = m->serial;
   g.stress = stress;
   g.outputs = outputs;
   g.forces = forces;
@@ -1819,7 +1835,7 @@ static void pgraph_record(rgpu_gap_model * m, rgpu_structures * s, bool stress, 
   }
   s->nl_valid = false;
   s->feat_valid = false;
-  s->fwd_model = nullptr;
+  s->fwd_model = 0;
   if (!ok) {
     (void)cudaGetLastError();
     reset_status(s);
@@ -2043,7 +2059,7 @@ rgpu_status rgpu_structures_set(rgpu_structures * s, int32_t n_structures, const
     upload_inputs(s, ups);
     s->nl_valid = false;
     s->feat_valid = false;
-    s->fwd_model = nullptr;
+    s->fwd_model = 0;
   });
 }
 
@@ -2053,7 +2069,7 @@ rgpu_status rgpu_structures_update_positions(rgpu_structures * s, const double *
     upload_positions(s, positions);
     s->nl_valid = false;
     s->feat_valid = false;
-    s->fwd_model = nullptr;
+    s->fwd_model = 0;
   });
 }
 
@@ -2062,7 +2078,7 @@ rgpu_status rgpu_structures_invalidate(rgpu_structures * s) {
     OnDevice on_dev(s);
     s->nl_valid = false;
     s->feat_valid = false;
-    s->fwd_model = nullptr;
+    s->fwd_model = 0;
   });
 }
 
@@ -2138,7 +2154,7 @@ rgpu_status rgpu_get_feature_keys(const rgpu_calculator * calc, const rgpu_struc
                                   int32_t * keys) {
   return guard([&] {
     OnDevice on_dev(s);
-    if (!s->feat_valid || s->feat_calc != calc) throw Error(RGPU_ERR_NOT_COMPUTED, "features have not been computed");
+    if (!s->feat_valid || s->feat_calc != serial_of(calc)) throw Error(RGPU_ERR_NOT_COMPUTED, "features have not been computed");
     auto k = present_keys(calc, s);
     *n_keys = int32_t(k.size());
     if (keys)
@@ -2153,7 +2169,7 @@ rgpu_status rgpu_get_features(const rgpu_calculator * calc, const rgpu_structure
                               const int32_t * keys, double * out) {
   return guard([&] {
     OnDevice on_dev(s);
-    if (!s->feat_valid || s->feat_calc != calc) throw Error(RGPU_ERR_NOT_COMPUTED, "features have not been computed");
+    if (!s->feat_valid || s->feat_calc != serial_of(calc)) throw Error(RGPU_ERR_NOT_COMPUTED, "features have not been computed");
     const FeatureDims & fd = s->fd;
     const int64_t nc = s->nl.n_centers;
     const bool ps = calc->hy.kind == "sphericalinvariants";
@@ -2194,7 +2210,7 @@ rgpu_status rgpu_get_features_gradient(const rgpu_calculator * calc, const rgpu_
   return guard([&] {
     OnDevice on_dev(s_in);
     rgpu_structures * s = const_cast<rgpu_structures *>(s_in);
-    if (!s->feat_valid || s->feat_calc != calc) throw Error(RGPU_ERR_NOT_COMPUTED, "features have not been computed");
+    if (!s->feat_valid || s->feat_calc != serial_of(calc)) throw Error(RGPU_ERR_NOT_COMPUTED, "features have not been computed");
     if (!s->feat_gradients) throw Error(RGPU_ERR_NOT_COMPUTED, "gradients were not requested (compute_gradients)");
     if (s->feat_precision != RGPU_PRECISION_FP64)
       throw Error(RGPU_ERR_INVALID_ARGUMENT, "dense gradients are exported from the FP64 path");
