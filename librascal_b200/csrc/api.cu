@@ -173,6 +173,7 @@ struct rgpu_calculator {
 // A part of a device buffer.
 struct DevView {
   void * p{nullptr};
+  size_t bytes{0};
   template <class T>
   T * as() const {
     return static_cast<T *>(p);
@@ -404,6 +405,7 @@ void upload_inputs(rgpu_structures * s, const std::vector<Upload> & ups) {
   size_t off = 0;
   for (const Upload & u : ups) {
     u.dst->p = s->in_d.as<unsigned char>() + off;
+    u.dst->bytes = u.bytes;
     if (u.bytes) std::memcpy(base + off, u.src, u.bytes);
     off += (u.bytes + 255) & ~size_t(255);
   }
@@ -414,6 +416,7 @@ void upload_inputs(rgpu_structures * s, const std::vector<Upload> & ups) {
 void upload_positions(rgpu_structures * s, const double * positions) {
   const size_t bytes = sizeof(double) * 3 * size_t(s->n_atoms);
   if (bytes == 0) return;
+  if (bytes > s->pos_d.bytes) throw Error(RGPU_ERR_INVALID_ARGUMENT, "the structures have not been uploaded");
   RGPU_CUDA(cudaStreamSynchronize(s->st));  // staging buffer reuse
   void * p = staging(s, bytes);
   std::memcpy(p, positions, bytes);
@@ -1997,88 +2000,98 @@ rgpu_status rgpu_structures_set(rgpu_structures * s, int32_t n_structures, const
   return guard([&] {
     OnDevice on_dev(s);
     if (!s || n_structures < 0 || !atom_offsets) throw Error(RGPU_ERR_INVALID_ARGUMENT, "null argument");
+    // everything is checked before the handle changes: a batch that is refused
+    // leaves the former one in place
+    if (atom_offsets[0] != 0) throw Error(RGPU_ERR_INVALID_ARGUMENT, "atom_offsets must start at 0");
+    for (int i = 0; i < n_structures; ++i)
+      if (atom_offsets[i + 1] < atom_offsets[i])
+        throw Error(RGPU_ERR_INVALID_ARGUMENT, "atom_offsets must be non-decreasing");
+    const int64_t n_atoms = atom_offsets[n_structures];
+    if (n_atoms > (int64_t(1) << 31) - 1) throw Error(RGPU_ERR_INVALID_ARGUMENT, "too many atoms");
+    bool seen[130] = {false};
+    for (int64_t a = 0; a < n_atoms; ++a) {
+      if (numbers[a] < 0 || numbers[a] >= 130)
+        throw Error(RGPU_ERR_STRUCTURE, "atom types (or atomic numbers) should be in the range [0, 130].");
+      seen[numbers[a]] = true;
+    }
+    ensure_stream(s);
     md_drop(s);
     s->md_no_graph = false;
-    ensure_stream(s);
-    s->n_struct = n_structures;
-    s->atom_off.assign(atom_offsets, atom_offsets + n_structures + 1);
-    if (s->atom_off[0] != 0) throw Error(RGPU_ERR_INVALID_ARGUMENT, "atom_offsets must start at 0");
-    for (int i = 0; i < n_structures; ++i)
-      if (s->atom_off[i + 1] < s->atom_off[i]) throw Error(RGPU_ERR_INVALID_ARGUMENT, "atom_offsets must be non-decreasing");
-    s->n_atoms = s->atom_off[n_structures];
-    if (s->n_atoms > (int64_t(1) << 31) - 1) throw Error(RGPU_ERR_INVALID_ARGUMENT, "too many atoms");
-    s->types.assign(numbers, numbers + s->n_atoms);
-    s->cells_h.assign(cells, cells + 9 * size_t(n_structures));
-    bool seen[130] = {false};
-    for (int64_t a = 0; a < s->n_atoms; ++a) {
-      if (s->types[a] < 0 || s->types[a] >= 130)
-        throw Error(RGPU_ERR_STRUCTURE, "atom types (or atomic numbers) should be in the range [0, 130].");
-      seen[s->types[a]] = true;
-    }
-    s->batch_species.clear();
-    for (int z = 0; z < 130; ++z)
-      if (seen[z]) s->batch_species.push_back(z);
-    s->has_mask = false;
-    if (center_mask)
+    drop_results(s);
+    try {
+      s->n_struct = n_structures;
+      s->atom_off.assign(atom_offsets, atom_offsets + n_structures + 1);
+      s->n_atoms = n_atoms;
+      s->types.assign(numbers, numbers + s->n_atoms);
+      s->cells_h.assign(cells, cells + 9 * size_t(n_structures));
+      s->batch_species.clear();
+      for (int z = 0; z < 130; ++z)
+        if (seen[z]) s->batch_species.push_back(z);
+      s->has_mask = false;
+      if (center_mask)
+        for (int64_t a = 0; a < s->n_atoms; ++a)
+          if (!center_mask[a]) s->has_mask = true;
+      std::fill(s->centres_of_type, s->centres_of_type + 130, int64_t(0));
       for (int64_t a = 0; a < s->n_atoms; ++a)
-        if (!center_mask[a]) s->has_mask = true;
-    std::fill(s->centres_of_type, s->centres_of_type + 130, int64_t(0));
-    for (int64_t a = 0; a < s->n_atoms; ++a)
-      if (!center_mask || center_mask[a]) ++s->centres_of_type[s->types[a]];
-    std::vector<int32_t> ncent(n_structures), astruct(s->n_atoms);
-    s->center_off_h.assign(n_structures + 1, 0);
-    std::vector<int32_t> tag2idx;
-    if (s->has_mask) tag2idx.resize(s->n_atoms);
-    for (int i = 0; i < n_structures; ++i) {
-      int64_t a0 = s->atom_off[i], a1 = s->atom_off[i + 1];
-      int nc = 0;
-      for (int64_t a = a0; a < a1; ++a) {
-        astruct[a] = i;
-        if (!center_mask || center_mask[a]) ++nc;
+        if (!center_mask || center_mask[a]) ++s->centres_of_type[s->types[a]];
+      std::vector<int32_t> ncent(n_structures), astruct(s->n_atoms);
+      s->center_off_h.assign(n_structures + 1, 0);
+      std::vector<int32_t> tag2idx;
+      if (s->has_mask) tag2idx.resize(s->n_atoms);
+      for (int i = 0; i < n_structures; ++i) {
+        int64_t a0 = s->atom_off[i], a1 = s->atom_off[i + 1];
+        int nc = 0;
+        for (int64_t a = a0; a < a1; ++a) {
+          astruct[a] = i;
+          if (!center_mask || center_mask[a]) ++nc;
+        }
+        ncent[i] = nc;
+        s->center_off_h[i + 1] = s->center_off_h[i] + nc;
+        if (s->has_mask) {
+          int64_t t = a0;
+          for (int64_t a = a0; a < a1; ++a)
+            if (center_mask[a]) tag2idx[t++] = int32_t(a);
+          for (int64_t a = a0; a < a1; ++a)
+            if (!center_mask[a]) tag2idx[t++] = int32_t(a);
+        }
       }
-      ncent[i] = nc;
-      s->center_off_h[i + 1] = s->center_off_h[i] + nc;
-      if (s->has_mask) {
-        int64_t t = a0;
-        for (int64_t a = a0; a < a1; ++a)
-          if (center_mask[a]) tag2idx[t++] = int32_t(a);
-        for (int64_t a = a0; a < a1; ++a)
-          if (!center_mask[a]) tag2idx[t++] = int32_t(a);
-      }
+      std::vector<Upload> ups = {
+          {&s->atom_off_d, s->atom_off.data(), sizeof(int64_t) * (n_structures + 1)},
+          {&s->pos_d, positions, sizeof(double) * 3 * s->n_atoms},
+          {&s->types_d, numbers, sizeof(int32_t) * s->n_atoms},
+          {&s->cells_d, cells, sizeof(double) * 9 * n_structures},
+          {&s->pbc_d, pbc, sizeof(int32_t) * 3 * n_structures},
+          {&s->ncent_d, ncent.data(), sizeof(int32_t) * n_structures},
+          {&s->center_off_d, s->center_off_h.data(), sizeof(int64_t) * (n_structures + 1)},
+          {&s->atom_struct_d, astruct.data(), sizeof(int32_t) * s->n_atoms}};
+      if (s->has_mask) ups.push_back({&s->tag2idx_d, tag2idx.data(), sizeof(int32_t) * s->n_atoms});
+      upload_inputs(s, ups);
+    } catch (...) {
+      // the former inputs may be gone and the new ones are not there: the
+      // handle is left without structures
+      s->n_struct = 0;
+      s->n_atoms = 0;
+      s->atom_off.assign(1, 0);
+      s->center_off_h.assign(1, 0);
+      s->batch_species.clear();
+      std::fill(s->centres_of_type, s->centres_of_type + 130, int64_t(0));
+      throw;
     }
-    std::vector<Upload> ups = {
-        {&s->atom_off_d, s->atom_off.data(), sizeof(int64_t) * (n_structures + 1)},
-        {&s->pos_d, positions, sizeof(double) * 3 * s->n_atoms},
-        {&s->types_d, numbers, sizeof(int32_t) * s->n_atoms},
-        {&s->cells_d, cells, sizeof(double) * 9 * n_structures},
-        {&s->pbc_d, pbc, sizeof(int32_t) * 3 * n_structures},
-        {&s->ncent_d, ncent.data(), sizeof(int32_t) * n_structures},
-        {&s->center_off_d, s->center_off_h.data(), sizeof(int64_t) * (n_structures + 1)},
-        {&s->atom_struct_d, astruct.data(), sizeof(int32_t) * s->n_atoms}};
-    if (s->has_mask) ups.push_back({&s->tag2idx_d, tag2idx.data(), sizeof(int32_t) * s->n_atoms});
-    upload_inputs(s, ups);
-    s->nl_valid = false;
-    s->feat_valid = false;
-    s->fwd_model = 0;
   });
 }
 
 rgpu_status rgpu_structures_update_positions(rgpu_structures * s, const double * positions) {
   return guard([&] {
     OnDevice on_dev(s);
+    drop_results(s);
     upload_positions(s, positions);
-    s->nl_valid = false;
-    s->feat_valid = false;
-    s->fwd_model = 0;
   });
 }
 
 rgpu_status rgpu_structures_invalidate(rgpu_structures * s) {
   return guard([&] {
     OnDevice on_dev(s);
-    s->nl_valid = false;
-    s->feat_valid = false;
-    s->fwd_model = 0;
+    drop_results(s);
   });
 }
 

@@ -87,7 +87,6 @@ class StructureSet:
         return self._h
 
     def set(self, batch):
-        self.batch = batch
         off = N.i64(batch["atom_offsets"])
         pos = N.f64(batch["positions"])
         num = N.i32(batch["numbers"])
@@ -101,6 +100,7 @@ class StructureSet:
                                             N.ptr(pos, N.c_dbl_p), N.ptr(num, N.c_int_p),
                                             N.ptr(cel, N.c_dbl_p), N.ptr(pbc, N.c_int_p),
                                             N.ptr(m, N.c_u8_p)))
+        self.batch = batch  # a batch that is refused leaves the former one in place
         self.n_structures = len(off) - 1
         self.n_atoms = int(off[-1])
 
