@@ -1619,8 +1619,12 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
   ensure_stream(s);
   bool replay = false;
   if (s->md_exec) {
-    if (s->md_model != m->serial || s->md_stress != stress || m->layout_species != s->species ||
-        s->md_species != s->species)
+    if (s->md_model == m->serial) {
+      // the model's device copies may be laid out for another set's species
+      set_layout(s, m->calc->hy, m->species);
+      model_layout(m, s, true);
+    }
+    if (s->md_model != m->serial || s->md_stress != stress || s->md_species != s->species)
       s->md_reason = 3;
     else if (md_buffers(m, s) != s->md_buffers)
       s->md_reason = 1;
@@ -1629,7 +1633,7 @@ static void md_step_impl(rgpu_gap_model * m, rgpu_structures * s, const double *
   }
   if (replay) {
     std::memcpy(s->md_pos_h, positions, sizeof(double) * 3 * na);
-    ensure_chunk_map(s, make_dims(m->calc->hy, int(s->species.size())));
+    ensure_chunk_map(s, s->fd);
     drop_results(s);  // the replay overwrites positions, list and features
     RGPU_CUDA(cudaGraphLaunch(s->md_exec, s->st));
     RGPU_CUDA(cudaStreamSynchronize(s->st));
