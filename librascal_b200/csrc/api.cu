@@ -1287,6 +1287,7 @@ static void gap_backward_dev_impl(rgpu_gap_model * m, rgpu_structures * s, const
                                        "no other call on the structures in between");
   s->timed = false;
   const int64_t na = s->n_atoms;
+  model_layout(m, s, true);  // another set may have used the model since
   zero_outputs(s, true, false);
   gap_fast_backward(m, s, s->F(), nullptr, energies_grad_dev);
   // the adjoint accumulates forces, -dE/dr

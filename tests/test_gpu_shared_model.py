@@ -60,3 +60,21 @@ def test_recorded_step_after_other_layouts(make_model):
         E0, F0 = own.predict(alone, "fp32")
         assert close(E, E0) and close(F, F0)
     assert replays >= 1
+
+
+@pytest.mark.parametrize("species", [[1, 6, 8], [1, 6, 7, 8], [8]])
+def test_backward_after_another_forward(make_model, species):
+    """Two forwards of one model, then both backwards, in either order."""
+    import torch
+    a, b = box([1, 8], 3), box(species, 4, n_atoms=70)
+    model = make_model()
+    for first in (0, 1):
+        batches = [a, b]
+        pos = [torch.tensor(x["positions"], device="cuda", requires_grad=True) for x in batches]
+        E = [rb.gap_energy(p, model, rb.StructureSet(x)).sum() for p, x in zip(pos, batches)]
+        for k in (first, 1 - first):
+            (g,) = torch.autograd.grad(E[k], pos[k])
+            alone = rb.StructureSet(batches[k])
+            alone.use_graphs(False)
+            _, F0 = make_model().predict(alone, "fp32")
+            assert close(-g.cpu().numpy(), F0)
