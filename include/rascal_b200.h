@@ -349,15 +349,18 @@ rgpu_status rgpu_get_tile_config(int32_t n_species, int32_t max_radial, int32_t 
  * (which sizes buffers through a few host synchronisations) and records the
  * bucket with the neighbour list built to capacities 12.5 % above its
  * counts; later calls of the bucket replay the graph with one
- * synchronisation. A replay whose list outgrows the capacities, or whose
- * input is invalid, is redone by the ordinary path (which reports input
- * errors with the reference's messages) and the bucket is recorded again.
+ * synchronisation. Calls for energies alone, which skip the force half, have
+ * a recording of their own in the bucket, made at the second such call, or
+ * at the third where the first two can replay the full one. A replay whose
+ * list outgrows the capacities, or whose input is invalid, is redone by the
+ * ordinary path (which reports input errors with the reference's messages)
+ * and recorded again.
  * A handle keeps at most four buckets (least recently used dropped). A
  * replayed call records no stage times (rgpu_stage_times keeps those of the
  * last ordinary call). The reference has no counterpart: it prepares each
  * manager on the host (structure_manager_collection.hh:178-184). */
 rgpu_status rgpu_structures_use_graphs(rgpu_structures * s, int enable);
-/* info[0] = recorded buckets held, info[1] = replays, info[2] = recordings,
+/* info[0] = recordings held, info[1] = replays, info[2] = recordings,
  * info[3] = kernels launched by the last replayed graph. */
 rgpu_status rgpu_structures_graph_info(const rgpu_structures * s, int64_t * info /* [4] */);
 /* Measured FMA throughput of the current device's CUDA cores in TFLOP/s,

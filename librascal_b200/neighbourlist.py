@@ -125,7 +125,7 @@ class StructureSet:
         N.check(N.lib().rgpu_structures_use_graphs(self._h, int(bool(enable))))
 
     def graph_info(self):
-        """(buckets held, replays, recordings, kernels of the last replayed
+        """(recordings held, replays, recordings, kernels of the last replayed
         graph) of the recorded FP32 predictions."""
         info = np.zeros(4, np.int64)
         N.check(N.lib().rgpu_structures_graph_info(self._h, N.ptr(info, N.c_i64_p)))
