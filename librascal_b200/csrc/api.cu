@@ -1215,7 +1215,8 @@ static void gap_predict_impl(rgpu_gap_model * m, rgpu_structures * s, int precis
     // neighbour list, layout, features
     build_nl(s, m->calc->hy.cutoff);
     mark(s, 1);
-    compute_features(m->calc, s, precision, want_forces, m->species, /*need_x32=*/false);
+    // the gradients of what a prediction computed may be exported, forces or not
+    compute_features(m->calc, s, precision, /*grads=*/true, m->species, /*need_x32=*/false);
     model_layout(m, s, precision == RGPU_PRECISION_FP32);
     const int64_t na = s->n_atoms;
     zero_outputs(s, want_forces, neg_stress != nullptr);
