@@ -29,6 +29,14 @@ constexpr int kMaxWarps = 8;
 // 1.11 ms against 0.84 per 161 000 centres (its sums are written species by
 // species), and at 34 neighbours of 2 species 37 us against 33 per 2 000.
 constexpr int64_t kFewPairs = 40;
+// With one species the chunked kernel rewrites that species' sums alone, and
+// the registers pay only where a lane has between 17 and 63 of them: few sums
+// are cheap to rewrite, and from 64 on one block is resident per SM. Registers
+// and chunks, ms, 20 000 centres with 65 neighbours: n = 8, l = 6 (16 sums)
+// 0.35 and 0.31; n = 9, l = 8 (36) 0.74 and 0.71; n = 12, l = 9 (48) 0.88 and
+// 1.00; n = 14, l = 10 (64) 1.96 and 1.50; n = 16, l = 12 (96) 2.62 and 2.05.
+// With two species the two are within 5 % at both ends.
+constexpr int kSumsLow = 16, kSumsHigh = 64;
 // Centres per SM up to which a centre gets a block rather than a warp (warp
 // and block, us): 1 000 centres of a box 30 and 22, 1 600 of 100 clusters 26
 // and 22, 1 728 of a box at n = 12, l = 9 76 and 61; 2 000 of a box 33.5 and
@@ -626,7 +634,9 @@ void launch_expansion_fp32(const ExpansionArgs & a, float * C, uint32_t * presen
   RGPU_CUDA(cudaGetDevice(&dev));
   RGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const bool block = a.n_centers <= kFewCentres * sms;
-  if (!block && a.n_pairs < kFewPairs * a.n_centers) {
+  const int sums = (a.fd.K + 31) / 32 * (a.fd.n <= 8 ? 8 : a.fd.n <= 12 ? 12 : 16);
+  const bool few = a.n_pairs < kFewPairs * a.n_centers || (a.fd.S == 1 && (sums <= kSumsLow || sums >= kSumsHigh));
+  if (!block && few) {
     launch_few(a, C, present, st);
     RGPU_LAUNCHED();
     RGPU_CUDA(cudaGetLastError());
