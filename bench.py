@@ -290,6 +290,14 @@ def fma_peaks(lib):
     return out
 
 
+def fp64_tensor_peak(lib):
+    """FP64 tensor TFLOP/s of this GPU, measured by the library's
+    microbenchmark (rgpu_measure_fp64_tensor_peak); None if it failed."""
+    import ctypes
+    v = ctypes.c_double()
+    return v.value if lib.rgpu_measure_fp64_tensor_peak(ctypes.byref(v)) == 0 else None
+
+
 # DRAM bytes (read + write) per grouped GEMM launch at the molecule-cluster
 # workload: the average of the forward and backward launches of one ncu
 # capture of the 2 000-cluster case (32 505 atoms), scaled by atoms to
@@ -357,7 +365,7 @@ def gemm_flops_algorithmic(st, batch, species, msp, n, L):
 
 
 TRAINING_METRIC = "GAP training K_NM rows (energy + position gradients) atoms/s on 1 B200, FP64"
-FP64_NOMINAL_TFLOPS = 37.0  # B200 nominal FP64 (CUDA cores), used only if the measurement fails
+FP64_NOMINAL_TFLOPS = 37.0  # B200 nominal FP64, used only if the measurement fails
 
 
 def run_training(args):
@@ -429,8 +437,8 @@ def run_training(args):
         cpu = dict(value=float(off[ns]) / secs, unit="atoms/s", cores=1, kind="port",
                    sample="first %d clusters (%d atoms), K_NM energy + gradient rows, CPU FP64 restatement, "
                           "1 thread, %.1f s" % (ns, int(off[ns]), secs))
-    fp64_peak = fma_peaks(lib)["fp64"]
-    fp64_kind = "measured FP64 FMA rate of this GPU (rgpu_measure_fma_peak)"
+    fp64_peak = fp64_tensor_peak(lib)
+    fp64_kind = "measured FP64 tensor rate of this GPU (rgpu_measure_fp64_tensor_peak)"
     if not fp64_peak:
         fp64_peak, fp64_kind = FP64_NOMINAL_TFLOPS, "nominal FP64 (the measurement failed)"
     line = dict(metric=TRAINING_METRIC, value=value, unit="atoms/s", n_gpus=1, steps=args.steps,

@@ -369,6 +369,9 @@ rgpu_status rgpu_structures_graph_info(const rgpu_structures * s, int64_t * info
  * events (2 flops per FMA). The denominator of the FP32- and FP64-pipe
  * roofline fractions. No counterpart in the reference. */
 rgpu_status rgpu_measure_fma_peak(int precision, double * tflops);
+/* The same for the FP64 tensor pipe (chains of the tile GEMM's instruction on
+ * register operands): the denominator of the FP64 GEMMs' fractions. */
+rgpu_status rgpu_measure_fp64_tensor_peak(double * tflops);
 
 /* ---------------------------------------------------------------------- */
 /* Unit-test hook for the tensor-core GEMM (no reference counterpart; the

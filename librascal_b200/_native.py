@@ -76,6 +76,7 @@ SIGNATURES = {
     "rgpu_kernel_launches": (ctypes.c_int64, [ctypes.c_int]),
     "rgpu_stage_times": (ctypes.c_int, [ctypes.c_void_p, c_dbl_p, ctypes.c_int32]),
     "rgpu_measure_fma_peak": (ctypes.c_int, [ctypes.c_int, c_dbl_p]),
+    "rgpu_measure_fp64_tensor_peak": (ctypes.c_int, [c_dbl_p]),
     "rgpu_set_tile_config": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, c_int_p,
                                             ctypes.c_int32]),
     "rgpu_get_tile_config": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, c_int_p]),

@@ -2605,6 +2605,13 @@ rgpu_status rgpu_measure_fma_peak(int precision, double * tflops) {
   });
 }
 
+rgpu_status rgpu_measure_fp64_tensor_peak(double * tflops) {
+  return guard([&] {
+    if (!tflops) throw Error(RGPU_ERR_INVALID_ARGUMENT, "null argument");
+    *tflops = measure_fp64_tensor_peak();
+  });
+}
+
 rgpu_status rgpu_synchronize(rgpu_structures * s) {
   return guard([&] {
     OnDevice on_dev(s);

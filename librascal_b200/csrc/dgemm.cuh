@@ -6,14 +6,13 @@
 // planes that the caller's next kernel adds.
 //
 // What bounds it: the FP64 tensor pipe (37.0 TFLOP/s measured with register
-// operands against 29.1 for the same chains of DFMA), which only a full
-// grid reaches. The tile is 64 x 64 rather than 128 x 128 because a warp's
-// 16 x 8 x 8 product needs so few operands (24 doubles for 1024 FMAs) that
-// shared memory does not care, and because the GAP contractions are ragged:
-// per species a few hundred to a few thousand rows by 50..2000 sparse
-// points. 128 x 128 tiles of one species at a time left 6 to 84 blocks on
-// 148 SMs. Splits of K fill the chip where even 64 x 64 tiles of every
-// species do not.
+// operands, peaks.cu; FMA chains reach 34.2), which only a full grid reaches.
+// The tile is 64 x 64 rather than 128 x 128 because a warp's 32 x 32 part of it
+// reads 64 doubles per 1024 FMAs, which shared memory delivers in time, and
+// because the GAP contractions are ragged: per species a few hundred to a few
+// thousand rows by 50..2000 sparse points. 128 x 128 tiles of one species at a
+// time left 6 to 84 blocks on 148 SMs. Splits of K fill the chip where even
+// 64 x 64 tiles of every species do not.
 //
 // 128 threads, 2 x 2 warps of 32 x 32; slices of 16 k in a three-deep
 // cp.async ring. The shared row strides (20 doubles for k-major tiles, 68

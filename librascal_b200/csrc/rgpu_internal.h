@@ -475,6 +475,7 @@ void gap_energies_noalloc(int64_t M, int64_t N, int64_t K, const float * A, cons
 // Measured FMA throughput (TFLOP/s) of the current device's FP32 or FP64
 // pipe (peaks.cu).
 double measure_fma_peak(int precision);
+double measure_fp64_tensor_peak();
 // hi/lo BF16 split of a row-major FP32 matrix (columns >= cols become 0).
 void split_bf16(const float * x, int64_t rows, int64_t cols, int64_t ldx, __nv_bfloat16 * hi,
                 __nv_bfloat16 * lo, int64_t ldo, cudaStream_t st);
