@@ -25,7 +25,6 @@
 
 namespace rgpu {
 int64_t launches(bool reset);
-extern bool g_tf32_split;
 }  // namespace rgpu
 
 using namespace rgpu;

@@ -32,12 +32,6 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
-__device__ __forceinline__ float to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return __uint_as_float(r);
-}
-
 inline int div_up(int64_t a, int64_t b) { return int((a + b - 1) / b); }
 
 // Radial factor u(r) of the RadialScaling cutoff and its derivative

@@ -151,7 +151,7 @@ expansion_f32_kernel(ExpansionArgs a, float * __restrict__ C, uint32_t * __restr
         if (hq < np) {
           float * y = Y + hq * SM::KP;
           pair_harmonics<L>(hc, geo[at + hq], geo[kWindow + at + hq], geo[2 * kWindow + at + hq], hj,
-                            [&](int l, int m, float v, float, float re, float im, float, float) {
+                            [&](int l, int m, float v, float re, float im) {
                               const int o = l * l + l;
                               if (m == 0) {
                                 y[o] = v * 0.707106781186547524400844362104849039f;
@@ -474,7 +474,7 @@ expansion_block_kernel(ExpansionArgs a, float * __restrict__ C, uint32_t * __res
       for (int q = threadIdx.x / NL; q < np && threadIdx.x < kBlockThreads / NL * NL; q += kBlockThreads / NL) {
         float * y = Y + q * RS;
         pair_harmonics<L>(hc, geo[0][q], geo[1][q], geo[2][q], threadIdx.x % NL,
-                          [&](int l, int m, float v, float, float re, float im, float, float) {
+                          [&](int l, int m, float v, float re, float im) {
                             float * o = y + offp_rt(l) + l;
                             if (m == 0) {
                               *o = v * 0.707106781186547524400844362104849039f;

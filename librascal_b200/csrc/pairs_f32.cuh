@@ -46,44 +46,41 @@ struct HarmonicConstants {
 };
 
 // The harmonics of the unit vector (x, y, z) that belong to lane j of the
-// pair's NL lanes. emit(l, m, q, dq, re, im, re1, im1) gets, for every l >= m
-// of its orders, q_lm and dq_lm/dz, (x + iy)^m and (x + iy)^(m-1):
-// Y_l,m = q re, Y_l,-m = q im (m > 0), Y_l0 = q / sqrt2.
+// pair's NL lanes. emit(l, m, q, re, im) gets, for every l >= m of its orders,
+// q_lm and (x + iy)^m: Y_l,m = q re, Y_l,-m = q im (m > 0), Y_l0 = q / sqrt2.
 template <int L, class Emit>
 __device__ __forceinline__ void pair_harmonics(const HarmonicConstants<L> & c, float x, float y, float z, int j,
                                                Emit && emit) {
   const int m2 = L - j;
   float re = 1.f, im = 0.f;
-  float ra = 1.f, ia = 0.f, pa = 0.f, sa = 0.f;  // powers j and j - 1
-  float rb = 1.f, ib = 0.f, pb = 0.f, sb = 0.f;  // powers L - j and L - j - 1
+  float ra = 1.f, ia = 0.f;  // power j
+  float rb = 1.f, ib = 0.f;  // power L - j
 #pragma unroll
   for (int k = 1; k <= L; ++k) {
     const float nr = re * x - im * y, ni = re * y + im * x;
-    if (k == j) ra = nr, ia = ni, pa = re, sa = im;
-    if (k == m2) rb = nr, ib = ni, pb = re, sb = im;
+    if (k == j) ra = nr, ia = ni;
+    if (k == m2) rb = nr, ib = ni;
     re = nr;
     im = ni;
   }
   int m = j, l = j;
   bool on = true;
-  float q0 = c.cmm[j], q1 = 0.f, d0 = 0.f, d1 = 0.f;
+  float q0 = c.cmm[j], q1 = 0.f;
 #pragma unroll
   for (int step = 0; step < L + 2; ++step) {
-    if (on) emit(l, m, q0, d0, ra, ia, pa, sa);
+    if (on) emit(l, m, q0, ra, ia);
     if (l < L) {
       ++l;
       const float2 r = c.rec[m * (L + 1) + l];
-      const float az = r.x * z, q = az * q0 + r.y * q1, d = az * d0 + r.x * q0 + r.y * d1;
+      const float q = r.x * z * q0 + r.y * q1;
       q1 = q0;
       q0 = q;
-      d1 = d0;
-      d0 = d;
     } else {
       on = m < m2;  // the second order, once
       m = l = m2;
       q0 = c.cmm[m2];
-      q1 = d0 = d1 = 0.f;
-      ra = rb, ia = ib, pa = pb, sa = sb;
+      q1 = 0.f;
+      ra = rb, ia = ib;
     }
   }
 }

@@ -398,23 +398,6 @@ void launch_gap_pointwise_fp64(const GapGroup & g, double * Kmat, const double *
 // One FP64 GEMM C = A B^T.
 void gemm_nt_fp64(int64_t M, int64_t N, int64_t K, const double * A, int64_t lda,
                   const double * B, int64_t ldb, double * C, int64_t ldc, cudaStream_t st);
-// TF32 tensor-core GEMM C = A B^T (both K-major) with optional GAP epilogue.
-struct Tf32GemmArgs {
-  int64_t M, N, K;  // rows of A, rows of B, reduction length (multiple of 32)
-  const float * A;
-  int64_t lda;
-  const float * B;
-  int64_t ldb;
-  float * C;  // plain store (epilogue 0) or W (epilogue 1)
-  int64_t ldc;
-  // GAP epilogue
-  int epilogue;          // 0: store C; 1: GAP forward
-  const float * alpha;   // [N]
-  int zeta;
-  float * e_part;        // [n_tiles_N][M] row partial energies
-};
-void gemm_tf32(const Tf32GemmArgs & g, cudaStream_t st);
-
 // tcgen05 GEMM, C = A B^T as a 3-term BF16 split (A_hi B_hi + A_hi B_lo +
 // A_lo B_hi), FP32 accumulation in TMEM. A [M x K] and B [N x K] are
 // row-major hi/lo BF16 pairs (row strides lda, ldb; 16-byte aligned).
@@ -575,7 +558,6 @@ void launch_mask_sort(int64_t n, const int32_t * types, const int32_t * center_a
 // Stable sort of centres by species.
 void launch_species_sort(int64_t n, const int32_t * types, const int32_t * center_atom, const int8_t * lut, int S,
                          int32_t * row_of_center, int32_t * center_of_row, DevBuf & tmp, cudaStream_t st);
-void launch_round_tf32(float * x, int64_t n, cudaStream_t st);
 void launch_fill_f64(double * p, int64_t n, double v, cudaStream_t st);
 void launch_fill_f32(float * p, int64_t n, float v, cudaStream_t st);
 // out = a + b; out = a x (n doubles, device)

@@ -445,10 +445,6 @@ small_sort_kernel(int n, const int32_t * __restrict__ types, const int32_t * __r
   }
 }
 
-__global__ void round_tf32_kernel(float * x, int64_t n) {
-  int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) x[i] = to_tf32(x[i]);
-}
 __global__ void fill_f64_kernel(double * p, int64_t n, double v) {
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n) p[i] = v;
@@ -535,11 +531,6 @@ void launch_species_sort(int64_t n, const int32_t * types, const int32_t * cente
   RGPU_LAUNCHED();
 }
 
-void launch_round_tf32(float * x, int64_t n, cudaStream_t st) {
-  if (n <= 0) return;
-  round_tf32_kernel<<<div_up(n, 256), 256, 0, st>>>(x, n);
-  RGPU_LAUNCHED();
-}
 void launch_fill_f64(double * p, int64_t n, double v, cudaStream_t st) {
   if (n <= 0) return;
   fill_f64_kernel<<<div_up(n, 256), 256, 0, st>>>(p, n, v);
