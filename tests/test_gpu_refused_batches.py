@@ -24,12 +24,15 @@ def refused(batch, how):
     elif how == "more structures":
         bad = dict(atom_offsets=np.concatenate([np.arange(n), [n - 2]]), positions=batch["positions"],
                    numbers=batch["numbers"], cells=np.tile(batch["cells"], (n, 1, 1)), pbc=np.tile(batch["pbc"], (n, 1)))
+    elif how in ("nan", "inf"):
+        bad["cells"] = np.array(batch["cells"])
+        bad["cells"][0, 1, 1] = float(how)
     else:
         bad["atom_offsets"] = np.array([1, n])
     return bad
 
 
-@pytest.mark.parametrize("how", ["type", "more atoms", "more structures", "first offset"])
+@pytest.mark.parametrize("how", ["type", "more atoms", "more structures", "first offset", "nan", "inf"])
 def test_former_batch_stays(how):
     batch, model = setup_box(seed=31)
     st = rb.StructureSet(batch)
