@@ -44,23 +44,24 @@ __host__ __device__ constexpr int staged_row(int row_len) { return ((row_len + 3
 // derivative is the next order's q, and whose plain gradient sum is projected
 // onto the sphere once per pair at the end.
 //
-// Two reads bounded this kernel, and a warp or block shares both:
+// Two reads would bound this kernel if each lane made its own, and a warp or
+// block shares both:
 //  - dE/dc of the centre, n (l+1)^2 values per pair, n contiguous ones per lm:
-//    each waited on L1 or L2 with about 20 warps per SM to hide it. With STAGE
+//    each waits on L1 or L2 with about 20 warps per SM to hide it. With STAGE
 //    the rows of the block's centres (`rows` at a time) are copied to shared
 //    memory first, every copy in flight at once. That pays while a block spans
 //    few centres; the launch decides (10 000 clusters with 12 neighbours and
 //    7.8 KB rows read theirs through L2, after a prefetch).
 //  - the spline table: every pair lies in another interval, so 32 lanes read
 //    32 lines per channel (30 wavefronts a load, half of the LSU's time). 8 or
-//    4 lanes now copy neighbouring channels of one pair's interval to shared
+//    4 lanes copy neighbouring channels of one pair's interval to shared
 //    memory, asynchronously and one l ahead, and its own lane reads them there.
 // What is left is issue: 1.6 instructions a cycle with 12 warps per SM.
-// The loop over l is rolled: unrolled it outgrew the instruction cache (2.2 of
-// 15 cycles per instruction waited for it). FULL (n = NV) keeps the bounds of
+// The loop over l is rolled: unrolled it outgrows the instruction cache (2.2 of
+// 15 cycles per instruction wait for it). FULL (n = NV) keeps the bounds of
 // the channel loops and the strides of 16-byte reads out of it.
-// Before and now: 100 000 atoms with 46 neighbours at n = 12, l = 9, 4.2 and
-// 1.9 ms; 10 000 clusters (n = 8, l = 6, 5 species) 1.04 and 0.64 ms; a box of
+// Each lane on its own and shared: 100 000 atoms with 46 neighbours at n = 12,
+// l = 9, 4.2 and 1.9 ms; 10 000 clusters (n = 8, l = 6, 5 species) 1.04 and 0.64 ms; a box of
 // 150 atoms with 34 neighbours (n = 8, l = 6) 26 and 13.6 us; 97 cells at
 // n = 7, l = 5, 384 and 254 us.
 //

@@ -7,9 +7,9 @@
 // warp per centre, pairs by species (pairs_f32.cuh). The coefficients of
 // one species stay in registers, lanes over lm and n per lane, while its pairs
 // pass: per pair and 32 lm one value of Y and n/4 broadcast loads of f_c RI
-// feed n products. They are written once per species. The previous kernel kept
-// them in global memory between chunks of 8 or 16 pairs (12.7 KB read and
-// written per chunk at S = 2, n = 12, l = 9, some 15 GB for 100 000 atoms).
+// feed n products. They are written once per species. Kept in global memory
+// between chunks of 8 or 16 pairs they are 12.7 KB read and written per chunk
+// at S = 2, n = 12, l = 9, some 15 GB for 100 000 atoms.
 #include <cuda_runtime.h>
 
 #include <algorithm>

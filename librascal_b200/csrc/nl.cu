@@ -164,7 +164,7 @@ __device__ __forceinline__ bool ghost_pos(const NlGeom & g, const double * x0, c
 }
 
 // kImageLanes lanes share an atom: with 27 and more images per atom of a
-// periodic structure, one thread's loop over them was a chain of 10 to 40 us
+// periodic structure, one thread's loop over them is a chain of 10 to 40 us
 // whatever the batch.
 constexpr int kImageLanes = 8;
 __device__ __forceinline__ unsigned image_group_bits(unsigned ballot) {
@@ -312,9 +312,9 @@ __global__ void nl_scatter_kernel(int64_t n_sites, const int64_t * __restrict__ 
 
 // Ascending site (= tag) order inside every box, with the positions packed in
 // that order. A warp takes `per` boxes and sorts the occupied ones by rank, one
-// lane per site (a thread per box was an insertion sort in global memory).
+// lane per site.
 // One box per warp where the boxes are few, 32 where they are many and mostly
-// empty: at 1 000 boxes of a dense cell 32 took 18 to 23 us, a chain of 32.
+// empty: at 1 000 boxes of a dense cell 32 take 18 to 23 us, a chain of 32.
 __global__ void nl_boxsort_kernel(int64_t n_boxes, int per, const int64_t * __restrict__ box_ptr,
                                   const int64_t * __restrict__ binned, const double * __restrict__ site_x,
                                   int64_t * __restrict__ sorted, double * __restrict__ sorted_x) {

@@ -140,7 +140,7 @@ namespace {
 // beyond, tiles of kScanTile values are scanned by themselves and a second
 // launch adds to each the sum of the tiles before it, which every block takes
 // from the tile sums itself. What bounds the small ones is the launch (about
-// 2 us each in a recorded graph; the recursive form took two to five nodes).
+// 2 us each in a recorded graph; a recursive form takes two to five nodes).
 constexpr int kScanBlock = 1024, kScanTile = 4 * kScanBlock, kScanOne = 2 * kScanTile;
 
 // Exclusive scan over the block of the four values each thread holds;
