@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <memory>
 #include <set>
@@ -2051,12 +2052,15 @@ rgpu_status rgpu_structures_set(rgpu_structures * s, int32_t n_structures, const
         throw Error(RGPU_ERR_INVALID_ARGUMENT, "atom_offsets must be non-decreasing");
     const int64_t n_atoms = atom_offsets[n_structures];
     if (n_atoms > (int64_t(1) << 31) - 1) throw Error(RGPU_ERR_INVALID_ARGUMENT, "too many atoms");
-    for (int64_t k = 0; k < 9 * int64_t(n_structures); ++k)
-      if (!std::isfinite(cells[k])) {
-        // the mesh of such a cell has no boxes, and every site falls outside
-        throw Error(RGPU_ERR_STRUCTURE, "the unit cell holds a value that is not finite (structure " +
-                                            std::to_string(k / 9) + ")");
-      }
+    // The mesh of a cell that is not finite has no boxes, and every site falls
+    // outside. One pass without branches, then the search.
+    const int64_t n_cell = 9 * int64_t(n_structures);
+    unsigned bad = 0;
+    for (int64_t k = 0; k < n_cell; ++k) bad |= unsigned(!(std::fabs(cells[k]) <= std::numeric_limits<double>::max()));
+    for (int64_t k = 0; bad && k < n_cell; ++k)
+      if (!std::isfinite(cells[k]))
+        throw Error(RGPU_ERR_STRUCTURE,
+                    "the unit cell holds a value that is not finite (structure " + std::to_string(k / 9) + ")");
     bool seen[130] = {false};
     for (int64_t a = 0; a < n_atoms; ++a) {
       if (numbers[a] < 0 || numbers[a] >= 130)
